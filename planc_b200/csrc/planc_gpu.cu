@@ -329,15 +329,15 @@ void launch(planc_gpu_ctx* c, int cls, Fn&& fn) {
   c->launch_count++;
 }
 
-// Launches `kern` as one thread-block cluster of `ncta` CTAs of NES_THREADS
-// threads (cluster sizes above 8 need the kernel's non-portable attribute,
-// set by enable_cluster16).
+// Launches `kern` as one thread-block cluster of `ncta` CTAs (cluster sizes
+// above 8 need the kernel's non-portable attribute, set by enable_cluster16).
 template <typename... KArgs, typename... Args>
-void launch_cluster(void (*kern)(KArgs...), int ncta, cudaStream_t s, Args... args) {
+void launch_cluster(void (*kern)(KArgs...), int ncta, int threads, size_t smem, cudaStream_t s,
+                    Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ncta, 1, 1);
-  cfg.blockDim = dim3(NES_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = 0;
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -349,9 +349,12 @@ void launch_cluster(void (*kern)(KArgs...), int ncta, cudaStream_t s, Args... ar
   CK(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 
-// Allows clusters of 16 for `kern` and reports whether one fits on the device.
+// Allows `smem` bytes of dynamic shared memory and clusters of 16 for `kern`
+// and reports whether such a cluster fits on the device.
 template <typename... KArgs>
-bool enable_cluster16(void (*kern)(KArgs...)) {
+bool enable_cluster16(void (*kern)(KArgs...), int threads = NES_THREADS, size_t smem = 0) {
+  if (smem)
+    CK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
       cudaSuccess) {
     cudaGetLastError();
@@ -359,7 +362,8 @@ bool enable_cluster16(void (*kern)(KArgs...)) {
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(NES_CTAS_MAX, 1, 1);
-  cfg.blockDim = dim3(NES_THREADS, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = NES_CTAS_MAX;
@@ -373,6 +377,12 @@ bool enable_cluster16(void (*kern)(KArgs...)) {
     return false;
   }
   return n >= 1;
+}
+
+// The same for a shape of the register-resident Nesterov loop.
+template <int KP, int R>
+bool enable_nes16() {
+  return enable_cluster16(k_nes_inner_reg<KP, R>, NesReg<KP, R>::THREADS, NesReg<KP, R>::SMEM);
 }
 
 template <int BE>
@@ -1078,7 +1088,7 @@ void run_update(planc_gpu_ctx* c, int algo, int n) {
     if ((k <= 32 && rpw <= 8) || rpw <= 4) {
       launch(c, KC_UPDATE, [&] {
 #define ADMM_CL(KP, R)                                                                       \
-  launch_cluster(k_admm_cluster<KP, R>, c->cl_ctas, c->stream, c->F[n], c->aux[n],           \
+  launch_cluster(k_admm_cluster<KP, R>, c->cl_ctas, NES_THREADS, 0, c->stream, c->F[n], c->aux[n], \
                  (const double*)c->M[n], (const double*)c->Gloo, I, k, 0.01, c->status_dev)
         if (k <= 32 && rpw <= 1) ADMM_CL(32, 1);
         else if (k <= 32 && rpw <= 2) ADMM_CL(32, 2);
@@ -1125,24 +1135,27 @@ void run_update(planc_gpu_ctx* c, int algo, int n) {
     // the accelerated proximal-gradient loop from the proximal point, in one
     // cluster launch.
     launch(c, KC_UPDATE, [&] {
-      k_nes_prep<<<1, 256, 0, c->stream>>>(c->Gloo, k, c->nes, n, c->nes_lam, c->nes_lam + k);
+      k_nes_prep<<<1, NES_PREP_THREADS, 0, c->stream>>>(c->Gloo, k, c->nes, n, c->nes_lam, c->nes_lam + k);
     });
-    // rows per warp of the cluster; up to 8 (rank <= 32) or 4 (rank <= 64)
-    // rows stay in registers, beyond that the state lives in global scratch
-    const int64_t warps = (int64_t)c->cl_ctas * (NES_THREADS / 32);
-    const int64_t rpw = (I + warps - 1) / warps;
+    // the smallest register-resident shape whose cluster holds every row;
+    // beyond the largest the state lives in global scratch
+    auto fits = [&](int64_t rows_per_cta) { return I <= rows_per_cta * c->cl_ctas; };
     launch(c, KC_UPDATE, [&] {
 #define NES_REG(KP, R)                                                                       \
-  launch_cluster(k_nes_inner_reg<KP, R>, c->cl_ctas, c->stream, c->F[n],                      \
-                 (const double*)c->prox[n], c->prev[n], (const double*)c->M[n],               \
-                 (const double*)c->Gloo, c->nes, I, k, c->nes_max_steps, c->status_dev)
-      if (k <= 32 && rpw <= 1) NES_REG(32, 1);
-      else if (k <= 32 && rpw <= 2) NES_REG(32, 2);
-      else if (k <= 32 && rpw <= 4) NES_REG(32, 4);
-      else if (k <= 32 && rpw <= 8) NES_REG(32, 8);
-      else if (k > 32 && rpw <= 1) NES_REG(64, 1);
-      else if (k > 32 && rpw <= 2) NES_REG(64, 2);
-      else if (k > 32 && rpw <= 4) NES_REG(64, 4);
+  launch_cluster(k_nes_inner_reg<KP, R>, c->cl_ctas, NesReg<KP, R>::THREADS, NesReg<KP, R>::SMEM, \
+                 c->stream, c->F[n], (const double*)c->prox[n], c->prev[n],                  \
+                 (const double*)c->M[n], (const double*)c->Gloo, c->nes, I, k, c->nes_max_steps, \
+                 c->status_dev)
+      if (k <= 16 && fits(NesReg<16, 1>::ROWS)) NES_REG(16, 1);
+      else if (k <= 16 && fits(NesReg<16, 2>::ROWS)) NES_REG(16, 2);
+      else if (k <= 16 && fits(NesReg<16, 4>::ROWS)) NES_REG(16, 4);
+      else if (k <= 32 && fits(NesReg<32, 1>::ROWS)) NES_REG(32, 1);
+      else if (k <= 32 && fits(NesReg<32, 2>::ROWS)) NES_REG(32, 2);
+      else if (k <= 32 && fits(NesReg<32, 4>::ROWS)) NES_REG(32, 4);
+      else if (k <= 32 && fits(NesReg<32, 8>::ROWS)) NES_REG(32, 8);
+      else if (k > 32 && fits(NesReg<64, 1>::ROWS)) NES_REG(64, 1);
+      else if (k > 32 && fits(NesReg<64, 2>::ROWS)) NES_REG(64, 2);
+      else if (k > 32 && fits(NesReg<64, 4>::ROWS)) NES_REG(64, 4);
       else if (k <= 32)
         k_nes_inner<32><<<NES_CTAS, NES_THREADS, 0, c->stream>>>(
             c->F[n], c->prox[n], c->prev[n], c->M[n], c->Gloo, c->nes, c->nes_acc, c->nes_grad,
@@ -1389,10 +1402,16 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
     ok = ok && enable_cluster16(k_admm_cluster<32, 4>) && enable_cluster16(k_admm_cluster<32, 8>);
     ok = ok && enable_cluster16(k_admm_cluster<64, 1>) && enable_cluster16(k_admm_cluster<64, 2>);
     ok = ok && enable_cluster16(k_admm_cluster<64, 4>);
-    ok = ok && enable_cluster16(k_nes_inner_reg<32, 1>) && enable_cluster16(k_nes_inner_reg<32, 2>);
-    ok = ok && enable_cluster16(k_nes_inner_reg<32, 4>) && enable_cluster16(k_nes_inner_reg<32, 8>);
-    ok = ok && enable_cluster16(k_nes_inner_reg<64, 1>) && enable_cluster16(k_nes_inner_reg<64, 2>);
-    ok = ok && enable_cluster16(k_nes_inner_reg<64, 4>);
+    ok = enable_nes16<16, 1>() && ok;
+    ok = enable_nes16<16, 2>() && ok;
+    ok = enable_nes16<16, 4>() && ok;
+    ok = enable_nes16<32, 1>() && ok;
+    ok = enable_nes16<32, 2>() && ok;
+    ok = enable_nes16<32, 4>() && ok;
+    ok = enable_nes16<32, 8>() && ok;
+    ok = enable_nes16<64, 1>() && ok;
+    ok = enable_nes16<64, 2>() && ok;
+    ok = enable_nes16<64, 4>() && ok;
     c->cl_ctas = ok ? NES_CTAS_MAX : NES_CTAS;
   }
   const int k = c->k;

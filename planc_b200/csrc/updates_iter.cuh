@@ -681,112 +681,139 @@ __device__ __forceinline__ double nes_alpha_of(double alpha, double q) {
   return (-b + sqrt(D)) / 2;
 }
 
-// Extreme eigenvalues of the symmetric G (arma::eig_sym, ntfnes.hpp:111-113)
-// by cyclic Jacobi rotations, k/2 disjoint rotations per round in the
-// round-robin order, until a sweep finds every off-diagonal entry below the
-// rounding level of its two diagonal entries.
+// Number of eigenvalues below sigma of the symmetric tridiagonal matrix with
+// diagonal d and squared off-diagonals e2 (both scaled so that no entry
+// exceeds 1): the sign changes of the leading minors of T - sigma I
+// (p_i+1 = (d_i - sigma) p_i - e_i^2 p_i-1). No division on the chain; a
+// vanishing minor counts as a change, and both minors are rescaled by a power
+// of two whenever they leave [2^-300, 2^300].
+__device__ __forceinline__ int nes_count_below(const double* d, const double* e2, int k, double sigma) {
+  double p0 = 1.0, p1 = d[0] - sigma;
+  if (p1 == 0.0) p1 = -0x1p-60;
+  int cnt = p1 < 0.0;
+  for (int i = 1; i < k; ++i) {
+    double p2 = fma(d[i] - sigma, p1, -(e2[i - 1] * p0));
+    if (p2 == 0.0) p2 = p1 * -0x1p-60;
+    cnt += (p2 < 0.0) != (p1 < 0.0);
+    p0 = p1;
+    p1 = p2;
+    const double m = fmax(fabs(p0), fabs(p1));
+    const double f = m > 0x1p300 ? 0x1p-300 : m < 0x1p-300 ? 0x1p300 : 1.0;
+    p0 *= f;
+    p1 *= f;
+  }
+  return cnt;
+}
+
+// Extreme eigenvalues of the symmetric G (arma::eig_sym, ntfnes.hpp:111-113),
+// as LAPACK's symmetric drivers find them: Householder reduction to
+// tridiagonal form (Golub & Van Loan, Matrix Computations, 8.3.1), then
+// bisection with Sturm counts (ibid., 8.4.1), 32 shifts a round (one per
+// lane; warp 0 narrows the smallest eigenvalue, warp 1 the largest). Bound by
+// the k - 2 dependent reflections: eight threads per row, two barriers a
+// reflection, the short sums taken by every warp redundantly so that they
+// need no barrier: 29 us at k = 16 (cyclic Jacobi rotations, k/2 disjoint ones
+// a round, took 105 us). One CTA.
 // Then lambda, q and 1/(L + lambda) of the update (ntfnes.hpp:114-117). For
 // mode 0 it also copies the proximal lambda to the previous one
-// (ntfnes.hpp:102-104). One CTA of 256 threads.
-__global__ void __launch_bounds__(256) k_nes_prep(const double* __restrict__ G, int k,
+// (ntfnes.hpp:102-104).
+constexpr int NES_PREP_THREADS = 512;
+__global__ void __launch_bounds__(NES_PREP_THREADS) k_nes_prep(const double* __restrict__ G, int k,
                                                   NesDev* __restrict__ st, int mode,
                                                   const double* __restrict__ prox_lam,
                                                   double* __restrict__ prev_lam) {
   constexpr int LD = kMaxRank + 1;
   __shared__ double A[kMaxRank * LD];
-  __shared__ double rc[kMaxRank / 2], rs[kMaxRank / 2];
-  __shared__ int rp[kMaxRank / 2], rq[kMaxRank / 2];
-  __shared__ int s_rot;
-  const int tid = threadIdx.x;
+  __shared__ double pv[kMaxRank];                     // p = tau A v of the reflection
+  __shared__ double td[kMaxRank], te[kMaxRank];       // diagonal, off-diagonal
+  __shared__ double ext[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (mode == 0 && tid < k) prev_lam[tid] = prox_lam[tid];
-  for (int e = tid; e < k * k; e += blockDim.x) A[(e / k) * LD + e % k] = G[e];
+  for (int e = tid; e < k * k; e += NES_PREP_THREADS) A[(e / k) * LD + e % k] = G[e];
   __syncthreads();
-  const int n2 = (k + 1) & ~1;  // even player count of the round-robin
-  const int np = n2 / 2;
-  if (tid == 0) s_rot = 0;
-  __syncthreads();
-  for (int sweep = 0; sweep < 60; ++sweep) {
-    for (int round = 0; round < n2 - 1; ++round) {
-      if (tid < np) {
-        // circle method: player 0 fixed, x_j = ((j + round) mod m) + 1 rotate;
-        // pairs (0, x_0) and (x_j, x_{m-j}) for 0 < j < np
-        const int m = n2 - 1;
-        const int a = tid == 0 ? 0 : ((tid + round) % m) + 1;
-        const int b = tid == 0 ? (round % m) + 1 : ((m - tid + round) % m) + 1;
-        const int p = a < b ? a : b, q = a < b ? b : a;
-        double c = 1.0, s = 0.0;
-        if (q < k) {
-          const double apq = A[p * LD + q];
-          const double app = A[p * LD + p], aqq = A[q * LD + q];
-          // a pair whose coupling is below the rounding level of its diagonal
-          // is converged (the classical threshold of cyclic Jacobi)
-          if (fabs(apq) > 1e-17 * sqrt(fabs(app * aqq)) && apq != 0.0) {
-            const double theta = (aqq - app) / (2.0 * apq);
-            double t;
-            if (fabs(theta) > 1e150)
-              t = 0.5 / theta;
-            else
-              t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(1.0 + theta * theta));
-            c = 1.0 / sqrt(1.0 + t * t);
-            s = t * c;
-            s_rot = 1;
-          }
-        }
-        rp[tid] = p;
-        rq[tid] = q;
-        rc[tid] = c;
-        rs[tid] = s;
-      }
-      __syncthreads();
-      // A <- J^T A J in one pass: the rotations are disjoint, so every 2 x 2
-      // block (pair pi's rows, pair pj's columns) changes only through its own
-      // four entries; a thread rotates its block's rows, then its columns (the
-      // same operations as a row pass followed by a column pass)
-      for (int blk = tid; blk < np * np; blk += blockDim.x) {
-        const int pi = blk / np, pj = blk % np;
-        const int p1 = rp[pi], q1 = rq[pi], p2 = rp[pj], q2 = rq[pj];
-        const double s1 = rs[pi], s2 = rs[pj];
-        if (s1 == 0.0 && s2 == 0.0) continue;
-        const double c1 = rc[pi], c2 = rc[pj];
-        const bool q1ok = q1 < k, q2ok = q2 < k;
-        const double a11 = A[p1 * LD + p2];
-        const double a12 = q2ok ? A[p1 * LD + q2] : 0.0;
-        const double a21 = q1ok ? A[q1 * LD + p2] : 0.0;
-        const double a22 = (q1ok && q2ok) ? A[q1 * LD + q2] : 0.0;
-        double r11 = a11, r12 = a12, r21 = a21, r22 = a22;
-        if (s1 != 0.0) {
-          r11 = c1 * a11 - s1 * a21;
-          r21 = s1 * a11 + c1 * a21;
-          r12 = c1 * a12 - s1 * a22;
-          r22 = s1 * a12 + c1 * a22;
-        }
-        double o11 = r11, o12 = r12, o21 = r21, o22 = r22;
-        if (s2 != 0.0) {
-          o11 = c2 * r11 - s2 * r12;
-          o12 = s2 * r11 + c2 * r12;
-          o21 = c2 * r21 - s2 * r22;
-          o22 = s2 * r21 + c2 * r22;
-        }
-        A[p1 * LD + p2] = o11;
-        if (q2ok) A[p1 * LD + q2] = o12;
-        if (q1ok) A[q1 * LD + p2] = o21;
-        if (q1ok && q2ok) A[q1 * LD + q2] = o22;
-      }
-      __syncthreads();
+  const int row = tid >> 3, part = tid & 7;
+  for (int j = 0; j + 2 < k; ++j) {
+    // v = x + sign(x_0) ||x|| e_0 for x = A(j+1:, j); every warp forms the norm
+    const int c0 = j + 1 + lane, c1 = c0 + 32;
+    const double x0 = c0 < k ? A[c0 * LD + j] : 0.0, x1 = c1 < k ? A[c1 * LD + j] : 0.0;
+    const double tail = fma(x1, x1, lane == 0 ? 0.0 : x0 * x0);
+    double s2 = tail;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    const double head = A[(j + 1) * LD + j];
+    if (s2 == 0.0) {  // the column is already reduced (the same in every thread)
+      if (tid == 0) te[j] = head;
+      continue;
     }
-    const int rotated = s_rot;  // read by every thread before it is reset
+    const double nrm = sqrt(fma(head, head, s2));
+    const double e = head > 0.0 ? -nrm : nrm;
+    const double v_head = head - e;
+    const double tau = 2.0 / fma(v_head, v_head, s2);
+    auto v_at = [&](int c) { return c == j + 1 ? v_head : A[c * LD + j]; };
+    const bool mine = row > j && row < k;
+    double acc = 0.0;
+    if (mine)
+      for (int c = j + 1 + part; c < k; c += 8) acc = fma(A[row * LD + c], v_at(c), acc);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (mine && part == 0) pv[row] = tau * acc;
+    if (tid == 0) te[j] = e;
     __syncthreads();
-    if (!rotated) break;  // a sweep without a rotation: converged
-    if (tid == 0) s_rot = 0;
+    // K = tau / 2 v^T p, w = p - K v, A -= v w^T + w v^T
+    const double vl0 = c0 < k ? (lane == 0 ? v_head : x0) : 0.0, vl1 = x1;
+    double vp = fma(vl1, c1 < k ? pv[c1] : 0.0, c0 < k ? vl0 * pv[c0] : 0.0);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vp += __shfl_xor_sync(0xffffffffu, vp, o);
+    const double K = 0.5 * tau * vp;
+    if (mine) {
+      const double vr = v_at(row), wr = fma(-K, vr, pv[row]);
+      for (int c = j + 1 + part; c < k; c += 8) {
+        const double vc = v_at(c), wc = fma(-K, vc, pv[c]);
+        A[row * LD + c] -= fma(vr, wc, wr * vc);
+      }
+    }
     __syncthreads();
   }
-  if (tid == 0) {
-    double lo = A[0], hi = A[0];
-    for (int i = 1; i < k; ++i) {
-      const double d = A[i * LD + i];
-      lo = d < lo ? d : lo;
-      hi = d > hi ? d : hi;
+  if (tid < k) td[tid] = A[tid * LD + tid];
+  if (tid == 0 && k >= 2) te[k - 2] = A[(k - 1) * LD + k - 2];
+  __syncthreads();
+  if (warp < 2) {
+    // a power of two above the Gershgorin bound scales the matrix into [-1, 1]
+    double bound = 0.0;
+    for (int i = lane; i < k; i += 32)
+      bound = fmax(bound, fabs(td[i]) + (i + 1 < k ? fabs(te[i]) : 0.0) + (i > 0 ? fabs(te[i - 1]) : 0.0));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bound = fmax(bound, __shfl_xor_sync(0xffffffffu, bound, o));
+    int ex = 0;
+    frexp(bound, &ex);
+    const double scale = ldexp(1.0, -ex);
+    double* d = A + warp * 2 * kMaxRank;  // the reduced matrix is no longer needed
+    double* e2 = d + kMaxRank;
+    for (int i = lane; i < k; i += 32) {
+      const double e = i + 1 < k ? te[i] * scale : 0.0;
+      d[i] = td[i] * scale;
+      e2[i] = e * e;
     }
+    __syncwarp();
+    const int want = warp == 0 ? 1 : k;  // smallest: count >= 1; largest: count >= k
+    double lo = -1.0, hi = 1.0;
+    // 2^-59 of the norm, or two units in the last place: rounds end there
+    for (int it = 0; it < 24 && hi - lo > fmax(0x1p-59, 0x1p-52 * fmax(fabs(lo), fabs(hi))); ++it) {
+      const double h = (hi - lo) * (1.0 / 33.0);
+      const double sg = fma(h, (double)(lane + 1), lo);
+      const unsigned b = __ballot_sync(0xffffffffu, nes_count_below(d, e2, k, sg) >= want);
+      const int f = b ? __ffs(b) - 1 : 32;  // first shift with enough eigenvalues below it
+      const double nh = f < 32 ? fma(h, (double)(f + 1), lo) : hi;
+      lo = f > 0 ? fma(h, (double)f, lo) : lo;
+      hi = nh;
+    }
+    // an interval that holds zero at the rounding level of the norm is zero
+    const double mid = (lo <= 0.0 && hi >= 0.0) ? 0.0 : 0.5 * (lo + hi);
+    if (lane == 0) ext[warp] = ldexp(mid, ex);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    const double lo = ext[0], hi = ext[1];
     const double lam = nes_lambda_of(hi, lo);
     st->L = hi;
     st->mu = lo;
@@ -937,162 +964,250 @@ __global__ void __cluster_dims__(NES_CTAS, 1, 1) __launch_bounds__(NES_THREADS, 
   if (blockIdx.x == 0 && threadIdx.x == 0) st->steps = t;
 }
 
-// The same loop with every row's state in registers: each warp holds up to
-// R rows (row0 + r * 128); no global traffic inside the loop, and the R
-// matrix-vector products of a step are interleaved. Used when the mode has at
-// most R * 128 rows.
+// The same loop with every row's state in registers, for modes whose rows fit
+// the cluster. A warp holds R groups of rows, 32 / KP rows a group at KP = 16
+// and one above, lane c of a row holding column c (and c + 32 at KP = 64).
+//
+// A step is bound by latencies (a row's k dependent fused multiply-adds, the
+// exchange of the stopping test over the cluster), not by a unit, so:
+//  * the test is a yes or no (any entry with |grad .* acc| > 1e-2 or grad <
+//    -1e-2; NaN counts as passed, as in a max / min), one bit a step, and S
+//    steps run before the cluster exchanges their bits: the steps past the
+//    one that ends the loop are speculative, and the result is recomputed
+//    from the state kept (in shared memory) at the start of its S steps;
+//  * the exchange of one group of S steps travels while the next S steps run;
+//  * a row's acc reaches its lanes as broadcast 16-byte shared-memory loads
+//    (two shuffles per entry would bound the loop), a lane's column of
+//    G + lambda I stays in registers where it fits (GREG);
+//  * the step lengths beta, a chain of a square root and a division a step,
+//    come from one extra warp, S steps ahead.
+// Values and step counts are those of the one-step loop, which took 205 us a
+// call at 200 x 150 x 120, k = 16 (FP64), against 41 us.
 template <int KP, int R>
-__global__ void __launch_bounds__(NES_THREADS, 1)
+struct NesReg {
+  static constexpr int LPR = KP < 32 ? KP : 32;   // lanes of a row
+  static constexpr int RW = 32 / LPR;             // rows of a group
+  static constexpr int PER = KP / LPR;            // columns of a lane
+  static constexpr int S = R <= 2 ? 4 : 2;        // steps per exchange
+  static constexpr bool GREG = KP == 16 || (KP == 32 && R <= 2);
+  // warps that hold rows: 15 beside the step-length warp leave 128 registers
+  // a thread (room for the column of G + lambda I), 16 leave 96
+  static constexpr int NW = R <= 2 ? NES_THREADS / 32 - 1 : NES_THREADS / 32;
+  static constexpr int THREADS = (NW + 1) * 32;
+  static constexpr int64_t ROWS = (int64_t)NW * RW * R;         // rows of a CTA
+  static constexpr size_t ACC = (size_t)NW * R * RW * KP;       // row vectors
+  static constexpr size_t KEEP = (size_t)4 * R * PER * NW * 32; // two kept states
+  static constexpr size_t SMEM = (ACC + KEEP + (GREG ? 0 : (size_t)KP * KP)) * sizeof(double);
+};
+
+template <int KP, int R>
+__global__ void __launch_bounds__(NesReg<KP, R>::THREADS, 1)
     k_nes_inner_reg(double* __restrict__ Ht_out, const double* __restrict__ prox,
                     double* __restrict__ prev, const double* __restrict__ M,
                     const double* __restrict__ G, NesDev* __restrict__ st, int64_t I, int k,
                     int max_steps, int* __restrict__ status) {
-  constexpr int PER = KP / 32;
-  constexpr int NW = NES_THREADS / 32;
+  using C = NesReg<KP, R>;
+  constexpr int PER = C::PER, NW = C::NW, S = C::S;
   cg::cluster_group cluster = cg::this_cluster();
-  __shared__ double Gs[KP * KP];
-  __shared__ double wmax[NW], wmin[NW];
-  __shared__ double slot[2][NES_CTAS_MAX][2];  // pushed by every CTA, read locally
+  extern __shared__ __align__(16) double nes_sm[];
+  double* arow = nes_sm;                 // [warp][group][row of the group][KP]
+  double* keep = arow + C::ACC;          // [parity][ht, acc][group][PER][thread]
+  double* Gs = keep + C::KEEP;           // !GREG: G + lambda I, k x k at stride KP
+  __shared__ double betas[4][S];
+  __shared__ unsigned wmask[2][NW];
+  __shared__ unsigned slot[2][NES_CTAS_MAX];  // pushed by every CTA, read locally
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ncta = (int)cluster.num_blocks(), me = (int)cluster.block_rank();
   const double lam = st->lambda, q = st->q, inv = st->inv;
-  for (int e = threadIdx.x; e < k * k; e += NES_THREADS)
-    Gs[e] = G[e] + ((e / k) == (e % k) ? lam : 0.0);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t stride = (int64_t)gridDim.x * NW;
-  const int64_t row0 = (int64_t)blockIdx.x * NW + warp;
+  const bool holder = warp < NW;         // the last warp forms the step lengths
+  const int c0 = lane % C::LPR, half = lane / C::LPR;
+  auto g_at = [&](int j, int c) {
+    return (j < k && c < k) ? G[j * k + c] + (j == c ? lam : 0.0) : 0.0;
+  };
+  if constexpr (!C::GREG) {
+    for (int e = tid; e < KP * KP; e += C::THREADS) Gs[e] = g_at(e / KP, e % KP);
+  }
+  double greg[C::GREG ? KP : 1];
+  if constexpr (C::GREG) {
+#pragma unroll
+    for (int j = 0; j < KP; ++j) greg[j] = g_at(j, c0);
+  }
   double ht[R][PER], acc[R][PER], gr[R][PER], mm[R][PER];
   bool live[R][PER];
+  // rows go round the CTAs, so that every CTA holds as many
+  auto row_of = [&](int r) {
+    return ((int64_t)(r * NW + warp) * ncta + me) * C::RW + half;
+  };
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t row = row0 + r * stride;
+  for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int p = 0; p < PER; ++p) {
-      const int c = lane + 32 * p;
-      live[r][p] = row < I && c < k;
+      const int64_t row = row_of(r);
+      const int c = c0 + 32 * p;
+      live[r][p] = holder && row < I && c < k;
       const double h0 = live[r][p] ? prox[row * k + c] : 0.0;
       ht[r][p] = h0;
       acc[r][p] = h0;
       mm[r][p] = live[r][p] ? (-1 * lam) * h0 - M[row * k + c] : 0.0;
+      gr[r][p] = 0.0;
       if (live[r][p]) prev[row * k + c] = h0;
     }
-  }
-  double vmax, vmin;
-  // grad = modM + (G + lambda I) acc for every held row, and the stopping
-  // test's max |grad .* acc| and min grad over them
+  const bool working = __any_sync(0xffffffffu, live[0][0]);  // the warp's first group has rows
+  double* my_rows = arow + (size_t)(holder ? warp : 0) * R * C::RW * KP;
+  // gr = mm + (G + lambda I) acc for every held row (sums over j in order)
   auto all_grads = [&]() {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int p = 0; p < PER; ++p) my_rows[(r * C::RW + half) * KP + c0 + 32 * p] = acc[r][p];
+    __syncwarp();
     double g[R][PER];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int p = 0; p < PER; ++p) g[r][p] = 0.0;
-    for (int j = 0; j < k; ++j) {
-      double gv[PER];
 #pragma unroll
-      for (int p = 0; p < PER; ++p) {
-        const int c = lane + 32 * p;
-        gv[p] = c < k ? Gs[j * k + c] : 0.0;
-      }
+    for (int j = 0; j < KP; j += 4) {
+      if (j < k) {
+        double gv[4][PER];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const double aj = __shfl_sync(0xffffffffu, slot_get<PER>(acc[r], j >> 5), j & 31);
+        for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int p = 0; p < PER; ++p) g[r][p] = fma(aj, gv[p], g[r][p]);
-      }
-    }
-    vmax = 0.0;
-    vmin = INFINITY;
+          for (int p = 0; p < PER; ++p) {
+            if constexpr (C::GREG)
+              gv[u][p] = greg[j + u];
+            else
+              gv[u][p] = Gs[(j + u) * KP + c0 + 32 * p];
+          }
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R; ++r) {
+          const double2* a = reinterpret_cast<const double2*>(my_rows + (r * C::RW + half) * KP + j);
+          const double2 a0 = a[0], a1 = a[1];
 #pragma unroll
-      for (int p = 0; p < PER; ++p) {
-        gr[r][p] = mm[r][p] + g[r][p];
-        if (live[r][p]) {
-          vmax = fmax(vmax, fabs(gr[r][p] * acc[r][p]));
-          vmin = fmin(vmin, gr[r][p]);
+          for (int p = 0; p < PER; ++p) {
+            g[r][p] = fma(a0.x, gv[0][p], g[r][p]);
+            g[r][p] = fma(a0.y, gv[1][p], g[r][p]);
+            g[r][p] = fma(a1.x, gv[2][p], g[r][p]);
+            g[r][p] = fma(a1.y, gv[3][p], g[r][p]);
+          }
         }
       }
-  };
-  all_grads();
-
-  // Each step's cluster barrier is split: after a CTA has pushed its max /
-  // min it arrives, forms the next step speculatively (the same arithmetic
-  // the loop would do next), and only then waits; when the test says stop,
-  // the step's iterate saved before the speculation is the result. The
-  // barrier's latency overlaps a step's math; the values are unchanged.
-  double alpha = 1.0, beta = 1.0;
-  int t = 0;
-  double hsave[R][PER];
-  cluster.sync();  // every CTA of the cluster running before remote stores
-  for (;;) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-      vmin = fmin(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
     }
-    if (lane == 0) {
-      wmax[warp] = vmax;
-      wmin[warp] = vmin;
-    }
-    __syncthreads();
-    if (warp == 0) {  // CTA max / min over the warps, pushed to every CTA
-      double m = lane < NW ? wmax[lane] : 0.0, n = lane < NW ? wmin[lane] : INFINITY;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        n = fmin(n, __shfl_xor_sync(0xffffffffu, n, o));
-      }
-      if (lane < (int)cluster.num_blocks()) {
-        double* dst = cluster.map_shared_rank(&slot[t & 1][cluster.block_rank()][0], lane);
-        dst[0] = m;
-        dst[1] = n;
-      }
-    }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    // speculative step t + 1
-    const double alpha_n = nes_alpha_of(alpha, q);
-    const double beta_n = (alpha * (1 - alpha)) / (alpha_n + alpha * alpha);
+    __syncwarp();  // the rows are read before the next step replaces them
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int p = 0; p < PER; ++p) {
-        hsave[r][p] = ht[r][p];
+      for (int p = 0; p < PER; ++p) gr[r][p] = mm[r][p] + g[r][p];
+  };
+  auto step = [&](double beta) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int p = 0; p < PER; ++p)
         if (live[r][p]) {
           const double hprev = ht[r][p];
           const double v = acc[r][p] - (inv * gr[r][p]);
           const double hn = v > 0.0 ? v : 0.0;
-          acc[r][p] = hn + beta_n * (hn - hprev);
+          acc[r][p] = hn + beta * (hn - hprev);
           ht[r][p] = hn;
         }
-      }
     all_grads();
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    double gmax = 0.0, gmin = INFINITY;
-    for (unsigned r = 0; r < cluster.num_blocks(); ++r) {
-      gmax = fmax(gmax, slot[t & 1][r][0]);
-      gmin = fmin(gmin, slot[t & 1][r][1]);
-    }
-    const bool stop = gmax <= 1e-2 && gmin >= -1e-2;  // stop_iter, ntfnes.hpp:52-62
-    if (stop || t >= max_steps) {
-      if (!stop && blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(status, 0, kStMaxIter);
+  };
+  auto kept = [&](int par, int what, int r, int p) -> double& {
+    return keep[(((size_t)par * 2 + what) * R * PER + r * PER + p) * (NW * 32) + tid];
+  };
+  double alpha = 1.0;
+  auto next_betas = [&](int b) {  // ntfnes.hpp:143-145, the last warp
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int p = 0; p < PER; ++p) ht[r][p] = hsave[r][p];
-      break;
+    for (int s = 0; s < S; ++s) {
+      const double an = nes_alpha_of(alpha, q);
+      const double beta = (alpha * (1 - alpha)) / (an + alpha * alpha);
+      if (lane == 0) betas[b][s] = beta;
+      alpha = an;
     }
-    ++t;
-    alpha = alpha_n;
-    beta = beta_n;
+  };
+  if constexpr (!C::GREG) __syncthreads();
+  if (working) all_grads();
+  if (!holder) next_betas(0);
+  cluster.sync();  // every CTA runs before remote stores; the first betas are there
+  int stop_at = 0;   // the step of group `stop_grp` whose state is the result
+  int stop_grp = 0;
+  for (int grp = 0;; ++grp) {
+    if (holder) {
+      unsigned bits = 0;
+      if (working) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int p = 0; p < PER; ++p) {
+            kept(grp & 1, 0, r, p) = ht[r][p];
+            kept(grp & 1, 1, r, p) = acc[r][p];
+          }
+#pragma unroll 1
+        for (int s = 0; s < S; ++s) {
+          bool open = false;  // this state does not pass the stopping test
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int p = 0; p < PER; ++p)
+              open |= live[r][p] && (fabs(gr[r][p] * acc[r][p]) > 1e-2 || gr[r][p] < -1e-2);
+          bits |= open ? 1u << s : 0u;
+          step(betas[grp & 3][s]);
+        }
+        bits = __reduce_or_sync(0xffffffffu, bits);
+      }
+      if (lane == 0) wmask[grp & 1][warp] = bits;
+    } else {
+      next_betas((grp + 1) & 3);
+    }
+    if (grp > 0) {  // the previous group's exchange is complete
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      unsigned open = 0;
+      for (int b = 0; b < ncta; ++b) open |= slot[(grp - 1) & 1][b];
+      const int first = __ffs(~open) - 1;  // first state that passes (bits >= S are clear)
+      const int t0 = (grp - 1) * S;
+      if (first < S && first <= max_steps - t0) {  // stop_iter, ntfnes.hpp:52-62
+        stop_at = first;
+        stop_grp = grp - 1;
+        break;
+      }
+      if (max_steps - t0 < S) {
+        stop_at = max_steps - t0;
+        stop_grp = grp - 1;
+        if (me == 0 && tid == 0) atomicCAS(status, 0, kStMaxIter);
+        break;
+      }
+    }
+    __syncthreads();
+    if (tid < ncta) {
+      unsigned m = 0;
+      for (int w = 0; w < NW; ++w) m |= wmask[grp & 1][w];
+      *cluster.map_shared_rank(&slot[grp & 1][me], tid) = m;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   }
-  (void)beta;
+  if (!holder) return;
+  if (working) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int p = 0; p < PER; ++p) {
+        ht[r][p] = kept(stop_grp & 1, 0, r, p);
+        acc[r][p] = kept(stop_grp & 1, 1, r, p);
+      }
+    if (stop_at > 0) {
+      all_grads();
+      for (int s = 0; s < stop_at; ++s) step(betas[stop_grp & 3][s]);
+    }
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int64_t row = row0 + r * stride;
+    const int64_t row = row_of(r);
 #pragma unroll
     for (int p = 0; p < PER; ++p)
-      if (live[r][p]) Ht_out[row * k + lane + 32 * p] = ht[r][p];
+      if (live[r][p]) Ht_out[row * k + c0 + 32 * p] = ht[r][p];
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->steps = t;
+  if (me == 0 && tid == 0) st->steps = stop_grp * S + stop_at;
 }
 
 // After the mode's normalisation: prox = the normalised factor, and for the

@@ -148,3 +148,20 @@ def test_nesterov_step_cap_reports_maxiter(gpu, monkeypatch, dims):
         c.set_factors(F0)
         e = c.run("nesterov", 3)
     assert np.all(np.isfinite(e))
+
+
+# edges of the register-resident Nesterov shapes: ranks 1 and 2 (no reflection
+# in the eigenvalue bounds), either side of the lane groups (16 / 17, 32 / 33),
+# row counts one past a shape's capacity over 16 CTAs (480 and 240 rows)
+@pytest.mark.parametrize("dims,k", [((12, 9, 10), 1), ((12, 9, 10), 2), ((40, 30, 17), 16),
+                                    ((481, 18, 17), 16), ((241, 19, 18), 17), ((481, 33, 34), 32),
+                                    ((66, 35, 34), 33)])
+def test_nesterov_register_shapes(gpu, oracle_lib, dims, k):
+    X, _ = cp_tensor(dims, k, noise=0.01, seed=65)
+    F0 = init_factors(dims, k, seed=66)
+    Fo, lamo, eo = oracle_lib.ntf_run(X, F0, "nesterov", 8, dimtree=True)
+    F, lam, e = _run(gpu, X, F0, "nesterov", 8)
+    assert rel(e, eo) < TOL, (e, eo)
+    for a, b in zip(F, Fo):
+        assert rel(a, b) < TOL
+    assert rel(lam, lamo) < TOL

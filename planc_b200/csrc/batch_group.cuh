@@ -10,7 +10,7 @@
 // past a member's own grid return at once.
 #pragma once
 #include "kernels_f64.cuh"
-#include "updates_iter.cuh"
+#include "mode_cluster.cuh"
 
 namespace pg {
 
@@ -38,23 +38,11 @@ __global__ void __launch_bounds__(256) k_grp_mu(const GrpUpd* __restrict__ a, do
   mu_warp_body<KP>(u.H, u.M, u.G, u.I, u.k, eps, blockIdx.x);
 }
 
-// normalisation + Gram + next leave-one-out product (k_normgram_cluster); the
-// launch's cluster spans x and has the largest member's size
-struct GrpNg {
-  double* F;
-  int64_t I;
-  int k;
-  double* lambda;
-  double* Gall;
-  int N, n, next;
-  double* Gloo;
-  int CLm;  // the member's own cluster size
-};
-
-template <int BE>
-__global__ void __launch_bounds__(NGC_THREADS, 1) k_grp_normgram(const GrpNg* __restrict__ a) {
-  const GrpNg& g = a[blockIdx.z];
-  normgram_cluster_body<BE>(g.F, g.I, g.k, g.lambda, g.Gall, g.N, g.n, g.next, g.Gloo, g.CLm);
+// normalisation + Grams (+ error) of one factor (k_mode_cluster); the launch's
+// cluster spans x and has the largest member's size
+template <int KP>
+__global__ void __launch_bounds__(MODE_THREADS) k_grp_mode(const ModeArgs* __restrict__ a) {
+  mode_cluster_body<KP, MODE_NONE>(a[blockIdx.z]);
 }
 
 // left multi-TTV of the FP32 intermediate (k_ttv_left<float> / k_ttv_left_f4)
@@ -116,24 +104,6 @@ __global__ void k_grp_reduce(const GrpRed* __restrict__ a) {
   const GrpRed& g = a[blockIdx.z];
   if (blockIdx.x >= g.gx) return;
   reduce_splits_body(g.part, g.nsplit, g.stride, g.n, g.out, blockIdx.x, g.gx);
-}
-
-// Gram-form relative error (k_error)
-struct GrpErr {
-  const double* Mlast;
-  const double* Flast;
-  int64_t I;
-  const double* lambda;
-  const double* Gall;
-  int N, k;
-  const double* normX2;
-  double* errs;
-  int* counter;
-};
-
-__global__ void __launch_bounds__(1024) k_grp_error(const GrpErr* __restrict__ a) {
-  const GrpErr& g = a[blockIdx.z];
-  error_body(g.Mlast, g.Flast, g.I, g.lambda, g.Gall, g.N, g.k, g.normX2, g.errs, g.counter);
 }
 
 }  // namespace pg

@@ -1,0 +1,393 @@
+// mode_cluster.cuh -- the end of one factor's step of the outer iteration in
+// one cluster launch: [HALS or MU row update, rank <= 16] -> normalisation ->
+// Gram -> next leave-one-out product -> [relative error].
+//
+// Reference: NTFHALS / NTFMU::update (ntf/ntfhals.hpp:13-29, ntf/ntfmu.hpp:
+// 11-16), NCPFactors::normalize(int) (common/ncpfactors.hpp:346-351), the Gram
+// of the normalised factor and the leave-one-out product
+// (common/ncpfactors.hpp:139-148), AUNTF::computeObjectiveError
+// (ntf/auntf.hpp:200-246).
+//
+// What bounds it: a factor is small (I x k doubles), so nothing but the chain
+// of dependent steps counts -- launches, trips to L2, barriers, a row's k
+// dependent column steps. So the rows stay in shared memory from the update to
+// the normalised store, and everything between is one launch.
+//
+// Layout: a cluster of up to 16 CTAs splits the rows evenly, 64 (16 above rank
+// 32) or more a CTA. U^T U of a CTA's rows is summed row by row in increasing
+// order, one upper-triangle block of outputs a thread (the transposed outputs
+// have the same products in the same order), and over the cluster in rank
+// order: the sums, hence the bits, depend on I and k alone, not on the launch
+// (alone, or a member of a grouped launch) nor on how the threads share it.
+// The update gives a row to 4 lanes, each holding 4 columns in pairs, so that a
+// warp carries 8 rows through the recurrence at once; G is read as 16-byte
+// loads and only the step's change travels by shuffle. Its sums run in the
+// order of the one-row-per-warp kernels (the same bits). Above rank 16 the
+// loads of G by 16 SMs would cost more than the launch they save (at 1024 rows,
+// rank 32: 4.4 us for k_hals_warp over the whole GPU), so the update stays a
+// launch of its own there.
+// Measured a mode: 64^3 rank 8, HALS and error included, 6.8 us (2.2 + 8.8 as
+// two launches, and 4.7 a sweep for the error's own); without the update, at
+// 333 rows of rank 20, 8.8 us with the error (9.5, and 6.4 for the error), at
+// 1024 rows of rank 32 10.9 us (12.0 and 9.4).
+#pragma once
+#include "common.cuh"
+#include "updates_iter.cuh"
+
+namespace pg {
+
+enum ModeUpdate { MODE_NONE = 0, MODE_HALS = 1, MODE_MU = 2 };
+
+constexpr int MODE_THREADS = 256;
+constexpr int64_t MODE_MAX_ROWS = 4096;
+constexpr int MODE_MAX_CL = 16;
+
+struct ModeArgs {
+  double* F;             // I x k: the factor, replaced by the normalised update
+  const double* M;       // MTTKRP of the mode, I x k (update and error)
+  int64_t I;
+  int k;
+  double eps;            // MU
+  double* lambda;
+  double* Gall;          // N x k x k Grams
+  int N, n, next;        // updated mode; mode whose leave-one-out product is formed (-1: none)
+  double* Gloo;          // in: leave-one-out product of mode n; out: of mode next
+  int CLm;               // CTAs that hold rows (<= the cluster's size)
+  const double* normX2;  // relative error after the update (errs null: none)
+  double* errs;
+  int* counter;
+};
+
+template <int KP>
+struct ModeShape {
+  static constexpr int LPR = 4;                     // lanes of a row in the update
+  static constexpr int CP = KP / LPR;               // columns of a lane
+  static constexpr int RPW = 32 / LPR;              // rows of a warp
+  static constexpr int CHUNK = RPW * (MODE_THREADS / 32);
+  static constexpr int LDH = KP + 2;                // row stride: conflict-free 16-byte rows
+  static constexpr int BE = KP == 16 ? 1 : KP == 32 ? 2 : 4;  // edge of a thread's block of outputs
+  static constexpr int KB = KP / BE;                // blocks per edge: KB (KB + 1) / 2 <= 256 threads
+};
+
+// CTAs of a factor's cluster: one per 64 rows (16 above rank 32, where a
+// row's outer product is four times the work)
+__host__ __device__ constexpr int mode_ctas(int64_t I, int k, int most) {
+  const int64_t rpc = k > 32 ? 16 : 64;
+  const int64_t c = (I + rpc - 1) / rpc;
+  return (int)(c < 1 ? 1 : c > most ? most : c);
+}
+
+// dynamic shared memory for `rows` rows a CTA
+template <int KP>
+constexpr size_t mode_smem_bytes(int64_t rows) {
+  using S = ModeShape<KP>;
+  return ((size_t)rows * S::LDH + (KP == 16 ? (size_t)S::CHUNK * S::LDH : 0) + 2 * (size_t)KP * KP) *
+         sizeof(double);
+}
+inline size_t mode_smem(int k, int64_t rows) {
+  return k <= 16 ? mode_smem_bytes<16>(rows) : k <= 32 ? mode_smem_bytes<32>(rows) : mode_smem_bytes<64>(rows);
+}
+
+template <int KP, int UPD>
+__device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
+  using S = ModeShape<KP>;
+  constexpr int LPR = S::LPR, CP = S::CP, LDH = S::LDH, CHUNK = S::CHUNK;
+  static_assert(UPD == MODE_NONE || KP == 16, "the fused update is for ranks up to 16");
+  cg::cluster_group cluster = cg::this_cluster();
+  const int me = (int)cluster.block_rank(), CLm = a.CLm;
+  const int k = a.k, kk2 = k * k;
+  const int64_t I = a.I;
+  extern __shared__ __align__(16) double mode_sm[];
+  const int64_t per = (I + CLm - 1) / CLm;
+  const int64_t r0 = me < CLm ? (int64_t)me * per : I;
+  const int64_t r1 = (r0 + per) < I ? (r0 + per) : I;
+  const int nrows = (int)(r1 > r0 ? r1 - r0 : 0);
+  double* gs = mode_sm;                    // G of the update; later the factor's U^T U
+  double* gsum = gs + KP * KP;             // U^T U of this CTA's rows
+  double* tile = gsum + KP * KP;           // rows at stride LDH
+  double* mt = tile + (size_t)per * LDH;   // CHUNK rows of M (update)
+  __shared__ double lam[KP];
+  __shared__ double red[MODE_THREADS / 32];
+  __shared__ double inner_sum;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool err = a.errs != nullptr;
+
+  // ---- stage G and the rows (columns past k as zeros)
+  if constexpr (UPD != MODE_NONE) {
+    for (int e = tid; e < KP * KP; e += MODE_THREADS) {
+      const int i = e / KP, j = e % KP;
+      gs[e] = (i < k && j < k) ? a.Gloo[i * k + j] : 0.0;
+    }
+  }
+  {
+    const double* F0 = a.F + r0 * k;
+    for (int e = tid; e < nrows * KP; e += MODE_THREADS) {
+      const int i = e / KP, c = e % KP;
+      tile[i * LDH + c] = c < k ? F0[i * k + c] : 0.0;
+    }
+  }
+  if constexpr (UPD != MODE_NONE) {
+    for (int ch = 0; ch < nrows; ch += CHUNK) {
+      const int nr = (nrows - ch) < CHUNK ? (nrows - ch) : CHUNK;
+      if (ch > 0) __syncthreads();  // the previous chunk's M is read
+      const double* M0 = a.M + (r0 + ch) * k;
+      for (int e = tid; e < nr * KP; e += MODE_THREADS) {
+        const int i = e / KP, c = e % KP;
+        mt[i * LDH + c] = c < k ? M0[i * k + c] : 0.0;
+      }
+      __syncthreads();  // M, and for the first chunk G and the rows
+      const int q = lane % LPR;
+      const int row = ch + warp * S::RPW + lane / LPR;  // this lane's row
+      if (ch + warp * S::RPW < nrows) {
+        const bool live = row < nrows;
+        // lanes past the last row shadow the warp's first one
+        double* hrow = tile + (size_t)(live ? row : ch + warp * S::RPW) * LDH;
+        double g[CP], h[CP];
+#pragma unroll
+        for (int s = 0; s < CP; ++s) g[s] = 0.0;
+#pragma unroll 2
+        for (int j = 0; j < k; j += 2) {
+          const double2 hj = *reinterpret_cast<const double2*>(hrow + j);
+#pragma unroll
+          for (int p = 0; p < CP / 2; ++p) {
+            const double2 ga = *reinterpret_cast<const double2*>(gs + j * KP + p * 2 * LPR + 2 * q);
+            const double2 gb = *reinterpret_cast<const double2*>(gs + (j + 1) * KP + p * 2 * LPR + 2 * q);
+            g[2 * p] = fma(hj.y, gb.x, fma(hj.x, ga.x, g[2 * p]));
+            g[2 * p + 1] = fma(hj.y, gb.y, fma(hj.x, ga.y, g[2 * p + 1]));
+          }
+        }
+#pragma unroll
+        for (int p = 0; p < CP / 2; ++p) {
+          const double2 v = *reinterpret_cast<const double2*>(hrow + p * 2 * LPR + 2 * q);
+          h[2 * p] = v.x;
+          h[2 * p + 1] = v.y;
+        }
+        const double* mrow = mt + (size_t)(live ? row - ch : warp * S::RPW) * LDH;
+        if constexpr (UPD == MODE_HALS) {
+          double m[CP];
+#pragma unroll
+          for (int p = 0; p < CP / 2; ++p) {
+            const double2 v = *reinterpret_cast<const double2*>(mrow + p * 2 * LPR + 2 * q);
+            m[2 * p] = v.x;
+            m[2 * p + 1] = v.y;
+          }
+          // columns in order; column i's lane forms the new entry, its
+          // change reaches the row's other lanes by one shuffle, and every
+          // later column's H G takes it in
+#pragma unroll
+          for (int p = 0; p < CP / 2; ++p)
+#pragma unroll
+            for (int o = 0; o < LPR; ++o)
+#pragma unroll
+              for (int b = 0; b < 2; ++b) {
+                const int i = p * 2 * LPR + 2 * o + b;
+                if (i < k) {
+                  double u = h[2 * p + b] + (m[2 * p + b] - g[2 * p + b]);
+                  u = (u < kEps17) ? kEps17 : u;
+                  const double delta = __shfl_sync(0xffffffffu, u - h[2 * p + b], o, LPR);
+                  if (q == o) h[2 * p + b] = u;
+#pragma unroll
+                  for (int p2 = p; p2 < CP / 2; ++p2) {
+                    const double2 gi = *reinterpret_cast<const double2*>(gs + i * KP + p2 * 2 * LPR + 2 * q);
+                    g[2 * p2] = fma(delta, gi.x, g[2 * p2]);
+                    g[2 * p2 + 1] = fma(delta, gi.y, g[2 * p2 + 1]);
+                  }
+                }
+              }
+        } else {
+#pragma unroll
+          for (int p = 0; p < CP / 2; ++p)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              const int i = p * 2 * LPR + 2 * q + b;
+              if (i < k) h[2 * p + b] = (h[2 * p + b] * mrow[i]) / (g[2 * p + b] + a.eps);
+            }
+        }
+        __syncwarp();  // every lane of the row has read the old values
+        if (live)
+#pragma unroll
+          for (int p = 0; p < CP / 2; ++p) {
+            const int c = p * 2 * LPR + 2 * q;
+            if (c < k) hrow[c] = h[2 * p];
+            if (c + 1 < k) hrow[c + 1] = h[2 * p + 1];
+          }
+        __syncwarp();
+      }
+    }
+  }
+  __syncthreads();  // the (updated) rows
+  if (err) {  // <M, U> over this CTA's rows
+    double inner = 0.0;
+    const double* M0 = a.M + r0 * k;
+    for (int e = tid; e < nrows * k; e += MODE_THREADS) {
+      const int i = e / k, c = e - i * k;
+      inner = fma(M0[e], tile[i * LDH + c], inner);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) inner += __shfl_xor_sync(0xffffffffu, inner, o);
+    if (lane == 0) red[warp] = inner;
+    __syncthreads();
+    if (tid == 0) {
+      double s = 0.0;
+      for (int w = 0; w < MODE_THREADS / 32; ++w) s += red[w];
+      inner_sum = s;
+    }
+  }
+
+  // ---- U^T U of this CTA's rows: a BE x BE block of the upper triangle a
+  // thread, rows in increasing order
+  {
+    constexpr int BE = S::BE, KB = S::KB;
+    // block t of the triangle: row ta, column tb >= ta
+    int ta = 0, t0 = 0;
+    while (ta < KB && t0 + (KB - ta) <= tid) {
+      t0 += KB - ta;
+      ++ta;
+    }
+    const int tb = ta + (tid - t0);
+    if (ta < KB && BE * ta < k) {
+      double acc[BE][BE];
+#pragma unroll
+      for (int u = 0; u < BE; ++u)
+#pragma unroll
+        for (int v = 0; v < BE; ++v) acc[u][v] = 0.0;
+#pragma unroll 4
+      for (int i = 0; i < nrows; ++i) {
+        const double* r = tile + (size_t)i * LDH;
+        double av[BE], bv[BE];
+        if constexpr (BE == 1) {
+          av[0] = r[ta];
+          bv[0] = r[tb];
+        } else {
+#pragma unroll
+          for (int u = 0; u < BE; u += 2) {
+            const double2 x = *reinterpret_cast<const double2*>(r + BE * ta + u);
+            const double2 y = *reinterpret_cast<const double2*>(r + BE * tb + u);
+            av[u] = x.x;
+            av[u + 1] = x.y;
+            bv[u] = y.x;
+            bv[u + 1] = y.y;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < BE; ++u)
+#pragma unroll
+          for (int v = 0; v < BE; ++v) acc[u][v] = fma(av[u], bv[v], acc[u][v]);
+      }
+#pragma unroll
+      for (int u = 0; u < BE; ++u)
+#pragma unroll
+        for (int v = 0; v < BE; ++v) {
+          gsum[(BE * ta + u) * KP + BE * tb + v] = acc[u][v];
+          gsum[(BE * tb + v) * KP + BE * ta + u] = acc[u][v];
+        }
+    }
+    __syncthreads();
+  }
+
+  // ---- the factor's U^T U in every CTA: partials summed in rank order
+  const double* gram = gsum;
+  if (cluster.num_blocks() > 1) {
+    cluster.sync();
+    gram = gs;
+    if constexpr (KP == 16) {
+      // every CTA reads every partial: few entries, one exchange
+      for (int e = tid; e < k * KP && me < CLm; e += MODE_THREADS) {
+        double v[MODE_MAX_CL];
+#pragma unroll
+        for (int b = 0; b < MODE_MAX_CL; ++b) v[b] = b < CLm ? *cluster.map_shared_rank(gsum + e, b) : 0.0;
+        double t = v[0];
+#pragma unroll
+        for (int b = 1; b < MODE_MAX_CL; ++b)
+          if (b < CLm) t += v[b];
+        gs[e] = t;
+      }
+      __syncthreads();
+    } else {
+      // CTA c sums slice c and stores it into every CTA's copy
+      const int ne = k * KP, sl = (ne + CLm - 1) / CLm;
+      const int e0 = me * sl, e1 = me < CLm ? ((e0 + sl) < ne ? (e0 + sl) : ne) : 0;
+      for (int e = e0 + tid; e < e1; e += MODE_THREADS) {
+        double v[MODE_MAX_CL];
+#pragma unroll
+        for (int b = 0; b < MODE_MAX_CL; ++b) v[b] = b < CLm ? *cluster.map_shared_rank(gsum + e, b) : 0.0;
+        double t = v[0];
+#pragma unroll
+        for (int b = 1; b < MODE_MAX_CL; ++b)
+          if (b < CLm) t += v[b];
+#pragma unroll
+        for (int b = 0; b < MODE_MAX_CL; ++b)
+          if (b < CLm) *cluster.map_shared_rank(gs + e, b) = t;
+      }
+      cluster.sync();
+    }
+  }
+  double inner_all = 0.0;
+  if (err && me == 0 && tid == 0)
+    for (int b = 0; b < CLm; ++b) inner_all += *cluster.map_shared_rank(&inner_sum, b);
+  // no CTA reads another's shared memory from here on; a CTA may leave once
+  // all have come this far
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (me < CLm) {
+    if (tid < k) lam[tid] = sqrt(gram[tid * KP + tid]);
+    __syncthreads();
+    // normalised rows
+    double* F0 = a.F + r0 * k;
+    for (int e = tid; e < nrows * k; e += MODE_THREADS) {
+      const int i = e / k, c = e - i * k;
+      const double nrm = lam[c], u = tile[i * LDH + c];
+      F0[e] = nrm > 0 ? u / nrm : u;
+    }
+    if (me == 0 && tid < k && a.lambda) a.lambda[tid] = lam[tid];
+    // G_n and the leave-one-out product of mode `next`: a slice per CTA
+    const int sl = (kk2 + CLm - 1) / CLm;
+    const int e0 = me * sl, e1 = (e0 + sl) < kk2 ? (e0 + sl) : kk2;
+    double* Gn = a.Gall + (int64_t)a.n * kk2;
+    for (int e = e0 + tid; e < e1; e += MODE_THREADS) {
+      const int i = e / k, j = e - i * k;
+      const double la = lam[i], lb = lam[j], s = gram[i * KP + j];
+      const double gn = (la > 0 && lb > 0) ? s / (la * lb) : s;
+      Gn[e] = gn;
+      if (a.next >= 0) {
+        double g = 1.0;
+        for (int m = 0; m < a.N; ++m)
+          if (m != a.next) g = g * (m == a.n ? gn : a.Gall[(int64_t)m * kk2 + e]);
+        a.Gloo[e] = g;
+      }
+    }
+    if (err && me == 0) {
+      // ||X||^2 - 2 <M, U> + sum_ab lambda_a lambda_b prod_m G_m[a, b], with
+      // lambda_a lambda_b G_n[a, b] = (U^T U)_ab
+      double mn = 0.0;
+      for (int e = tid; e < kk2; e += MODE_THREADS) {
+        const int i = e / k, j = e - i * k;
+        const double la = lam[i], lb = lam[j];
+        double g = (la > 0 && lb > 0) ? gram[i * KP + j] : 0.0;
+        for (int m = 0; m < a.N; ++m)
+          if (m != a.n) g = g * a.Gall[(int64_t)m * kk2 + e];
+        mn += g;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mn += __shfl_xor_sync(0xffffffffu, mn, o);
+      if (lane == 0) red[warp] = mn;
+      __syncthreads();
+      if (tid == 0) {
+        double t = 0.0;
+        for (int w = 0; w < MODE_THREADS / 32; ++w) t += red[w];
+        const double nx = *a.normX2;
+        const double e2 = nx - 2.0 * inner_all + t;
+        const int c = *a.counter;
+        a.errs[c] = sqrt(fabs(e2) / nx);
+        *a.counter = c + 1;
+      }
+    }
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int KP, int UPD>
+__global__ void __launch_bounds__(MODE_THREADS, 1) k_mode_cluster(const __grid_constant__ ModeArgs a) {
+  mode_cluster_body<KP, UPD>(a);
+}
+
+}  // namespace pg

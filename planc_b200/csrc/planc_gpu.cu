@@ -24,6 +24,7 @@
 #include "tc_mttkrp.cuh"
 #include "nmf.cuh"
 #include "updates_iter.cuh"
+#include "mode_cluster.cuh"
 #include "batch_group.cuh"
 #include "tc_group.cuh"
 
@@ -86,7 +87,7 @@ struct planc_gpu_ctx {
   bool own_stream = false;
   int sm_count = 148;
   size_t smem_optin = 0;     // dynamic shared memory the cooperative W sweep may use
-  int ngc_ctas = 0;          // largest cluster of k_normgram_cluster (0: not used)
+  int mode_ctas = 0;         // largest cluster of k_mode_cluster (0: not used)
   int nes_max_steps = NES_MAX_STEPS;  // step cap of the Nesterov inner loop
   bool coop_launch = false;  // device takes cooperative launches
 
@@ -385,9 +386,18 @@ bool enable_nes16() {
   return enable_cluster16(k_nes_inner_reg<KP, R>, NesReg<KP, R>::THREADS, NesReg<KP, R>::SMEM);
 }
 
-template <int BE>
-int ngc_cluster_size_of() {
-  auto kern = k_normgram_cluster<BE>;
+// Dynamic shared memory a k_mode_cluster launch may use.
+constexpr size_t kModeSmemMax = 220 * 1024;
+
+// Attributes of one instance (or its grouped form), and its largest cluster
+// on the current device: 16, 8 or 0.
+template <typename Kern>
+int mode_cluster_size_of(Kern kern) {
+  if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kModeSmemMax) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
   for (int cl : {16, 8}) {
     if (cl == 16 &&
         cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
@@ -395,15 +405,10 @@ int ngc_cluster_size_of() {
       cudaGetLastError();
       continue;
     }
-    if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)ngc_smem_bytes(64)) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)cl, 1, 1);
-    cfg.blockDim = dim3(NGC_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = ngc_smem_bytes(64);
+    cfg.blockDim = dim3(MODE_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = kModeSmemMax;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)cl;
@@ -421,11 +426,36 @@ int ngc_cluster_size_of() {
   return 0;
 }
 
-// Cluster size of k_normgram_cluster on the current device: 16 where clusters
-// of 16 fit, else 8 where 8 fit, else 0 (the three-launch form).
-int ngc_cluster_size() {
-  const int a = ngc_cluster_size_of<2>(), b = ngc_cluster_size_of<4>();
-  return a < b ? a : b;
+// Largest cluster every instance runs with on `dev` (the current device),
+// found once per device: 0 leaves the separate launches.
+std::mutex g_mode_attr_mutex;
+int g_mode_ctas[64];
+bool g_mode_known[64] = {false};
+int mode_cluster_size(int dev) {
+  std::lock_guard<std::mutex> lock(g_mode_attr_mutex);
+  if (dev >= 0 && dev < 64 && g_mode_known[dev]) return g_mode_ctas[dev];
+  int m = 16;
+  for (auto kern : {k_mode_cluster<16, MODE_NONE>, k_mode_cluster<16, MODE_HALS>, k_mode_cluster<16, MODE_MU>,
+                    k_mode_cluster<32, MODE_NONE>, k_mode_cluster<64, MODE_NONE>})
+    m = std::min(m, mode_cluster_size_of(kern));
+  for (auto kern : {k_grp_mode<32>, k_grp_mode<64>}) m = std::min(m, mode_cluster_size_of(kern));
+  if (dev >= 0 && dev < 64) {
+    g_mode_ctas[dev] = m;
+    g_mode_known[dev] = true;
+  }
+  return m;
+}
+
+// Whether a factor of I rows takes the one-launch form, with CL its cluster.
+bool mode_fits(const planc_gpu_ctx* c, int64_t I, int k, int* CL) {
+  if (c->mode_ctas <= 0 || I > MODE_MAX_ROWS) return false;
+  *CL = mode_ctas(I, k, c->mode_ctas);
+  return mode_smem(k, (I + *CL - 1) / *CL) <= kModeSmemMax;
+}
+
+// The fixed-order sum of nsplit split-K partials in scratch.
+void split_sum(planc_gpu_ctx* c, int nsplit, int64_t stride, int64_t n, double* out) {
+  launch(c, KC_REDUCE, [&] { reduce_splits(c->stream, c->scratch, nsplit, stride, n, out); });
 }
 
 WGen make_wgen(planc_gpu_ctx* c, const std::vector<int>& modes) {
@@ -679,12 +709,7 @@ void run_contract(planc_gpu_ctx* c, const ContractPlan& p, bool left, const doub
 #undef CASE
     }
   });
-  if (p.nsplit > 1) {
-    int64_t n = p.g.M * k;
-    launch(c, KC_REDUCE, [&] {
-      reduce_splits(c->stream, c->scratch, p.nsplit, p.g.split_stride, n, out);
-    });
-  }
+  if (p.nsplit > 1) split_sum(c, p.nsplit, p.g.split_stride, p.g.M * k, out);
 }
 
 template <typename TT>
@@ -703,12 +728,7 @@ void run_ttv_right(planc_gpu_ctx* c, const TT* T, int64_t A, int64_t B, const WG
       default: k_ttv_right_tiled<TT, 64><<<p.grid, 256, 0, c->stream>>>(T, A, B, k, wg, p.bper, dst); break;
     }
   });
-  if (p.nsplit > 1) {
-    int64_t n = A * k;
-    launch(c, KC_REDUCE, [&] {
-      reduce_splits(c->stream, c->scratch, p.nsplit, n, n, out);
-    });
-  }
+  if (p.nsplit > 1) split_sum(c, p.nsplit, A * k, A * k, out);
 }
 
 template <typename TT>
@@ -842,8 +862,7 @@ void mttkrp_direct_tc(planc_gpu_ctx* c, int n, double* out) {
     launch(c, KC_CONTRACT_LEFT, [&] {
       nsplit = tc_long(t, true, c->k, out, c->scratch, c->status_dev, eff_sm(c), c->stream);
     });
-    if (nsplit > 1)
-      launch(c, KC_REDUCE, [&] { reduce_splits(c->stream, c->scratch, nsplit, nn, nn, out); });
+    if (nsplit > 1) split_sum(c, nsplit, nn, nn, out);
     return;
   }
   if (tc_scratch_elems(t, eff_sm(c), c->k) > c->scratch_elems)
@@ -852,7 +871,7 @@ void mttkrp_direct_tc(planc_gpu_ctx* c, int n, double* out) {
   launch(c, KC_CONTRACT_LEFT, [&] {
     nsplit = tc_left(t, wg, c->k, c->scratch, c->status_dev, eff_sm(c), c->stream, c->left_chunks);
   });
-  launch(c, KC_REDUCE, [&] { reduce_splits(c->stream, c->scratch, nsplit, nn, nn, out); });
+  split_sum(c, nsplit, nn, nn, out);
 }
 
 // Direct MTTKRP of mode n (common/tensor.hpp:246-327): FP64 contraction, or
@@ -923,10 +942,8 @@ void partial_left(planc_gpu_ctx* c, double* out) {
       nsplit = tc_left(c->tct, wg, c->k, c->scratch, c->status_dev, eff_sm(c), c->stream,
                        c->left_chunks);
     });
-    int64_t n = c->R * c->k;
-    launch(c, KC_REDUCE, [&] {
-      reduce_splits(c->stream, c->scratch, nsplit, n, n, out);
-    });
+    const int64_t n = c->R * c->k;
+    split_sum(c, nsplit, n, n, out);
   }
 }
 
@@ -941,12 +958,8 @@ void long_contract(planc_gpu_ctx* c, bool left, const std::vector<int>& modes, d
   launch(c, left ? KC_CONTRACT_LEFT : KC_CONTRACT, [&] {
     nsplit = tc_long(c->tct, left, c->k, out, c->scratch, c->status_dev, eff_sm(c), c->stream);
   });
-  if (nsplit > 1) {
-    const int64_t n = (left ? c->R : c->L) * c->k;
-    launch(c, KC_REDUCE, [&] {
-      reduce_splits(c->stream, c->scratch, nsplit, n, n, out);
-    });
-  }
+  const int64_t n = (left ? c->R : c->L) * c->k;
+  if (nsplit > 1) split_sum(c, nsplit, n, n, out);
 }
 
 // MTTKRP of mode n on the balanced 4-way tree {0,1} | {2,3} (tensor-core
@@ -995,9 +1008,7 @@ void mttkrp_dimtree(planc_gpu_ctx* c, int n, double* out) {
                        c->stream, c->tc_cpa);
         });
         const int64_t nn = c->dims[0] * c->k;
-        launch(c, KC_REDUCE, [&] {
-          reduce_splits(c->stream, c->scratch, ns, nn, nn, out);
-        });
+        split_sum(c, ns, nn, nn, out);
         return;
       }
     }
@@ -1185,37 +1196,72 @@ void nes_post(planc_gpu_ctx* c, int n) {
   });
 }
 
-void normalize_gram(planc_gpu_ctx* c, int n, int next, double* lambda) {
+ModeArgs mode_args(planc_gpu_ctx* c, int n, int next, double* lambda, bool err, int CL) {
+  ModeArgs a{};
+  a.F = c->F[n];
+  a.M = c->M[n];
+  a.I = c->dims[n];
+  a.k = c->k;
+  a.eps = kEps6;
+  a.lambda = lambda ? lambda : c->lam_tmp;
+  a.Gall = c->Gall;
+  a.N = c->N;
+  a.n = n;
+  a.next = next;
+  a.Gloo = c->Gloo;
+  a.CLm = CL;
+  if (err) {
+    a.normX2 = c->normX2;
+    a.errs = c->errs_dev;
+    a.counter = c->counter_dev;
+  }
+  return a;
+}
+
+template <typename Kern, typename Arg>
+void launch_mode(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const Arg& arg) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(MODE_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = grid.x;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, kern, arg));
+}
+
+// One launch of k_mode_cluster (the caller checked mode_fits).
+void run_mode(planc_gpu_ctx* c, int upd, const ModeArgs& a) {
+  const size_t smem = mode_smem(c->k, (a.I + a.CLm - 1) / a.CLm);
+  const dim3 grid((unsigned)a.CLm, 1, 1);
+  launch(c, upd == MODE_NONE ? KC_NORMGRAM : KC_UPDATE, [&] {
+    if (c->k <= 16) {
+      if (upd == MODE_HALS) launch_mode(k_mode_cluster<16, MODE_HALS>, grid, smem, c->stream, a);
+      else if (upd == MODE_MU) launch_mode(k_mode_cluster<16, MODE_MU>, grid, smem, c->stream, a);
+      else launch_mode(k_mode_cluster<16, MODE_NONE>, grid, smem, c->stream, a);
+    } else if (c->k <= 32) {
+      launch_mode(k_mode_cluster<32, MODE_NONE>, grid, smem, c->stream, a);
+    } else {
+      launch_mode(k_mode_cluster<64, MODE_NONE>, grid, smem, c->stream, a);
+    }
+  });
+}
+
+void error_kernel(planc_gpu_ctx* c);
+
+// Normalisation, Gram and the next leave-one-out product of factor n; with
+// `err` the relative error of the iteration follows (n the last mode, its
+// MTTKRP in M[n]).
+void normalize_gram(planc_gpu_ctx* c, int n, int next, double* lambda, bool err = false) {
   const int64_t I = c->dims[n];
-  // one cluster launch per factor, a CTA per 64 rows (16 rows above rank 32,
-  // where a row's outer product is four times the work) up to the largest
-  // cluster: the size depends on I and k alone, so every context (a batch
-  // member too) sums a factor's Gram in the same order, and small factors
-  // take small clusters that run beside other contexts' kernels
-  if (I <= NGC_MAX_ROWS && c->ngc_ctas > 0) {
-    double* lam = lambda ? lambda : c->lam_tmp;
-    const int64_t rpc = c->k > 32 ? 16 : NGC_TILE;
-    const int cl = (int)std::min<int64_t>(c->ngc_ctas, std::max<int64_t>(1, (I + rpc - 1) / rpc));
-    launch(c, KC_NORMGRAM, [&] {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)cl, 1, 1);
-      cfg.blockDim = dim3(NGC_THREADS, 1, 1);
-      cfg.dynamicSmemBytes = ngc_smem_bytes(c->k);
-      cfg.stream = c->stream;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = (unsigned)cl;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      if (c->k <= 32)
-        CK(cudaLaunchKernelEx(&cfg, k_normgram_cluster<2>, c->F[n], I, c->k, lam, c->Gall, c->N,
-                              n, next, c->Gloo));
-      else
-        CK(cudaLaunchKernelEx(&cfg, k_normgram_cluster<4>, c->F[n], I, c->k, lam, c->Gall, c->N,
-                              n, next, c->Gloo));
-    });
+  int CL = 0;
+  if (mode_fits(c, I, c->k, &CL)) {
+    run_mode(c, MODE_NONE, mode_args(c, n, next, lambda, err, CL));
     return;
   }
   const int rpb = gram_rows_per_block(I);
@@ -1235,6 +1281,7 @@ void normalize_gram(planc_gpu_ctx* c, int n, int next, double* lambda) {
     k_scale_cols<<<(unsigned)std::min<int64_t>((ne + 255) / 256, 2048), 256, 0, c->stream>>>(
         c->F[n], I, c->k, lam);
   });
+  if (err) error_kernel(c);
 }
 
 void gram_loo(planc_gpu_ctx* c, int n) {
@@ -1307,13 +1354,22 @@ void nes_accelerate(planc_gpu_ctx* c, bool dimtree) {
 // One AUNTF outer iteration (ntf/auntf.hpp:131-170); `accel` appends the
 // Nesterov acceleration step (auntf.hpp:171).
 void one_iteration(planc_gpu_ctx* c, int algo, bool dimtree, bool err, bool accel = false) {
+  const bool sweep = algo == PLANC_GPU_HALS || algo == PLANC_GPU_MU;
   for (int n = 0; n < c->N; ++n) {
+    const int next = (n + 1) % c->N;
+    const bool last_err = err && n == c->N - 1;
+    int CL = 0;
     mttkrp_any(c, n, dimtree, c->M[n]);
+    if (sweep && c->k <= 16 && mode_fits(c, c->dims[n], c->k, &CL)) {
+      // update, normalisation, Grams and error in one launch
+      run_mode(c, algo == PLANC_GPU_HALS ? MODE_HALS : MODE_MU,
+               mode_args(c, n, next, c->lambda, last_err, CL));
+      continue;
+    }
     run_update(c, algo, n);
-    normalize_gram(c, n, (n + 1) % c->N, c->lambda);
+    normalize_gram(c, n, next, c->lambda, last_err);
     if (algo == PLANC_GPU_NESTEROV) nes_post(c, n);
   }
-  if (err) error_kernel(c);
   if (accel) nes_accelerate(c, dimtree);
 }
 
@@ -1547,7 +1603,7 @@ int planc_gpu_create(planc_gpu_ctx** out, int device, int precision, void* cuda_
     c->precision = precision;
     c->sm_count = prop.multiProcessorCount;
     c->smem_optin = nmfc_smem_limit(prop.sharedMemPerBlockOptin);
-    c->ngc_ctas = ngc_cluster_size();
+    c->mode_ctas = mode_cluster_size(device);
     // PLANC_GPU_NES_MAX_STEPS lowers the Nesterov inner loop's step cap for
     // contexts created while it is set (1 .. NES_MAX_STEPS)
     if (const char* e = getenv("PLANC_GPU_NES_MAX_STEPS")) {
@@ -2532,7 +2588,7 @@ void batch_capture(planc_gpu_batch* b, int algo, bool err) {
 
 // ---------------------------------------------------------------- grouped phases
 // A batch whose members are all 3-way tensor-core contexts running MU or HALS
-// on the dimension tree (factors of at most NGC_MAX_ROWS rows) runs each
+// on the dimension tree (factors of at most MODE_MAX_ROWS rows) runs each
 // outer iteration as phases: the tensor-core contractions of every member on
 // the worker streams (one per member, as before), and every other step of
 // the iteration -- the multi-TTVs, split-K sums, factor updates,
@@ -2544,9 +2600,10 @@ void batch_capture(planc_gpu_batch* b, int algo, bool err) {
 bool batch_groupable(const planc_gpu_batch* b, int algo) {
   if (!b->group || (algo != PLANC_GPU_HALS && algo != PLANC_GPU_MU)) return false;
   for (auto* m : b->members) {
-    if (m->N != 3 || m->precision == PLANC_GPU_PREC_FP64 || m->bal4 || m->ngc_ctas <= 0) return false;
+    int CL;
+    if (m->N != 3 || m->precision == PLANC_GPU_PREC_FP64 || m->bal4) return false;
     for (int n = 0; n < 3; ++n)
-      if (m->dims[n] > NGC_MAX_ROWS) return false;
+      if (!mode_fits(m, m->dims[n], m->k, &CL)) return false;
   }
   return true;
 }
@@ -2592,13 +2649,24 @@ GrpRed grp_red(const double* part, int nsplit, int64_t n, double* out) {
   return GrpRed{part, nsplit, n, n, out, reduce_blocks(nsplit, n)};
 }
 
-// run_update for every member (MU / HALS, one warp per row)
-void grp_update(GrpTables& tab, cudaStream_t st, const std::vector<planc_gpu_ctx*>& ms, int algo, int n) {
+// The update, then normalisation, Grams and (last mode, err) error of one mode
+// for every member: run_update and normalize_gram in two launches (the cluster
+// spans the largest member's CTAs).
+void grp_mode(GrpTables& tab, cudaStream_t st, const std::vector<planc_gpu_ctx*>& ms, int algo, int n,
+              bool err) {
   std::vector<GrpUpd> u32, u64;
+  std::vector<ModeArgs> v[2];
+  size_t smem[2] = {};
+  unsigned cls[2] = {};
   for (auto* m : ms) {
     const int64_t I = m->dims[n];
-    GrpUpd u{m->F[n], m->M[n], m->Gloo, I, m->k, (unsigned)((I + 7) / 8)};
-    (m->k <= 32 ? u32 : u64).push_back(u);
+    int CL = 0;
+    if (!mode_fits(m, I, m->k, &CL)) fail(PLANC_GPU_ERR_STATE, "internal: grouped factor too large");
+    (m->k <= 32 ? u32 : u64).push_back(GrpUpd{m->F[n], m->M[n], m->Gloo, I, m->k, (unsigned)((I + 7) / 8)});
+    const int ki = m->k <= 32 ? 0 : 1;
+    v[ki].push_back(mode_args(m, n, (n + 1) % 3, m->lambda, err, CL));
+    smem[ki] = std::max(smem[ki], mode_smem(ki ? 64 : 32, (I + CL - 1) / CL));
+    cls[ki] = std::max(cls[ki], (unsigned)CL);
   }
   if (!u32.empty()) {
     const dim3 g(grp_max(u32, &GrpUpd::gx), 1, (unsigned)u32.size());
@@ -2611,43 +2679,13 @@ void grp_update(GrpTables& tab, cudaStream_t st, const std::vector<planc_gpu_ctx
     else k_grp_mu<64><<<g, 256, 0, st>>>(tab.put(u64), kEps6);
   }
   grp_check(cudaGetLastError());
-}
-
-// normalize_gram(n, next, lambda) for every member (its cluster path)
-void grp_normgram(GrpTables& tab, cudaStream_t st, const std::vector<planc_gpu_ctx*>& ms, int n, int next) {
-  std::vector<GrpNg> g2, g4;
-  int cl2 = 1, cl4 = 1;
-  for (auto* m : ms) {
-    const int64_t I = m->dims[n];
-    const int64_t rpc = m->k > 32 ? 16 : NGC_TILE;
-    const int cl = (int)std::min<int64_t>(m->ngc_ctas, std::max<int64_t>(1, (I + rpc - 1) / rpc));
-    GrpNg g{m->F[n], I, m->k, m->lambda, m->Gall, m->N, n, next, m->Gloo, cl};
-    if (m->k <= 32) {
-      g2.push_back(g);
-      cl2 = std::max(cl2, cl);
-    } else {
-      g4.push_back(g);
-      cl4 = std::max(cl4, cl);
-    }
+  for (int ki = 0; ki < 2; ++ki) {
+    if (v[ki].empty()) continue;
+    const dim3 grid(cls[ki], 1, (unsigned)v[ki].size());
+    const ModeArgs* t = tab.put(v[ki]);
+    if (ki == 0) launch_mode(k_grp_mode<32>, grid, smem[ki], st, t);
+    else launch_mode(k_grp_mode<64>, grid, smem[ki], st, t);
   }
-  auto go = [&](auto kern, const std::vector<GrpNg>& v, int cl, int kp) {
-    if (v.empty()) return;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)cl, 1, (unsigned)v.size());
-    cfg.blockDim = dim3(NGC_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = ngc_smem_bytes(kp);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    grp_check(cudaLaunchKernelEx(&cfg, kern, tab.put(v)));
-  };
-  go(k_grp_normgram<2>, g2, cl2, 32);
-  go(k_grp_normgram<4>, g4, cl4, 64);
 }
 
 void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
@@ -2775,8 +2813,7 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
       grp_check(cudaGetLastError());
     }
     grp_reduce(tab, st, red);
-    grp_update(tab, st, ms, algo, 0);
-    grp_normgram(tab, st, ms, 0, 1);
+    grp_mode(tab, st, ms, algo, 0, false);
     // ---- mode 1: M_1 = TTV of P with the updated F_0 (run_ttv_left<float>)
     {
       std::vector<GrpTtvL> plain, f4;
@@ -2798,8 +2835,7 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
             tab.put(f4));
       grp_check(cudaGetLastError());
     }
-    grp_update(tab, st, ms, algo, 1);
-    grp_normgram(tab, st, ms, 1, 2);
+    grp_mode(tab, st, ms, algo, 1, false);
     // ---- mode 2: M_2 = X^T KRP(F_0, F_1) per member (split-K partials), then the sums
     // one grouped launch per (rank class, row tiles per CTA) for the generic
     // left contractions; the factored ones (I_0 % 64 == 0) keep their own
@@ -2869,16 +2905,7 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
     }
     join();
     grp_reduce(tab, st, red);
-    grp_update(tab, st, ms, algo, 2);
-    grp_normgram(tab, st, ms, 2, 0);
-    if (err) {
-      std::vector<GrpErr> e;
-      for (auto* m : ms)
-        e.push_back(GrpErr{m->M[2], m->F[2], m->dims[2], m->lambda, m->Gall, m->N, m->k, m->normX2,
-                           m->errs_dev, m->counter_dev});
-      k_grp_error<<<dim3(1, 1, (unsigned)e.size()), 1024, 0, st>>>(tab.put(e));
-      grp_check(cudaGetLastError());
-    }
+    grp_mode(tab, st, ms, algo, 2, err);
     for (auto* m : ms) m->capturing = false;
   } catch (...) {
     for (auto* m : ms) m->capturing = false;
@@ -2937,15 +2964,6 @@ int planc_gpu_batch_create(planc_gpu_batch** out, int device, int precision, int
     // PLANC_GPU_BATCH_GROUPED=0: per-member launches only (no grouped phases)
     if (const char* e = getenv("PLANC_GPU_BATCH_GROUPED")) b->group = strcmp(e, "0") != 0;
     try {
-      // the grouped normalisation + Gram runs clusters of up to 16 CTAs with
-      // up to 64 KB of dynamic shared memory (as k_normgram_cluster)
-      for (auto kern : {k_grp_normgram<2>, k_grp_normgram<4>}) {
-        if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess)
-          cudaGetLastError();
-        CK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)ngc_smem_bytes(64)));
-      }
       CK(cudaStreamCreateWithFlags(&b->master, cudaStreamNonBlocking));
       CK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
       for (int i = 0; i < nstreams; ++i) {

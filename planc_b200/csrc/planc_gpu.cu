@@ -353,7 +353,7 @@ void launch_cluster(void (*kern)(KArgs...), int ncta, int threads, size_t smem, 
 // Allows `smem` bytes of dynamic shared memory and clusters of 16 for `kern`
 // and reports whether such a cluster fits on the device.
 template <typename... KArgs>
-bool enable_cluster16(void (*kern)(KArgs...), int threads = NES_THREADS, size_t smem = 0) {
+bool enable_cluster16(void (*kern)(KArgs...), int threads, size_t smem) {
   if (smem)
     CK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
@@ -1092,8 +1092,8 @@ void run_update(planc_gpu_ctx* c, int algo, int n) {
     if (!c->admm_ready) fail(PLANC_GPU_ERR_STATE, "internal: AO-ADMM state not allocated");
     // NTFAOADMM::update (ntf/ntfaoadmm.hpp:23-77): Cholesky of G + alpha I,
     // at most admm_iter = 5 ADMM iterations, then the dual variable is
-    // normalised. Up to 1024 rows (rank <= 32) or 512 rows (rank <= 64): one
-    // cluster launch with the rows in registers.
+    // normalised. Up to 2048 rows (rank <= 32) or 1024 rows (rank <= 64) on
+    // clusters of 16: one cluster launch.
     const int64_t warps = (int64_t)c->cl_ctas * (NES_THREADS / 32);
     const int64_t rpw = (I + warps - 1) / warps;
     if ((k <= 32 && rpw <= 8) || rpw <= 4) {
@@ -1453,11 +1453,13 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
   if ((algo == PLANC_GPU_AOADMM || algo == PLANC_GPU_NESTEROV) && !c->admm_ready &&
       !c->nes_ready) {
     // clusters of 16 where every register-resident kernel accepts them
-    bool ok = true;
-    ok = ok && enable_cluster16(k_admm_cluster<32, 1>) && enable_cluster16(k_admm_cluster<32, 2>);
-    ok = ok && enable_cluster16(k_admm_cluster<32, 4>) && enable_cluster16(k_admm_cluster<32, 8>);
-    ok = ok && enable_cluster16(k_admm_cluster<64, 1>) && enable_cluster16(k_admm_cluster<64, 2>);
-    ok = ok && enable_cluster16(k_admm_cluster<64, 4>);
+    bool ok = enable_cluster16(k_admm_cluster<32, 1>, NES_THREADS, 0);
+    ok = enable_cluster16(k_admm_cluster<32, 2>, NES_THREADS, 0) && ok;
+    ok = enable_cluster16(k_admm_cluster<32, 4>, NES_THREADS, 0) && ok;
+    ok = enable_cluster16(k_admm_cluster<32, 8>, NES_THREADS, 0) && ok;
+    ok = enable_cluster16(k_admm_cluster<64, 1>, NES_THREADS, 0) && ok;
+    ok = enable_cluster16(k_admm_cluster<64, 2>, NES_THREADS, 0) && ok;
+    ok = enable_cluster16(k_admm_cluster<64, 4>, NES_THREADS, 0) && ok;
     ok = enable_nes16<16, 1>() && ok;
     ok = enable_nes16<16, 2>() && ok;
     ok = enable_nes16<16, 4>() && ok;

@@ -236,14 +236,25 @@ __global__ void __launch_bounds__(32 * ADMM_WARPS) k_admm_step(
   }
 }
 
-// The whole AO-ADMM update of one mode in one cluster of NES_CTAS CTAs, for
-// modes of at most R * 128 rows (every row's h, u and m in registers):
-// alpha and the Cholesky factor (each CTA computes the same one), at most 5
-// ADMM iterations whose stopping norms are summed per warp, per CTA (warp
-// order) and over the cluster (CTA order) -- the same sums in every CTA, so
-// every CTA takes the same decision -- then the column normalisation of the
-// dual variable with column sums formed the same way. Writes the new factor
-// (unnormalised) and the dual variable.
+// The whole AO-ADMM update of one mode in one cluster, for modes of at most
+// R * 16 rows a CTA (every row's h, u and m in registers): alpha and the
+// Cholesky factor (each CTA computes the same one), at most 5 ADMM iterations
+// whose stopping norms are summed per warp, per CTA (warp order) and over the
+// cluster (CTA order) -- the same sums in every CTA, so every CTA takes the
+// same decision -- then the column normalisation of the dual variable with
+// column sums formed the same way. Writes the new factor (unnormalised) and
+// the dual variable.
+//
+// Bound by latencies: the factor's k dependent columns, a row's 2 k dependent
+// substitution steps an iteration, the exchanges over the cluster. So the
+// factor is formed right-looking over the whole CTA (a thread keeps its
+// entries in registers; two barriers, a square root and a division a column,
+// every entry's subtractions in the order of the left-looking sums), and all
+// 5 iterations run before the cluster exchanges their 5 sets of norms: when
+// an earlier one meets the test (ntfaoadmm.hpp:63-71) the rows start again
+// from global memory and run that many. At 300 / 220 rows of rank 24: 42 / 36 us
+// (50 with a factor formed by dot products of one thread a pivot and an
+// exchange an iteration).
 template <int KP, int R>
 __global__ void __launch_bounds__(NES_THREADS, 1)
     k_admm_cluster(double* __restrict__ H, double* __restrict__ U, const double* __restrict__ M,
@@ -252,111 +263,145 @@ __global__ void __launch_bounds__(NES_THREADS, 1)
   constexpr int PER = KP / 32;
   constexpr int NW = NES_THREADS / 32;
   constexpr int LD = KP + 1;
+  constexpr int ITERS = 5;  // admm_iter, ntfaoadmm.hpp:87
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ double Ls[KP * LD];
-  __shared__ double wred[NW][4];
+  __shared__ double wred[ITERS][NW][4];
   // per-CTA partials pushed into every CTA of the cluster (remote shared-
-  // memory stores before the cluster barrier), read back locally after it
-  __shared__ double slot[2][NES_CTAS_MAX][4];
+  // memory stores before a cluster barrier), read back locally after it
+  __shared__ double slot[NES_CTAS_MAX][ITERS * 4];
+  __shared__ double tot[ITERS * 4];
   static_assert((NW + NES_CTAS_MAX) * KP <= KP * LD, "column partials must fit in Ls");
   __shared__ double rinv[KP];
+  __shared__ double piv[KP];  // the column being eliminated
   __shared__ double s_alpha;
-  __shared__ int s_bad;
   const int tid = threadIdx.x;
   // alpha = trace(G) / k (0.01 if not positive), L = chol(G + alpha I)
-  // (ntfaoadmm.hpp:29-35), left-looking
+  // (ntfaoadmm.hpp:29-35)
+  if (tid < KP) piv[tid] = tid < k ? G[tid * k + tid] : 0.0;
+  __syncthreads();
   if (tid == 0) {
     double tr = 0.0;
-    for (int i = 0; i < k; ++i) tr += G[i * k + i];
+    for (int i = 0; i < k; ++i) tr += piv[i];
     const double a = tr / k;
     s_alpha = (a > 0) ? a : 0.01;
-    s_bad = 0;
   }
   __syncthreads();
   const double alpha = s_alpha;
-  for (int e = tid; e < k * k; e += NES_THREADS) {
-    const int i = e / k, j = e % k;
-    Ls[i * LD + j] = G[e] + (i == j ? alpha : 0.0);
-  }
-  __syncthreads();
-  for (int j = 0; j < k; ++j) {
-    if (tid == 0) {
-      double d = Ls[j * LD + j];
-      for (int p = 0; p < j; ++p) d -= Ls[j * LD + p] * Ls[j * LD + p];
-      if (!(d > 0.0)) s_bad = 1;
-      Ls[j * LD + j] = d > 0.0 ? sqrt(d) : 1.0;
+  {
+    constexpr int TPR = NES_THREADS / KP;  // threads of a row
+    constexpr int E = KP / TPR;            // entries of a thread: columns q, q + TPR, ...
+    const int i = tid / TPR, q = tid % TPR;
+    double v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int c = q + e * TPR;
+      v[e] = (i < k && c <= i) ? G[i * k + c] + (i == c ? alpha : 0.0) : 0.0;
+      if (c == 0) piv[i] = v[e];
     }
     __syncthreads();
-    const double ljj = Ls[j * LD + j];
-    for (int i = j + 1 + tid; i < k; i += NES_THREADS) {
-      double v = Ls[i * LD + j];
-      for (int p = 0; p < j; ++p) v -= Ls[i * LD + p] * Ls[j * LD + p];
-      Ls[i * LD + j] = v / ljj;
+    bool bad = false;
+    for (int j = 0; j < k; ++j) {
+      if (tid < KP) {
+        const double d = piv[j];
+        if (!(d > 0.0)) bad = true;
+        const double ljj = d > 0.0 ? sqrt(d) : 1.0;
+        if (tid > j) Ls[tid * LD + j] = piv[tid] / ljj;
+        // the substitutions multiply by the reciprocal diagonal (as OpenBLAS's
+        // triangular-solve kernels do) instead of dividing on their chain
+        if (tid == j) rinv[j] = 1.0 / ljj;
+      }
+      __syncthreads();
+      if (i > j) {
+        const double l = Ls[i * LD + j];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const int c = q + e * TPR;
+          if (c > j && c <= i) {
+            v[e] = fma(-l, Ls[c * LD + j], v[e]);
+            if (c == j + 1) piv[i] = v[e];
+          }
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    if (bad && blockIdx.x == 0 && tid == 0) atomicCAS(status, 0, kStSingular);
   }
-  if (s_bad && blockIdx.x == 0 && tid == 0) atomicCAS(status, 0, kStSingular);
-  // reciprocal diagonal: the substitutions multiply by it (as OpenBLAS's
-  // triangular-solve kernels do) instead of dividing on the dependency chain
-  if (tid < k) rinv[tid] = 1.0 / Ls[tid * LD + tid];
-  __syncthreads();
 
   const int lane = tid & 31, warp = tid >> 5;
   const int64_t stride = (int64_t)gridDim.x * NW;
   const int64_t row0 = (int64_t)blockIdx.x * NW + warp;
   double h[R][PER], u[R][PER], m[R][PER];
   bool live[R][PER];
+  auto load_rows = [&]() {
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t row = row0 + r * stride;
+    for (int r = 0; r < R; ++r) {
+      const int64_t row = row0 + r * stride;
 #pragma unroll
-    for (int p = 0; p < PER; ++p) {
-      const int c = lane + 32 * p;
-      live[r][p] = row < I && c < k;
-      h[r][p] = live[r][p] ? H[row * k + c] : 0.0;
-      u[r][p] = live[r][p] ? U[row * k + c] : 0.0;
-      m[r][p] = live[r][p] ? M[row * k + c] : 0.0;
+      for (int p = 0; p < PER; ++p) {
+        const int c = lane + 32 * p;
+        live[r][p] = row < I && c < k;
+        h[r][p] = live[r][p] ? H[row * k + c] : 0.0;
+        u[r][p] = live[r][p] ? U[row * k + c] : 0.0;
+        m[r][p] = live[r][p] ? M[row * k + c] : 0.0;
+      }
     }
-  }
-  for (int it = 0; it < 5; ++it) {  // admm_iter, ntfaoadmm.hpp:87
+  };
+  // one ADMM iteration of the held rows (ntfaoadmm.hpp:44-61); s4 takes their
+  // squared norms of the stopping test
+  auto iterate = [&](double (&s4)[4]) {
     double y[R][PER];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int p = 0; p < PER; ++p) y[r][p] = m[r][p] + alpha * (h[r][p] + u[r][p]);
     // forward substitution with L, then back substitution with L^T (the
-    // column orders of dtrsm), all held rows interleaved
+    // column orders of dtrsm), all held rows interleaved; the next step's
+    // entries of L are loaded a step ahead, off the chain
+    double d = rinv[0], l[PER];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) l[p] = Ls[(lane + 32 * p) * LD];
     for (int j = 0; j < k; ++j) {
-      const double d = rinv[j];
+      const double dn = rinv[j + 1 < k ? j + 1 : j];
+      double ln[PER];
+#pragma unroll
+      for (int p = 0; p < PER; ++p) ln[p] = Ls[(lane + 32 * p) * LD + j + 1];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const double yj = __shfl_sync(0xffffffffu, slot_get<PER>(y[r], j >> 5), j & 31) * d;
 #pragma unroll
         for (int p = 0; p < PER; ++p) {
           const int c = lane + 32 * p;
-          if (c == j)
-            y[r][p] = yj;
-          else if (c > j && c < k)
-            y[r][p] -= yj * Ls[c * LD + j];
+          const double t = fma(-yj, l[p], y[r][p]);
+          y[r][p] = c == j ? yj : (c > j && c < k) ? t : y[r][p];
         }
       }
+      d = dn;
+#pragma unroll
+      for (int p = 0; p < PER; ++p) l[p] = ln[p];
     }
+#pragma unroll
+    for (int p = 0; p < PER; ++p) l[p] = Ls[(k - 1) * LD + lane + 32 * p];
     for (int j = k - 1; j >= 0; --j) {
-      const double d = rinv[j];
+      const int jn = j > 0 ? j - 1 : 0;
+      const double dn = rinv[jn];
+      double ln[PER];
+#pragma unroll
+      for (int p = 0; p < PER; ++p) ln[p] = Ls[jn * LD + lane + 32 * p];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const double xj = __shfl_sync(0xffffffffu, slot_get<PER>(y[r], j >> 5), j & 31) * d;
 #pragma unroll
         for (int p = 0; p < PER; ++p) {
           const int c = lane + 32 * p;
-          if (c == j)
-            y[r][p] = xj;
-          else if (c < j)
-            y[r][p] -= xj * Ls[j * LD + c];
+          const double t = fma(-xj, l[p], y[r][p]);
+          y[r][p] = c == j ? xj : c < j ? t : y[r][p];
         }
       }
+      d = dn;
+#pragma unroll
+      for (int p = 0; p < PER; ++p) l[p] = ln[p];
     }
-    double s4[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -374,33 +419,51 @@ __global__ void __launch_bounds__(NES_THREADS, 1)
           h[r][p] = hn;
           u[r][p] = un;
         }
+  };
+  load_rows();
+#pragma unroll 1
+  for (int it = 0; it < ITERS; ++it) {
+    double s4[4] = {0.0, 0.0, 0.0, 0.0};
+    iterate(s4);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
       for (int qd = 0; qd < 4; ++qd) s4[qd] += __shfl_xor_sync(0xffffffffu, s4[qd], o);
     if (lane == 0)
 #pragma unroll
-      for (int qd = 0; qd < 4; ++qd) wred[warp][qd] = s4[qd];
-    __syncthreads();
-    if (tid < (int)cluster.num_blocks()) {
-      double t4[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int w = 0; w < NW; ++w)
-        for (int qd = 0; qd < 4; ++qd) t4[qd] += wred[w][qd];
-      double* dst = cluster.map_shared_rank(&slot[it & 1][cluster.block_rank()][0], tid);
-      for (int qd = 0; qd < 4; ++qd) dst[qd] = t4[qd];
-    }
-    cluster.sync();
-    double tot[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int qd = 0; qd < 4; ++qd) wred[it][warp][qd] = s4[qd];
+  }
+  cluster.sync();  // every CTA runs before remote stores; this CTA's norms are there
+  if (tid < ITERS * 4) {
+    double t = 0.0;
+    for (int w = 0; w < NW; ++w) t += wred[tid >> 2][w][tid & 3];
     for (unsigned b = 0; b < cluster.num_blocks(); ++b)
-      for (int qd = 0; qd < 4; ++qd) tot[qd] += slot[it & 1][b][qd];
-    const double facnorm = sqrt(tot[0]), dualnorm = sqrt(tot[1]);
-    const double rn = sqrt(tot[2]), sn = sqrt(tot[3]);
-    if (rn < tol * facnorm && sn < tol * dualnorm) break;  // ntfaoadmm.hpp:63-71
+      *cluster.map_shared_rank(&slot[cluster.block_rank()][tid], b) = t;
+  }
+  cluster.sync();
+  if (tid < ITERS * 4) {
+    double t = 0.0;
+    for (unsigned b = 0; b < cluster.num_blocks(); ++b) t += slot[b][tid];
+    tot[tid] = t;
+  }
+  __syncthreads();
+  int run = ITERS;  // iterations of the update
+#pragma unroll
+  for (int it = ITERS - 2; it >= 0; --it) {
+    const double facnorm = sqrt(tot[it * 4]), dualnorm = sqrt(tot[it * 4 + 1]);
+    const double rn = sqrt(tot[it * 4 + 2]), sn = sqrt(tot[it * 4 + 3]);
+    if (rn < tol * facnorm && sn < tol * dualnorm) run = it + 1;  // ntfaoadmm.hpp:63-71
+  }
+  if (run < ITERS) {
+    load_rows();
+    double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int it = 0; it < run; ++it) iterate(s4);
   }
   // dual variable column norms (m_ncp_aux.normalize(mode), ntfaoadmm.hpp:74).
-  // Ls is dead in every CTA once all have passed the loop's last cluster
-  // barrier, so its space holds the per-warp column sums and the per-CTA
-  // partials the other CTAs push.
+  // No CTA needs its Ls once all are here, so its space holds the per-warp
+  // column sums and the per-CTA partials the other CTAs push.
+  cluster.sync();
   double(*colw)[KP] = reinterpret_cast<double(*)[KP]>(Ls);
   double(*colpart)[KP] = reinterpret_cast<double(*)[KP]>(Ls + NW * KP);
 #pragma unroll

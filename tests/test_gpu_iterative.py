@@ -165,3 +165,20 @@ def test_nesterov_register_shapes(gpu, oracle_lib, dims, k):
     for a, b in zip(F, Fo):
         assert rel(a, b) < TOL
     assert rel(lam, lamo) < TOL
+
+
+# edges of the AO-ADMM cluster form: one row, one past a row a warp over 16
+# CTAs, the largest and one past it (the launch-per-iteration form), ranks 1,
+# 16 / 17 and 32 / 33
+@pytest.mark.parametrize("dims,k", [((1, 9, 8), 1), ((257, 18, 17), 16), ((40, 19, 18), 17),
+                                    ((60, 35, 34), 32), ((60, 35, 34), 33), ((2048, 6, 5), 4),
+                                    ((2049, 6, 5), 4)])
+def test_admm_cluster_shapes(gpu, oracle_lib, dims, k):
+    X, _ = cp_tensor(dims, k, noise=0.01, seed=67)
+    F0 = init_factors(dims, k, seed=68)
+    Fo, lamo, eo = oracle_lib.ntf_run(X, F0, "aoadmm", 4, dimtree=True)
+    F, lam, e = _run(gpu, X, F0, "aoadmm", 4)
+    assert rel(e, eo) < TOL, (e, eo)
+    for a, b in zip(F, Fo):
+        assert rel(a, b) < TOL
+    assert rel(lam, lamo) < TOL

@@ -138,11 +138,13 @@ def _pd(a):
     return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
+_PD = ctypes.POINTER(ctypes.c_double)
+
+
 def _fptrs(F):
-    arr = (ctypes.POINTER(ctypes.c_double) * len(F))()
-    for i, f in enumerate(F):
-        arr[i] = _pd(f)
-    return arr
+    # addresses of the arrays as a double*[]
+    arr = (ctypes.c_void_p * len(F))(*[f.ctypes.data for f in F])
+    return ctypes.cast(arr, ctypes.POINTER(_PD))
 
 
 def _vps(ptrs):
@@ -230,8 +232,8 @@ class Context:
         return errs[:iters]
 
     def get_factors(self):
-        F = [np.zeros((d, self.k)) for d in self.dims]
-        lam = np.zeros(self.k)
+        F = [np.empty((d, self.k)) for d in self.dims]
+        lam = np.empty(self.k)
         _check(load().planc_gpu_get_factors(self.h, _fptrs(F), _pd(lam)))
         return F, lam
 
@@ -255,13 +257,13 @@ class Context:
         return obj[:iters], rel[:iters]
 
     def nmf_get_factors(self):
-        W, H = np.zeros((self.dims[0], self.k)), np.zeros((self.dims[1], self.k))
+        W, H = np.empty((self.dims[0], self.k)), np.empty((self.dims[1], self.k))
         _check(load().planc_gpu_nmf_get_factors(self.h, _pd(W), _pd(H)))
         return W, H
 
     def mttkrp(self, mode, dimtree=True):
         self.tree_epoch += 1
-        out = np.zeros((self.dims[mode], self.k))
+        out = np.empty((self.dims[mode], self.k))
         _check(load().planc_gpu_mttkrp(self.h, mode, int(dimtree), _pd(out)))
         return out
 
@@ -293,9 +295,9 @@ class Context:
         AtA = _c64(AtA)
         n, ncols = AtB.shape
         B = np.ascontiguousarray(np.asarray(AtB, dtype=np.float64).T)  # column-major n x ncols
-        X = np.zeros((ncols, n))
-        P = np.zeros((ncols, n), dtype=np.int32)
-        it = np.zeros(ncols, dtype=np.int32)
+        X = np.empty((ncols, n))
+        P = np.empty((ncols, n), dtype=np.int32)
+        it = np.empty(ncols, dtype=np.int32)
         _check(load().planc_gpu_bpp_solve(
             self.h, _pd(AtA), _pd(B), n, ncols, _pd(X),
             P.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)),
@@ -417,8 +419,8 @@ class Batch:
 
     def get_factors(self, index):
         dims, k = self.members[index]
-        F = [np.zeros((d, k)) for d in dims]
-        lam = np.zeros(k)
+        F = [np.empty((d, k)) for d in dims]
+        lam = np.empty(k)
         _check(load().planc_gpu_batch_get_factors(self.h, index, _fptrs(F), _pd(lam)))
         return F, lam
 

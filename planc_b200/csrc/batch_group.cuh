@@ -106,4 +106,34 @@ __global__ void k_grp_reduce(const GrpRed* __restrict__ a) {
   reduce_splits_body(g.part, g.nsplit, g.stride, g.n, g.out, blockIdx.x, g.gx);
 }
 
+// Set-up of a run for every member (blockIdx.z): the error counter at 0 and
+// the first leave-one-out product (k_gram_loo); and its results: ne error
+// values and the status word, gathered in member order.
+struct GrpRun {
+  const double* Gall;
+  double* Gloo;
+  int N, k;
+  int* counter;
+  const double* errs;
+  const int* status;
+};
+
+__global__ void __launch_bounds__(256) k_grp_begin(const GrpRun* __restrict__ a) {
+  const GrpRun& r = a[blockIdx.z];
+  if (threadIdx.x == 0) *r.counter = 0;
+  const int kk2 = r.k * r.k;
+  for (int e = threadIdx.x; e < kk2; e += 256) {
+    double g = 1.0;
+    for (int i = 1; i < r.N; ++i) g = g * r.Gall[(int64_t)i * kk2 + e];
+    r.Gloo[e] = g;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_grp_end(const GrpRun* __restrict__ a, int ne,
+                                                 double* __restrict__ errs, int* __restrict__ status) {
+  const GrpRun& r = a[blockIdx.z];
+  for (int e = threadIdx.x; e < ne; e += 256) errs[(int64_t)blockIdx.z * ne + e] = r.errs[e];
+  if (threadIdx.x == 0) status[blockIdx.z] = *r.status;
+}
+
 }  // namespace pg

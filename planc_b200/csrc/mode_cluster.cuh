@@ -390,4 +390,14 @@ __global__ void __launch_bounds__(MODE_THREADS, 1) k_mode_cluster(const __grid_c
   mode_cluster_body<KP, UPD>(a);
 }
 
+// Normalisation and Gram of every factor of a context (blockIdx.z = mode; the
+// cluster spans the largest factor's CTAs).
+struct ModeArgsAll {
+  ModeArgs m[kMaxModes];
+};
+template <int KP>
+__global__ void __launch_bounds__(MODE_THREADS) k_mode_all(const __grid_constant__ ModeArgsAll a) {
+  mode_cluster_body<KP, MODE_NONE>(a.m[blockIdx.z]);
+}
+
 }  // namespace pg

@@ -121,8 +121,16 @@ struct planc_gpu_ctx {
   double* krp_tail = nullptr;    // tail image, rows x k
   size_t krp_tail_elems = 0;
   double* normX2 = nullptr;      // device scalar ||X||^2
+  // the factors and lambda lie in one allocation (fslab: F[0], F[1], ...,
+  // lambda, each 16-byte aligned), so that small ones travel to and from the
+  // host in one copy through hstage
+  double* fslab = nullptr;
+  size_t fslab_elems = 0;
+  size_t lambda_off = 0;
   double* F[kMaxModes] = {nullptr};
   double* M[kMaxModes] = {nullptr};
+  std::vector<double> hstage;
+  cudaEvent_t hstage_read = nullptr;  // the last copy out of hstage
   double* Gall = nullptr;
   double* Gloo = nullptr;
   double* lambda = nullptr;
@@ -135,6 +143,8 @@ struct planc_gpu_ctx {
   double* lam_tmp = nullptr;    // lambda of a normalisation whose lambda is not kept
   double* gram_part = nullptr;  // per-row-block partial Grams
   size_t gram_part_elems = 0;
+  void* bpp_ws = nullptr;       // operands and results of planc_gpu_bpp_solve
+  size_t bpp_ws_bytes = 0;
   double* errs_dev = nullptr;
   int errs_cap = 0;
   int* counter_dev = nullptr;
@@ -223,7 +233,7 @@ struct planc_gpu_ctx {
   // is (re)allocated; cached graphs are rebuilt when it changes.
   int64_t buf_epoch = 0;
   size_t gall_elems = 0;  // capacity of Gall
-  int kvec = 0;           // rank the k-sized buffers (Gloo, lambda, lam_tmp) hold
+  int kvec = 0;           // rank the k-sized buffers (Gloo, lam_tmp) and lambda's place hold
   int64_t g_epoch = -1;
 };
 
@@ -439,6 +449,7 @@ int mode_cluster_size(int dev) {
                     k_mode_cluster<32, MODE_NONE>, k_mode_cluster<64, MODE_NONE>})
     m = std::min(m, mode_cluster_size_of(kern));
   for (auto kern : {k_grp_mode<32>, k_grp_mode<64>}) m = std::min(m, mode_cluster_size_of(kern));
+  for (auto kern : {k_mode_all<16>, k_mode_all<32>, k_mode_all<64>}) m = std::min(m, mode_cluster_size_of(kern));
   if (dev >= 0 && dev < 64) {
     g_mode_ctas[dev] = m;
     g_mode_known[dev] = true;
@@ -1288,6 +1299,34 @@ void gram_loo(planc_gpu_ctx* c, int n) {
   launch(c, KC_NORMGRAM, [&] { k_gram_loo<<<1, 1024, 0, c->stream>>>(c->Gall, c->N, c->k, n, c->Gloo); });
 }
 
+// Normalisation and Gram of every factor (lambda kept): one launch, a cluster
+// per mode, where every factor takes the cluster form.
+void normalize_all(planc_gpu_ctx* c) {
+  ModeArgsAll all{};
+  unsigned cl = 1;
+  size_t smem = 0;
+  bool fits = true;
+  for (int n = 0; n < c->N; ++n) {
+    int CL = 0;
+    fits = fits && mode_fits(c, c->dims[n], c->k, &CL);
+    if (!fits) break;
+    all.m[n] = mode_args(c, n, -1, c->lam_tmp, false, CL);
+    all.m[n].lambda = nullptr;
+    cl = std::max(cl, (unsigned)CL);
+    smem = std::max(smem, mode_smem(c->k, (c->dims[n] + CL - 1) / CL));
+  }
+  if (!fits) {
+    for (int n = 0; n < c->N; ++n) normalize_gram(c, n, -1, nullptr);
+    return;
+  }
+  const dim3 grid(cl, 1, (unsigned)c->N);
+  launch(c, KC_NORMGRAM, [&] {
+    if (c->k <= 16) launch_mode(k_mode_all<16>, grid, smem, c->stream, all);
+    else if (c->k <= 32) launch_mode(k_mode_all<32>, grid, smem, c->stream, all);
+    else launch_mode(k_mode_all<64>, grid, smem, c->stream, all);
+  });
+}
+
 // MTTKRP of the last mode from the current factors (the <X, model> term of
 // the Gram-form error): through the tree from its second root (the state an
 // in-order sweep leaves), or directly.
@@ -1514,6 +1553,44 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
   }
 }
 
+// Largest slab of factors and lambda that goes through one packed copy: above
+// 1 MB the second pass over host memory costs more than the calls it saves.
+constexpr size_t kPackElems = (size_t)1 << 17;
+
+void wait_hstage(planc_gpu_ctx* c) {
+  if (c->hstage_read) CK(cudaEventSynchronize(c->hstage_read));
+}
+
+// Factor, lambda and MTTKRP buffers for the context's shape and rank; any
+// reallocation bumps the buffer epoch.
+void ensure_factor_buffers(planc_gpu_ctx* c) {
+  size_t total = 0, off[kMaxModes + 1];
+  bool same = c->fslab != nullptr;
+  auto even = [](size_t n) { return (n + 1) & ~(size_t)1; };
+  for (int n = 0; n < c->N; ++n) {
+    const size_t need = (size_t)c->dims[n] * c->k;
+    off[n] = total;
+    total += even(need);
+    same = same && c->F[n] == c->fslab + off[n] && c->factor_cap[n] == (int64_t)need;
+  }
+  off[c->N] = total;
+  total += even(c->k);
+  if (same && c->lambda == c->fslab + off[c->N] && c->fslab_elems == total) return;
+  dalloc(&c->fslab, total);
+  c->fslab_elems = total;
+  for (int n = 0; n < c->N; ++n) {
+    c->F[n] = c->fslab + off[n];
+    if (c->factor_cap[n] != (int64_t)c->dims[n] * c->k) {
+      dalloc(&c->M[n], (size_t)c->dims[n] * c->k);
+      c->factor_cap[n] = (int64_t)c->dims[n] * c->k;
+    }
+  }
+  for (int n = c->N; n < kMaxModes; ++n) c->F[n] = nullptr;
+  c->lambda_off = off[c->N];
+  c->lambda = c->fslab + off[c->N];
+  c->buf_epoch++;
+}
+
 void free_all(planc_gpu_ctx* c) {
   free_update_state(c);
   auto f = [](auto*& p) {
@@ -1534,17 +1611,24 @@ void free_all(planc_gpu_ctx* c) {
   f(c->krp_tail);
   c->krp_tail_elems = 0;
   f(c->normX2);
+  f(c->fslab);
+  c->fslab_elems = 0;
   for (int n = 0; n < kMaxModes; ++n) {
-    f(c->F[n]);
+    c->F[n] = nullptr;
     f(c->M[n]);
     c->factor_cap[n] = 0;
   }
+  c->lambda = nullptr;
+  if (c->hstage_read) cudaEventDestroy(c->hstage_read);
+  c->hstage_read = nullptr;
+  if (c->bpp_ws) cudaFree(c->bpp_ws);
+  c->bpp_ws = nullptr;
+  c->bpp_ws_bytes = 0;
   f(c->Gall);
   f(c->gram_part);
   f(c->lam_tmp);
   c->gram_part_elems = 0;
   f(c->Gloo);
-  f(c->lambda);
   f(c->P);
   f(c->P32);
   f(c->Q);
@@ -1837,18 +1921,10 @@ int planc_gpu_set_factors(planc_gpu_ctx* c, const double* const* F, const double
       f(c->Q);
       for (int n = 0; n < kMaxModes; ++n) c->factor_cap[n] = 0;
     }
-    c->k = k;
-    for (int n = 0; n < c->N; ++n) {
+    for (int n = 0; n < c->N; ++n)
       if (!F[n]) fail(PLANC_GPU_ERR_ARG, "null factor");
-      size_t need = (size_t)c->dims[n] * k;
-      if (c->factor_cap[n] != (int64_t)need) {
-        dalloc(&c->F[n], need);
-        dalloc(&c->M[n], need);
-        c->factor_cap[n] = (int64_t)need;
-        c->buf_epoch++;
-      }
-      CK(cudaMemcpyAsync(c->F[n], F[n], need * 8, cudaMemcpyHostToDevice, c->stream));
-    }
+    c->k = k;
+    ensure_factor_buffers(c);
     if (!c->Gall || c->gall_elems != (size_t)c->N * k * k) {
       c->gall_elems = (size_t)c->N * k * k;
       dalloc(&c->Gall, c->gall_elems);
@@ -1866,19 +1942,37 @@ int planc_gpu_set_factors(planc_gpu_ctx* c, const double* const* F, const double
     }
     if (!c->Gloo || c->kvec != k) {
       dalloc(&c->Gloo, (size_t)k * k);
-      dalloc(&c->lambda, (size_t)k);
       dalloc(&c->lam_tmp, (size_t)k);
       c->kvec = k;
       c->buf_epoch++;
     }
-    // AUNTF::reset: update_factor_mode on every mode (normalise, Gram), then
-    // set_lambda(new lambda)
-    for (int n = 0; n < c->N; ++n) normalize_gram(c, n, n == c->N - 1 ? 0 : -1, c->lambda);
-    std::vector<double> lam(k, 1.0);
-    if (lambda) std::copy(lambda, lambda + k, lam.begin());
-    CK(cudaMemcpyAsync(c->lambda, lam.data(), k * 8, cudaMemcpyHostToDevice, c->stream));
+    // Small factors and lambda go in one copy from a packed host buffer of the
+    // context (waited for only before its next use); large ones are copied from
+    // where they are, and waited for (the caller may reuse them on return).
+    const bool packed = c->fslab_elems <= kPackElems;
+    if (packed) {
+      wait_hstage(c);
+      c->hstage.resize(c->fslab_elems);
+      for (int n = 0; n < c->N; ++n)
+        std::memcpy(c->hstage.data() + (c->F[n] - c->fslab), F[n], (size_t)c->dims[n] * k * 8);
+      double* lam = c->hstage.data() + c->lambda_off;
+      if (lambda) std::copy(lambda, lambda + k, lam);
+      else std::fill(lam, lam + k, 1.0);
+      CK(cudaMemcpyAsync(c->fslab, c->hstage.data(), c->fslab_elems * 8, cudaMemcpyHostToDevice, c->stream));
+      if (!c->hstage_read) CK(cudaEventCreateWithFlags(&c->hstage_read, cudaEventDisableTiming));
+      CK(cudaEventRecord(c->hstage_read, c->stream));
+    } else {
+      for (int n = 0; n < c->N; ++n)
+        CK(cudaMemcpyAsync(c->F[n], F[n], (size_t)c->dims[n] * k * 8, cudaMemcpyHostToDevice, c->stream));
+      std::vector<double> lam(k, 1.0);
+      if (lambda) std::copy(lambda, lambda + k, lam.begin());
+      CK(cudaMemcpyAsync(c->lambda, lam.data(), k * 8, cudaMemcpyHostToDevice, c->stream));
+    }
+    // AUNTF::reset: update_factor_mode on every mode (normalise, Gram), with
+    // lambda as set; the first leave-one-out product is formed by its user
+    normalize_all(c);
     ensure_buffers(c);
-    CK(cudaStreamSynchronize(c->stream));
+    if (!packed) CK(cudaStreamSynchronize(c->stream));
     c->have_factors = true;
     c->nmf_have = false;
   });
@@ -1973,6 +2067,17 @@ int planc_gpu_get_factors(planc_gpu_ctx* c, double* const* F, double* lambda) {
   return guarded([&] {
     require_ready(c);
     set_device(c);
+    if (c->fslab_elems <= kPackElems) {  // one copy, as in planc_gpu_set_factors
+      wait_hstage(c);
+      c->hstage.resize(c->fslab_elems);
+      CK(cudaMemcpyAsync(c->hstage.data(), c->fslab, c->fslab_elems * 8, cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      if (F)
+        for (int n = 0; n < c->N; ++n)
+          if (F[n]) std::memcpy(F[n], c->hstage.data() + (c->F[n] - c->fslab), (size_t)c->dims[n] * c->k * 8);
+      if (lambda) std::memcpy(lambda, c->hstage.data() + c->lambda_off, (size_t)c->k * 8);
+      return;
+    }
     if (F)
       for (int n = 0; n < c->N; ++n)
         if (F[n])
@@ -2080,35 +2185,33 @@ int planc_gpu_bpp_solve(planc_gpu_ctx* c, const double* AtA, const double* AtB, 
     if (ncols < 0) fail(PLANC_GPU_ERR_ARG, "ncols < 0");
     if (ncols == 0) return;
     set_device(c);
-    double *dA = nullptr, *dB = nullptr, *dX = nullptr;
-    int *dP = nullptr, *dI = nullptr;
-    auto cleanup = [&] {
-      cudaFree(dA);
-      cudaFree(dB);
-      cudaFree(dX);
-      cudaFree(dP);
-      cudaFree(dI);
-    };
-    try {
-      CK(cudaMalloc(&dA, (size_t)n * n * 8));
-      CK(cudaMalloc(&dB, (size_t)n * ncols * 8));
-      CK(cudaMalloc(&dX, (size_t)n * ncols * 8));
-      CK(cudaMalloc(&dP, (size_t)n * ncols * 4));
-      CK(cudaMalloc(&dI, (size_t)ncols * 4));
-      CK(cudaMemcpyAsync(dA, AtA, (size_t)n * n * 8, cudaMemcpyHostToDevice, c->stream));
-      CK(cudaMemcpyAsync(dB, AtB, (size_t)n * ncols * 8, cudaMemcpyHostToDevice, c->stream));
-      launch(c, KC_BPP, [&] { launch_bpp(c, dA, dB, n, ncols, dX, dP, dI, nullptr); });
-      CK(cudaMemcpyAsync(X, dX, (size_t)n * ncols * 8, cudaMemcpyDeviceToHost, c->stream));
-      if (passive)
-        CK(cudaMemcpyAsync(passive, dP, (size_t)n * ncols * 4, cudaMemcpyDeviceToHost, c->stream));
-      if (iters) CK(cudaMemcpyAsync(iters, dI, (size_t)ncols * 4, cudaMemcpyDeviceToHost, c->stream));
-      check_status(c);
-      drain_timing(c);
-    } catch (...) {
-      cleanup();
-      throw;
+    // one workspace for operands and results, kept by the context: five
+    // allocations and frees a call cost several times the solve
+    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const size_t nA = up((size_t)n * n * 8), nB = up((size_t)n * ncols * 8), nP = up((size_t)n * ncols * 4),
+                 nI = up((size_t)ncols * 4);
+    if (nA + 2 * nB + nP + nI > c->bpp_ws_bytes) {
+      if (c->bpp_ws) cudaFree(c->bpp_ws);
+      c->bpp_ws = nullptr;
+      c->bpp_ws_bytes = 0;
+      CK(cudaMalloc(&c->bpp_ws, nA + 2 * nB + nP + nI));
+      c->bpp_ws_bytes = nA + 2 * nB + nP + nI;
     }
-    cleanup();
+    uint8_t* w = (uint8_t*)c->bpp_ws;
+    double* dA = (double*)w;
+    double* dB = (double*)(w + nA);
+    double* dX = (double*)(w + nA + nB);
+    int* dP = (int*)(w + nA + 2 * nB);
+    int* dI = (int*)(w + nA + 2 * nB + nP);
+    CK(cudaMemcpyAsync(dA, AtA, (size_t)n * n * 8, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(dB, AtB, (size_t)n * ncols * 8, cudaMemcpyHostToDevice, c->stream));
+    launch(c, KC_BPP, [&] { launch_bpp(c, dA, dB, n, ncols, dX, dP, dI, nullptr); });
+    CK(cudaMemcpyAsync(X, dX, (size_t)n * ncols * 8, cudaMemcpyDeviceToHost, c->stream));
+    if (passive)
+      CK(cudaMemcpyAsync(passive, dP, (size_t)n * ncols * 4, cudaMemcpyDeviceToHost, c->stream));
+    if (iters) CK(cudaMemcpyAsync(iters, dI, (size_t)ncols * 4, cudaMemcpyDeviceToHost, c->stream));
+    check_status(c);
+    drain_timing(c);
   });
 }
 
@@ -2517,6 +2620,10 @@ struct planc_gpu_batch {
   uint8_t* grp_dev = nullptr;
   size_t grp_cap = 0;
   bool g_grouped = false;  // the cached graph runs grouped phases
+  const GrpRun* run_args = nullptr;  // in grp_dev: set-up and results of the members
+  double* out_dev = nullptr;         // gathered error histories and status words
+  size_t out_elems = 0;
+  std::vector<double> out_host;
 };
 
 namespace {
@@ -2725,6 +2832,12 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   try {
     for (auto* m : ms) m->capturing = true;
+    {
+      std::vector<GrpRun> r;
+      for (auto* m : ms)
+        r.push_back(GrpRun{m->Gall, m->Gloo, m->N, m->k, m->counter_dev, m->errs_dev, m->status_dev});
+      b->run_args = tab.put(r);
+    }
     // every member's tensor maps: right hi, right lo, left hi, left lo
     std::vector<CUtensorMap> maps(4 * ms.size());
     for (size_t i = 0; i < ms.size(); ++i) {
@@ -2933,19 +3046,52 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
 // per-run set-up of every member (error counters, first leave-one-out Gram),
 // ordered before the graph launches on the master stream
 void batch_prepare(planc_gpu_batch* b) {
-  for (auto* m : b->members) {
-    CK(cudaMemsetAsync(m->counter_dev, 0, sizeof(int), m->stream));
-    gram_loo(m, 0);
-  }
+  if (!b->g_grouped)
+    for (auto* m : b->members) {
+      CK(cudaMemsetAsync(m->counter_dev, 0, sizeof(int), m->stream));
+      gram_loo(m, 0);
+    }
   for (size_t i = 0; i < b->workers.size(); ++i) {
     CK(cudaEventRecord(b->joins[i], b->workers[i]));
     CK(cudaStreamWaitEvent(b->master, b->joins[i], 0));
   }
+  if (b->g_grouped) {
+    k_grp_begin<<<dim3(1, 1, (unsigned)b->members.size()), 256, 0, b->master>>>(b->run_args);
+    CK(cudaGetLastError());
+  }
 }
 
-void batch_finish(planc_gpu_batch* b) {
+// Waits for the run and reports the first member's failure. A grouped batch's
+// status words and (errs not null) error histories come in one copy each way
+// instead of two a member.
+void batch_finish(planc_gpu_batch* b, int iters = 0, double* errs = nullptr) {
+  const size_t n = b->members.size();
+  if (!b->g_grouped) {
+    CK(cudaStreamSynchronize(b->master));
+    for (auto* m : b->members) check_status(m);
+    if (errs)
+      for (size_t i = 0; i < n; ++i)
+        CK(cudaMemcpy(errs + i * iters, b->members[i]->errs_dev, iters * sizeof(double),
+                      cudaMemcpyDeviceToHost));
+    return;
+  }
+  const int ne = errs ? iters : 0;
+  const size_t words = n * ne + (n + 1) / 2;
+  if (b->out_elems < words) {
+    CK(cudaStreamSynchronize(b->master));
+    dalloc(&b->out_dev, words);
+    b->out_elems = words;
+  }
+  k_grp_end<<<dim3(1, 1, (unsigned)n), 256, 0, b->master>>>(b->run_args, ne, b->out_dev,
+                                                           (int*)(b->out_dev + n * ne));
+  CK(cudaGetLastError());
+  b->out_host.resize(words);
+  CK(cudaMemcpyAsync(b->out_host.data(), b->out_dev, words * 8, cudaMemcpyDeviceToHost, b->master));
   CK(cudaStreamSynchronize(b->master));
-  for (auto* m : b->members) check_status(m);
+  const int* st = (const int*)(b->out_host.data() + n * ne);
+  for (size_t i = 0; i < n; ++i)
+    if (st[i] != 0) check_status(b->members[i]);
+  if (errs) std::memcpy(errs, b->out_host.data(), n * ne * sizeof(double));
 }
 
 }  // namespace
@@ -3017,9 +3163,10 @@ int planc_gpu_batch_count(planc_gpu_batch* b) { return b ? (int)b->members.size(
 int planc_gpu_batch_set_factors(planc_gpu_batch* b, int index, const double* const* F, int k) {
   return guarded([&] {
     if (!b || index < 0 || index >= (int)b->members.size()) fail(PLANC_GPU_ERR_ARG, "bad index");
+    // the captured iteration stays valid unless a buffer moved (batch_ensure
+    // compares the members' buffer epochs)
     int rc = planc_gpu_set_factors(b->members[index], F, nullptr, k);
     if (rc != PLANC_GPU_OK) throw Fail{rc};
-    batch_reset_graph(b);
   });
 }
 
@@ -3038,12 +3185,7 @@ int planc_gpu_batch_run(planc_gpu_batch* b, int algo, int iters, int compute_err
     if (!b->gexec || b->g_algo != algo || b->g_err != (int)err) batch_capture(b, algo, err);
     batch_prepare(b);
     for (int it = 0; it < iters; ++it) CK(cudaGraphLaunch(b->gexec, b->master));
-    batch_finish(b);
-    if (err && errs) {
-      for (size_t i = 0; i < b->members.size(); ++i)
-        CK(cudaMemcpy(errs + i * iters, b->members[i]->errs_dev, iters * sizeof(double),
-                      cudaMemcpyDeviceToHost));
-    }
+    batch_finish(b, iters, err ? errs : nullptr);
   });
 }
 
@@ -3165,6 +3307,7 @@ int planc_gpu_batch_destroy(planc_gpu_batch* b) {
     cudaEventDestroy(b->fork);
     cudaStreamDestroy(b->master);
     if (b->grp_dev) cudaFree(b->grp_dev);
+    if (b->out_dev) cudaFree(b->out_dev);
     delete b;
   });
 }
@@ -3584,17 +3727,10 @@ int planc_gpu_nmf_set_factors(planc_gpu_ctx* c, const double* W, const double* H
       for (int i = 0; i < kMaxModes; ++i) c->factor_cap[i] = 0;
     }
     c->k = k;
+    ensure_factor_buffers(c);
     const double* src[2] = {W, H};
-    for (int i = 0; i < 2; ++i) {
-      const size_t need = (size_t)c->dims[i] * k;
-      if (c->factor_cap[i] != (int64_t)need) {
-        dalloc(&c->F[i], need);
-        dalloc(&c->M[i], need);
-        c->factor_cap[i] = (int64_t)need;
-        c->buf_epoch++;
-      }
-      CK(cudaMemcpyAsync(c->F[i], src[i], need * 8, cudaMemcpyHostToDevice, c->stream));
-    }
+    for (int i = 0; i < 2; ++i)
+      CK(cudaMemcpyAsync(c->F[i], src[i], (size_t)c->dims[i] * k * 8, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->have_factors = false;  // the NTF factors (normalised, with Grams) are not these
     c->nmf_have = true;

@@ -193,10 +193,14 @@ struct planc_gpu_ctx {
   int nmf_galgo = -1;
   int64_t nmf_gepoch = -1;
 
-  // cached iteration graphs: [0] the plain iteration, [1] iteration +
-  // Nesterov acceleration
+  // cached graphs of g_iters iterations: [0] the plain iteration, [1] iteration
+  // + Nesterov acceleration
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  int g_algo[2] = {-1, -1}, g_dimtree[2] = {-1, -1}, g_err[2] = {-1, -1};
+  int g_algo[2] = {-1, -1}, g_dimtree[2] = {-1, -1}, g_err[2] = {-1, -1}, g_iters[2] = {0, 0};
+  // configuration of the last run (its buffers' epoch with it): a run of
+  // another one launches its kernels one by one
+  int r_algo = -1, r_dimtree = -1, r_err = -1;
+  int64_t r_epoch = -1;
 
   bool timing = false;
   bool capturing = false;
@@ -1441,6 +1445,7 @@ void reset_graph(planc_gpu_ctx* c) {
       c->gexec[v] = nullptr;
     }
     c->g_algo[v] = c->g_dimtree[v] = c->g_err[v] = -1;
+    c->g_iters[v] = 0;
   }
 }
 
@@ -1987,11 +1992,24 @@ bool known_algo(int algo) {
          algo == PLANC_GPU_AOADMM || algo == PLANC_GPU_NESTEROV;
 }
 
-// Captures (once) and returns the graph of one iteration; variant 1 appends
-// the Nesterov acceleration.
-cudaGraphExec_t iteration_graph(planc_gpu_ctx* c, int algo, bool dt, bool err, int variant) {
+// Iterations of a graph for a run of `count`: up to 8, so that the run divides
+// evenly where it can (the rest are launched one by one). Between two graph
+// launches the GPU idles for 5 to 6 us, a tenth of a small iteration.
+int graph_iters(int count) {
+  if (count <= 8) return count;
+  int best = 8;
+  for (int u = 7; u >= 4; --u)
+    if (count % u < count % best) best = u;
+  return best;
+}
+
+// Captures (once) and returns the graph of g_iters[variant] iterations for a
+// run of `count`; variant 1 appends the Nesterov acceleration to each. A graph
+// of fewer iterations than such a run takes is captured again.
+cudaGraphExec_t iteration_graph(planc_gpu_ctx* c, int algo, bool dt, bool err, int variant, int count) {
+  const int iters = graph_iters(count);
   if (c->gexec[variant] && c->g_algo[variant] == algo && c->g_dimtree[variant] == (int)dt &&
-      c->g_err[variant] == (int)err)
+      c->g_err[variant] == (int)err && c->g_iters[variant] >= iters)
     return c->gexec[variant];
   if (c->gexec[variant]) {
     cudaGraphExecDestroy(c->gexec[variant]);
@@ -2001,7 +2019,7 @@ cudaGraphExec_t iteration_graph(planc_gpu_ctx* c, int algo, bool dt, bool err, i
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   c->capturing = true;
   try {
-    one_iteration(c, algo, dt, err, variant == 1);
+    for (int i = 0; i < iters; ++i) one_iteration(c, algo, dt, err, variant == 1);
   } catch (...) {
     c->capturing = false;
     cudaStreamEndCapture(c->stream, &graph);
@@ -2016,6 +2034,7 @@ cudaGraphExec_t iteration_graph(planc_gpu_ctx* c, int algo, bool dt, bool err, i
   c->g_algo[variant] = algo;
   c->g_dimtree[variant] = (int)dt;
   c->g_err[variant] = (int)err;
+  c->g_iters[variant] = iters;
   return c->gexec[variant];
 }
 
@@ -2043,17 +2062,30 @@ int planc_gpu_run(planc_gpu_ctx* c, int algo, int iters, int dimtree, int comput
     if (c->g_epoch != c->buf_epoch) reset_graph(c);
     CK(cudaMemsetAsync(c->counter_dev, 0, sizeof(int), c->stream));
     gram_loo(c, 0);
-    bool use_graph = !c->timing;
+    // A configuration's first short run launches its kernels one by one (the
+    // capture and instantiation of a graph cost more than it saves there), the
+    // next ones replay graphs.
+    const bool seen = c->r_algo == algo && c->r_dimtree == (int)dt && c->r_err == (int)err &&
+                      c->r_epoch == c->buf_epoch;
+    const bool use_graph = !c->timing && (seen || iters > 32);
+    c->r_algo = algo;
+    c->r_dimtree = dt;
+    c->r_err = err;
+    c->r_epoch = c->buf_epoch;
     // AUNTF::computeNTF restarts its iteration count at 0 on every call and
     // NTFNES accelerates from iteration acc_start + 1 = 6 on
     // (ntf/auntf.hpp:129, ntf/ntfnes.hpp:65)
-    auto accel_at = [&](int it) { return nes && it > 5; };
-    if (use_graph) {
-      for (int it = 0; it < iters; ++it)
-        CK(cudaGraphLaunch(iteration_graph(c, algo, dt, err, accel_at(it) ? 1 : 0), c->stream));
-      c->g_epoch = c->buf_epoch;
-    } else {
-      for (int it = 0; it < iters; ++it) one_iteration(c, algo, dt, err, accel_at(it));
+    const int plain = nes ? std::min(iters, 6) : iters;
+    for (int variant = 0; variant < 2; ++variant) {
+      const int count = variant == 0 ? plain : iters - plain;
+      int done = 0;
+      if (use_graph && count > 0) {
+        cudaGraphExec_t g = iteration_graph(c, algo, dt, err, variant, count);
+        for (; done + c->g_iters[variant] <= count; done += c->g_iters[variant])
+          CK(cudaGraphLaunch(g, c->stream));
+        c->g_epoch = c->buf_epoch;
+      }
+      for (; done < count; ++done) one_iteration(c, algo, dt, err, variant == 1);
     }
     if (compute_error && errs_out)
       CK(cudaMemcpyAsync(errs_out, c->errs_dev, iters * sizeof(double), cudaMemcpyDeviceToHost,

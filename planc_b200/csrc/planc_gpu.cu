@@ -1488,6 +1488,14 @@ void free_update_state(planc_gpu_ctx* c) {
   c->nmf_ready = false;
 }
 
+// The counters of a new NTFNES object (ntfnes.hpp:186-189).
+NesDev nes_initial() {
+  NesDev d{};
+  d.acc_exp = 3;
+  return d;
+}
+const NesDev kNesInit = nes_initial();
+
 // Allocates (zeroed) the solver-object state of `algo` if it is not there:
 // the reference's constructors zero m_ncp_aux (ntfaoadmm.hpp:86) and
 // m_prox_t / m_prev_t / m_acc_t / m_grad_t (ntfnes.hpp:179-182), set the
@@ -1549,9 +1557,7 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
     CK(cudaMemcpyAsync(c->nes_lam, ones.data(), ones.size() * 8, cudaMemcpyHostToDevice, c->stream));
     dalloc(&c->nes_gbak, (size_t)c->N * k * k);
     dalloc(&c->nes, 1);
-    NesDev init{};
-    init.acc_exp = 3;
-    CK(cudaMemcpyAsync(c->nes, &init, sizeof(NesDev), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->nes, &kNesInit, sizeof(NesDev), cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->nes_ready = true;
     c->buf_epoch++;
@@ -2494,8 +2500,20 @@ int planc_gpu_reset_update_state(planc_gpu_ctx* c) {
   return guarded([&] {
     if (!c) fail(PLANC_GPU_ERR_ARG, "null context");
     set_device(c);
-    CK(cudaStreamSynchronize(c->stream));
-    free_update_state(c);
+    // the buffers, and with them the captured graphs, stay
+    const int k = c->k;
+    if (c->admm_ready)
+      for (int n = 0; n < c->N; ++n)
+        CK(cudaMemsetAsync(c->aux[n], 0, (size_t)c->dims[n] * k * 8, c->stream));
+    if (c->nes_ready) {
+      for (int n = 0; n < c->N; ++n) {
+        CK(cudaMemsetAsync(c->prox[n], 0, (size_t)c->dims[n] * k * 8, c->stream));
+        CK(cudaMemsetAsync(c->prev[n], 0, (size_t)c->dims[n] * k * 8, c->stream));
+      }
+      k_fill<<<1, 256, 0, c->stream>>>(c->nes_lam, 3 * k, 1.0);
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(c->nes, &kNesInit, sizeof(NesDev), cudaMemcpyHostToDevice, c->stream));
+    }
   });
 }
 

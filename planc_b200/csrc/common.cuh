@@ -86,4 +86,16 @@ __device__ __forceinline__ double wgen_row(const WGen& g, const WIdx& w, int r, 
   return v;
 }
 
+// Block t of the upper triangle of kb x kb blocks, row by row: (ta, tb >= ta);
+// ta = kb for t past the last one.
+__device__ __forceinline__ void tri_block(int t, int kb, int& ta, int& tb) {
+  int t0 = 0;
+  ta = 0;
+  while (ta < kb && t0 + (kb - ta) <= t) {
+    t0 += kb - ta;
+    ++ta;
+  }
+  tb = ta + (t - t0);
+}
+
 }  // namespace pg

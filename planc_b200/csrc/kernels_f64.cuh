@@ -1281,7 +1281,8 @@ __global__ void __launch_bounds__(256) k_sumsq_partial(const T* __restrict__ X, 
 // Differentiable CP loss, 1/2 ||X - [[F_0..F_{N-1}]]||^2, in three fused
 // launches around the MTTKRPs (the gradient form of ntf/ntfnes.hpp:138-147).
 // ---------------------------------------------------------------------------
-constexpr int CPG_BLOCKS = 8;  // row blocks per factor of the Gram kernel
+constexpr int CPG_BLOCKS = 16;  // row blocks per factor of the Gram kernel
+constexpr int CPG_TILE = 32;    // rows of a shared-memory tile
 
 struct CpFactors {
   const double* F[kMaxModes];
@@ -1289,67 +1290,128 @@ struct CpFactors {
   int N, k;
 };
 
-// Grams G_n = F_n^T F_n of every factor: block (b, n) sums its share of the
-// rows of F_n into part[n][b]; the last block of factor n to finish (counter
-// ctr[n], left at 0 again) adds the CPG_BLOCKS partials in order into G_n.
-__global__ void __launch_bounds__(256) k_cp_grams(CpFactors f, double* __restrict__ part,
-                                                  double* __restrict__ G, unsigned* __restrict__ ctr) {
+// Grams G_n = F_n^T F_n of every factor and the loss
+// 1/2 ||X||^2 - <M_0, F_0> + 1/2 sum_ab prod_n G_n[a, b], in one launch.
+// Block (b, n) sums its share of the rows of F_n into part[n][b] (rows in
+// shared-memory tiles, a BE x BE block of the upper triangle a thread) and, for
+// n = 0, of <M_0, F_0>; the last block of a factor to finish (counter ctr[n])
+// adds the partials in order into G_n, and the last factor's (ctr[kMaxModes])
+// forms the loss. The counters are left at 0. Bound by latencies (a share is
+// 32 rows at 512); two loads from global memory a product, eight blocks a
+// factor and a launch of its own for the loss took 38 us at 512^3, rank 32.
+template <int KP>
+__global__ void __launch_bounds__(256) k_cp_grams(CpFactors f, const double* __restrict__ M0,
+                                                  double* __restrict__ part, double* __restrict__ G,
+                                                  unsigned* __restrict__ ctr,
+                                                  const double* __restrict__ normX2,
+                                                  double* __restrict__ loss) {
+  constexpr int BE = KP == 16 ? 1 : KP == 32 ? 2 : 4, KB = KP / BE, LDH = KP + 2;
+  __shared__ __align__(16) double tile[CPG_TILE * LDH];
+  __shared__ double red[8];
   __shared__ bool last;
   const int n = blockIdx.y, b = blockIdx.x, k = f.k, kk2 = k * k;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t I = f.I[n];
   const int64_t per = (I + CPG_BLOCKS - 1) / CPG_BLOCKS;
   const int64_t r0 = b * per, r1 = (r0 + per) < I ? (r0 + per) : I;
   const double* F = f.F[n];
-  double* dst = part + ((int64_t)n * CPG_BLOCKS + b) * kk2;
-  for (int e = threadIdx.x; e < kk2; e += 256) {
-    const int a = e / k, c = e % k;
-    double s0 = 0.0, s1 = 0.0;
-    int64_t i = r0;
-    for (; i + 1 < r1; i += 2) {
-      s0 = fma(F[i * k + a], F[i * k + c], s0);
-      s1 = fma(F[(i + 1) * k + a], F[(i + 1) * k + c], s1);
+  double* inner_part = part + (int64_t)kMaxModes * CPG_BLOCKS * kMaxRank * kMaxRank;
+  int ta, tb;
+  tri_block(tid, KB, ta, tb);
+  const bool owner = ta < KB && BE * ta < k;
+  double acc[BE][BE];
+#pragma unroll
+  for (int u = 0; u < BE; ++u)
+#pragma unroll
+    for (int v = 0; v < BE; ++v) acc[u][v] = 0.0;
+  double inner = 0.0;
+  for (int64_t c0 = r0; c0 < r1; c0 += CPG_TILE) {
+    const int nr = (int)((r1 - c0) < CPG_TILE ? (r1 - c0) : CPG_TILE);
+    for (int e = tid; e < nr * KP; e += 256) {
+      const int i = e / KP, c = e % KP;
+      const double x = c < k ? F[(c0 + i) * k + c] : 0.0;
+      tile[i * LDH + c] = x;
+      if (n == 0 && c < k) inner = fma(M0[(c0 + i) * k + c], x, inner);
     }
-    if (i < r1) s0 = fma(F[i * k + a], F[i * k + c], s0);
-    dst[e] = s0 + s1;
+    __syncthreads();
+    if (owner)
+#pragma unroll 4
+      for (int i = 0; i < nr; ++i) {
+        const double* r = tile + i * LDH;
+        double av[BE], bv[BE];
+#pragma unroll
+        for (int u = 0; u < BE; ++u) {
+          av[u] = r[BE * ta + u];
+          bv[u] = r[BE * tb + u];
+        }
+#pragma unroll
+        for (int u = 0; u < BE; ++u)
+#pragma unroll
+          for (int v = 0; v < BE; ++v) acc[u][v] = fma(av[u], bv[v], acc[u][v]);
+      }
+    __syncthreads();
+  }
+  double* dst = part + ((int64_t)n * CPG_BLOCKS + b) * kk2;
+  if (owner)
+#pragma unroll
+    for (int u = 0; u < BE; ++u)
+#pragma unroll
+      for (int v = 0; v < BE; ++v) {
+        const int i = BE * ta + u, j = BE * tb + v;
+        if (i < k && j < k) {
+          dst[i * k + j] = acc[u][v];
+          dst[j * k + i] = acc[u][v];
+        }
+      }
+  auto block_sum = [&](double v) {  // in thread 0
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    double s = 0.0;
+    for (int w = 0; w < 8; ++w) s += red[w];
+    return s;
+  };
+  if (n == 0) {
+    const double s = block_sum(inner);
+    if (tid == 0) inner_part[b] = s;
   }
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ctr + n, 1u) == CPG_BLOCKS - 1;
+  if (tid == 0) last = atomicAdd(ctr + n, 1u) == CPG_BLOCKS - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
   const double* src = part + (int64_t)n * CPG_BLOCKS * kk2;
-  for (int e = threadIdx.x; e < kk2; e += 256) {
+  for (int e = tid; e < kk2; e += 256) {
     double t = 0.0;
+#pragma unroll
     for (int q = 0; q < CPG_BLOCKS; ++q) t += __ldcg(src + (int64_t)q * kk2 + e);
     G[(int64_t)n * kk2 + e] = t;
   }
-  if (threadIdx.x == 0) ctr[n] = 0;
-}
-
-// loss = 1/2 ||X||^2 - <M_0, F_0> + 1/2 sum_ab prod_n G_n[a, b]  (one CTA)
-__global__ void __launch_bounds__(1024) k_cp_loss(const double* __restrict__ M0,
-                                                  const double* __restrict__ F0, int64_t I0,
-                                                  const double* __restrict__ G, int N, int k,
-                                                  const double* __restrict__ normX2,
-                                                  double* __restrict__ loss) {
-  __shared__ double red[1024];
-  const int tid = threadIdx.x;
-  double v = 0.0;
-  for (int64_t e = tid; e < I0 * k; e += 1024) v = fma(M0[e], F0[e], v);
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    ctr[n] = 0;
+    last = atomicAdd(ctr + kMaxModes, 1u) == (unsigned)f.N - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   double mm = 0.0;
-  for (int e = tid; e < k * k; e += 1024) {
+  for (int e = tid; e < kk2; e += 256) {
     double g = 1.0;
-    for (int n = 0; n < N; ++n) g *= G[(int64_t)n * k * k + e];
+    for (int m = 0; m < f.N; ++m) g *= __ldcg(G + (int64_t)m * kk2 + e);
     mm += g;
   }
-  red[tid] = 0.5 * mm - v;
-  __syncthreads();
-  for (int st = 512; st > 0; st >>= 1) {
-    if (tid < st) red[tid] += red[tid + st];
-    __syncthreads();
+  const double s = block_sum(mm);
+  if (tid == 0) {
+    double in = 0.0;
+    for (int q = 0; q < CPG_BLOCKS; ++q) in += __ldcg(inner_part + q);
+    *loss = 0.5 * (*normX2) + (0.5 * s - in);
+    ctr[kMaxModes] = 0;
   }
-  if (tid == 0) *loss = 0.5 * (*normX2) + red[0];
 }
 
 // grad_n = g * (F_n H_n - M_n), H_n = prod_{m != n} G_m (Hadamard), for every

@@ -238,13 +238,8 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
   // thread, rows in increasing order
   {
     constexpr int BE = S::BE, KB = S::KB;
-    // block t of the triangle: row ta, column tb >= ta
-    int ta = 0, t0 = 0;
-    while (ta < KB && t0 + (KB - ta) <= tid) {
-      t0 += KB - ta;
-      ++ta;
-    }
-    const int tb = ta + (tid - t0);
+    int ta, tb;
+    tri_block(tid, KB, ta, tb);
     if (ta < KB && BE * ta < k) {
       double acc[BE][BE];
 #pragma unroll

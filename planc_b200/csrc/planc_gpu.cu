@@ -105,8 +105,8 @@ struct planc_gpu_ctx {
   double* X64 = nullptr;         // FP64 tensor (plain path)
   int64_t x64_elems = 0;
   void* stage = nullptr;         // host-upload staging buffer (kStageBytes), made on first use
-  double* cp_part = nullptr;     // CP-loss Gram partials (N x CPG_BLOCKS x k x k)
-  unsigned* cp_ctr = nullptr;    // their per-factor completion counters
+  double* cp_part = nullptr;     // CP-loss Gram partials (N x CPG_BLOCKS x k x k) and <M_0, F_0> ones
+  unsigned* cp_ctr = nullptr;    // completion counters, one a factor and one over the factors
   double* norm_part = nullptr;   // per-block partial sums of squares of one chunk
   TcTensor tct;                  // tensor-core operand copy (BF16 paths)
   // copies with mode n moved last for the direct (non-tree) MTTKRP on the
@@ -2372,16 +2372,19 @@ int planc_gpu_cp_loss_device(planc_gpu_ctx* c, const double* const* F_dev, const
     const int k = c->k;
     if (!c->cp_part) {
       if (c->capturing) fail(PLANC_GPU_ERR_STATE, "CP-loss buffers would be made during capture");
-      CK(cudaMalloc(&c->cp_part, (size_t)kMaxModes * CPG_BLOCKS * kMaxRank * kMaxRank * 8));
-      CK(cudaMalloc(&c->cp_ctr, kMaxModes * sizeof(unsigned)));
-      CK(cudaMemsetAsync(c->cp_ctr, 0, kMaxModes * sizeof(unsigned), c->stream));
+      CK(cudaMalloc(&c->cp_part,
+                    ((size_t)kMaxModes * CPG_BLOCKS * kMaxRank * kMaxRank + CPG_BLOCKS) * 8));
+      CK(cudaMalloc(&c->cp_ctr, (kMaxModes + 1) * sizeof(unsigned)));
+      CK(cudaMemsetAsync(c->cp_ctr, 0, (kMaxModes + 1) * sizeof(unsigned), c->stream));
     }
     launch(c, KC_NORMGRAM, [&] {
-      k_cp_grams<<<dim3(CPG_BLOCKS, c->N), 256, 0, c->stream>>>(f, c->cp_part, G_out, c->cp_ctr);
-    });
-    launch(c, KC_ERROR, [&] {
-      k_cp_loss<<<1, 1024, 0, c->stream>>>(M0_dev, F_dev[0], c->dims[0], G_out, c->N, k, c->normX2,
-                                            loss_out);
+      const dim3 grid(CPG_BLOCKS, c->N);
+#define CP_GRAMS(KP) \
+  k_cp_grams<KP><<<grid, 256, 0, c->stream>>>(f, M0_dev, c->cp_part, G_out, c->cp_ctr, c->normX2, loss_out)
+      if (k <= 16) CP_GRAMS(16);
+      else if (k <= 32) CP_GRAMS(32);
+      else CP_GRAMS(64);
+#undef CP_GRAMS
     });
   });
 }

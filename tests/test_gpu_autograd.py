@@ -218,3 +218,24 @@ def test_cp_loss_captures_as_cuda_graph(gpu, prec):
                 y.mul_(0.9)
     del graph
     lossf.close()
+
+
+@pytest.mark.parametrize("dims,k", [((5, 4, 3), 1), ((64, 20, 19), 16), ((65, 17, 9), 17), ((40, 257, 8), 32),
+                                    ((33, 20, 1030), 33), ((24, 20, 70, 3), 64)])
+def test_cp_loss_grams_in_one_launch(gpu, oracle_lib, dims, k):
+    # every Gram, the loss and its gradient, either side of the kernel's rank
+    # groups and with modes of fewer and of many more rows than a CTA's share
+    X, F, lossf, Ft = _setup("fp64", dims=dims, k=k, seed=47)
+    loss = lossf(*Ft)
+    loss.backward()
+    letters = "abcd"[:len(dims)]
+    model = np.einsum(",".join(x + "z" for x in letters) + "->" + letters, *F)
+    ref_loss = 0.5 * np.sum((X - model) ** 2)
+    # 0.5 (|X|^2 - 2 <X,model> + |model|^2) in FP64: 1e-10 of its largest term
+    assert abs(loss.item() - ref_loss) < 1e-10 * max(ref_loss, 0.5 * np.sum(model ** 2))
+    for n in range(len(dims)):
+        M = oracle_lib.mttkrp_direct(X, F, n)
+        G = oracle_lib.gram_loo(F, n)
+        # the gradient is a difference of two terms of about this size
+        assert np.abs(Ft[n].grad.cpu().numpy() - (F[n] @ G - M)).max() < 1e-10 * np.abs(M).max()
+    lossf.close()

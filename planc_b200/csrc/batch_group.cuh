@@ -55,10 +55,13 @@ struct GrpTtvL {
   unsigned gx;
 };
 
+// Four consecutive b a CTA: a member's rows are few (32 to 256), and the
+// launch has CTAs enough (256 members: 340 us an iteration with one b a CTA).
+constexpr int GRP_TTVL_NB = 4;
 __global__ void __launch_bounds__(256) k_grp_ttv_left(const GrpTtvL* __restrict__ a) {
   const GrpTtvL& g = a[blockIdx.z];
   if (blockIdx.x >= g.gx) return;
-  ttv_left_body<float>(g.T, g.A, g.B, g.k, g.F, g.out, blockIdx.x, g.gx);
+  ttv_left_body<float, GRP_TTVL_NB>(g.T, g.A, g.B, g.k, g.F, g.out, blockIdx.x, g.gx);
 }
 
 __global__ void __launch_bounds__(256, 4) k_grp_ttv_left_f4(const GrpTtvL* __restrict__ a) {

@@ -2,6 +2,8 @@
 // (partial / direct MTTKRP), multi-TTV, split-K reduction, MU / HALS row
 // sweeps, normalisation + Gram, Gram-form error, tensor norm, synthetic data.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace pg {
@@ -490,38 +492,66 @@ inline void reduce_splits(cudaStream_t st, const double* part, int nsplit, int64
 // ---------------------------------------------------------------------------
 // (kernel bodies take the CTA's index and the grid size as arguments, so that
 // the grouped launches of a batch run every member through the same code)
-template <typename TT>
+// A thread owns rank r and the rows a = lane, lane + lanes, ... in four running
+// sums taken in turn; the CTA adds its row lanes in order. Bound by loads in
+// flight: each thread issues eight rows' loads (or the same four rows' of NB
+// consecutive b, for the many small members of a batch) before their products.
+// The sums' order does not depend on NB. T of 417 x 250 x 20 FP32: 9.6 us with
+// four rows' loads in flight, see the caller for NB.
+template <typename TT, int NB>
 __device__ __forceinline__ void ttv_left_body(const TT* __restrict__ T, int64_t A, int64_t B, int k,
                                               const double* __restrict__ F, double* __restrict__ out,
                                               int64_t bx, int64_t gx) {
-  __shared__ double red[256];
+  __shared__ double red[NB][256];
+  constexpr int U = NB == 1 ? 2 : 1;  // groups of four rows in flight
   const int lanes = 256 / k;
   const int tid = threadIdx.x;
   const int r = tid % k, lane = tid / k;
-  for (int64_t b = bx; b < B; b += gx) {
-    double s = 0.0;
+  for (int64_t b0 = bx * NB; b0 < B; b0 += gx * NB) {
+    const int nb = (int)((B - b0) < NB ? (B - b0) : NB);
+    double s[NB][4];
+#pragma unroll
+    for (int n = 0; n < NB; ++n)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[n][u] = 0.0;
     if (lane < lanes) {
-      const TT* Tb = T + (A * b) * k + r;
+      const TT* Tb = T + A * b0 * k + r;
       const double* Fr = F + r;
-      double s1 = 0.0, s2 = 0.0, s3 = 0.0;
-      const int64_t step = (int64_t)lanes * k;
+      const int64_t step = (int64_t)lanes * k, nstep = A * k;
       int64_t a = lane;
-      for (; a + 3 * lanes < A; a += 4 * lanes) {
-        const int64_t o = a * k;
-        s = fma((double)Tb[o], Fr[o], s);
-        s1 = fma((double)Tb[o + step], Fr[o + step], s1);
-        s2 = fma((double)Tb[o + 2 * step], Fr[o + 2 * step], s2);
-        s3 = fma((double)Tb[o + 3 * step], Fr[o + 3 * step], s3);
-      }
-      for (; a < A; a += lanes) s = fma((double)Tb[a * k], Fr[a * k], s);
-      s = (s + s1) + (s2 + s3);
+      auto rows = [&](auto groups) {
+        constexpr int G = decltype(groups)::value;
+        for (; a + (4 * G - 1) * (int64_t)lanes < A; a += 4 * G * lanes) {
+          const int64_t o = a * k;
+          double f[4 * G];
+          TT t[4 * G][NB];
+#pragma unroll
+          for (int u = 0; u < 4 * G; ++u) {
+            f[u] = Fr[o + u * step];
+#pragma unroll
+            for (int n = 0; n < NB; ++n) t[u][n] = n < nb ? Tb[o + u * step + n * nstep] : TT(0);
+          }
+#pragma unroll
+          for (int u = 0; u < 4 * G; ++u)
+#pragma unroll
+            for (int n = 0; n < NB; ++n) s[n][u & 3] = fma((double)t[u][n], f[u], s[n][u & 3]);
+        }
+      };
+      if constexpr (U > 1) rows(std::integral_constant<int, U>{});
+      rows(std::integral_constant<int, 1>{});
+      for (; a < A; a += lanes)
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+          if (n < nb) s[n][0] = fma((double)Tb[a * k + n * nstep], Fr[a * k], s[n][0]);
     }
-    red[tid] = s;
+#pragma unroll
+    for (int n = 0; n < NB; ++n) red[n][tid] = (s[n][0] + s[n][1]) + (s[n][2] + s[n][3]);
     __syncthreads();
-    if (tid < k) {
+    for (int e = tid; e < nb * k; e += 256) {
+      const int n = NB == 1 ? 0 : e / k, c = e - n * k;
       double t = 0.0;
-      for (int l = 0; l < lanes; ++l) t += red[l * k + tid];
-      out[b * k + tid] = t;
+      for (int l = 0; l < lanes; ++l) t += red[n][l * k + c];
+      out[b0 * k + e] = t;
     }
     __syncthreads();
   }
@@ -530,7 +560,7 @@ template <typename TT>
 __global__ void __launch_bounds__(256) k_ttv_left(const TT* __restrict__ T, int64_t A, int64_t B,
                                                   int k, const double* __restrict__ F,
                                                   double* __restrict__ out) {
-  ttv_left_body<TT>(T, A, B, k, F, out, blockIdx.x, gridDim.x);
+  ttv_left_body<TT, 1>(T, A, B, k, F, out, blockIdx.x, gridDim.x);
 }
 
 // k_ttv_left for an FP32 T with k a multiple of 4: a CTA takes TTVL_NB

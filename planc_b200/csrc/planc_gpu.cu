@@ -2993,7 +2993,7 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
           f4.push_back(GrpTtvL{m->P32, A, B, k, m->F[0], m->M[1], (unsigned)g2});
         else
           plain.push_back(GrpTtvL{m->P32, A, B, k, m->F[0], m->M[1],
-                                  (unsigned)std::min<int64_t>(B, 65535)});
+                                  (unsigned)std::min<int64_t>((B + GRP_TTVL_NB - 1) / GRP_TTVL_NB, 65535)});
       }
       if (!plain.empty())
         k_grp_ttv_left<<<dim3(grp_max(plain, &GrpTtvL::gx), 1, (unsigned)plain.size()), 256, 0, st>>>(

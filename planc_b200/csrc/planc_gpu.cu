@@ -3010,6 +3010,11 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
     red.clear();
     std::vector<TcgLeft> lmem(ms.size());
     std::vector<TcgUnit> lunits[3][2];
+    // members against a Khatri-Rao image: images and contractions grouped by
+    // (rank class, row tiles per CTA), each class on a worker stream of its own
+    std::vector<TcgLong> gmem(ms.size());
+    std::vector<TcgWimg> wimgs[3][2];
+    std::vector<TcgUnit> gunits[3][2];
     fork();
     for (size_t mi = 0; mi < ms.size(); ++mi) {
       planc_gpu_ctx* m = ms[mi];
@@ -3026,17 +3031,20 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
         continue;
       }
       if (left_via_long(m)) {
-        // the member's own Khatri-Rao image and long-K contraction (as
-        // long_contract), the split-K sum in the grouped reduction
-        launch(m, KC_PREP, [&] { tc_long_prep(m->tct, true, wg, m->k, m->stream); });
+        // as long_contract; min(splits, 8) partials are left to the grouped sum
         if (tc_long_scratch_elems(m->tct, true, m->k, eff_sm(m)) > m->scratch_elems)
           fail(PLANC_GPU_ERR_STATE, "internal: split-K scratch larger than planned");
-        int nsplit = 1;
-        launch(m, KC_CONTRACT_LEFT, [&] {
-          nsplit = tc_long(m->tct, true, m->k, m->M[2], m->scratch, m->status_dev, eff_sm(m),
-                           m->stream);
-        });
-        if (nsplit > 1) red.push_back(grp_red(m->scratch, nsplit, m->R * m->k, m->M[2]));
+        const int ci = kpi(m->k), kp = tc_kpad(m->k), MT = tc_long_mt(m->tct.R, m->k);
+        const int64_t nk = (m->tct.L + TC_BK - 1) / TC_BK;
+        int mg = 0, ns = 0;
+        tc_long_plan(m->tct.R, m->tct.L, m->k, eff_sm(m), &mg, &ns);
+        const int np = std::min(ns, 8);
+        wimgs[ci][MT - 1].push_back(TcgWimg{m->F[0], m->F[1], m->tct.L, nk, (int)m->dims[0], m->k,
+                                            tc_wimage_blocks(nk, kp), m->tct.wimg});
+        gmem[mi] = TcgLong{m->tct.wimg, np > 1 ? m->scratch : m->M[2], m->tct.R, m->tct.L, m->k, ns};
+        for (int jg = 0; jg < mg; ++jg)
+          for (int y = 0; y < np; ++y) gunits[ci][MT - 1].push_back(TcgUnit{(int)mi, jg, y, 0});
+        if (np > 1) red.push_back(grp_red(m->scratch, np, m->R * m->k, m->M[2]));
         continue;
       }
       int mg = 0, ns = 0;
@@ -3046,6 +3054,39 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
       for (int jg = 0; jg < mg; ++jg)
         for (int y = 0; y < ns; ++y) lunits[kpi(m->k)][MT - 1].push_back(TcgUnit{(int)mi, jg, y, 0});
       red.push_back(grp_red(m->scratch, ns, m->R * m->k, m->M[2]));
+    }
+    {
+      const TcgLong* dgm = tab.put(gmem);
+      for (int ci = 0; ci < 3; ++ci)
+        for (int mt = 1; mt <= 2; ++mt) {
+          auto& uv = gunits[ci][mt - 1];
+          if (uv.empty()) continue;
+          // longest units first: the CTAs take them in turn
+          std::stable_sort(uv.begin(), uv.end(), [&](const TcgUnit& a, const TcgUnit& c) {
+            return gmem[a.member].L > gmem[c.member].L;
+          });
+          const auto& wv = wimgs[ci][mt - 1];
+          cudaStream_t ws = b->workers[(size_t)(ci * 2 + mt - 1) % b->workers.size()];
+          const dim3 gb(grp_max(wv, &TcgWimg::gx), 1, (unsigned)wv.size());
+          const TcgWimg* dw = tab.put(wv);
+          const TcgUnit* du = tab.put(uv);
+          const int n = (int)uv.size();
+          const int grid = std::min(n, sms);
+          const int gr = tc_long_group();
+#define TCG_LONG(KP, MTV)                                                                             \
+  {                                                                                                   \
+    k_tc_wimage_grp<KP><<<gb, 256, 0, ws>>>(dw);                                                      \
+    if (x2) k_tc_long_grp<KP, MTV, true><<<grid, TCF_THREADS, tcg_long_smem<KP, MTV, true>(), ws>>>(  \
+        dmaps, dgm, du, n, gr, gst);                                                                  \
+    else k_tc_long_grp<KP, MTV, false><<<grid, TCF_THREADS, tcg_long_smem<KP, MTV, false>(), ws>>>(   \
+        dmaps, dgm, du, n, gr, gst);                                                                  \
+  }
+          if (ci == 0) { if (mt == 1) TCG_LONG(16, 1) else TCG_LONG(16, 2) }
+          else if (ci == 1) { if (mt == 1) TCG_LONG(32, 1) else TCG_LONG(32, 2) }
+          else TCG_LONG(64, 1)
+#undef TCG_LONG
+          grp_check(cudaGetLastError());
+        }
     }
     {
       const TcgLeft* dlm = tab.put(lmem);

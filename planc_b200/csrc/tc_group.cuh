@@ -472,6 +472,261 @@ __global__ void __launch_bounds__(TCL_THREADS, 1)
   }
 }
 
+// Khatri-Rao images of F_0 and F_1 of many 3-way members (k_tc_wimage)
+struct TcgWimg {
+  const double* f0;
+  const double* f1;
+  int64_t K, nk;
+  int d0, k;
+  unsigned gx;  // the member's own grid
+  uint8_t* img;
+};
+
+template <int KP>
+__global__ void k_tc_wimage_grp(const TcgWimg* __restrict__ a) {
+  const TcgWimg& g = a[blockIdx.z];
+  if (blockIdx.x >= g.gx) return;
+  tc_wimage2_body<KP>(g.f0, g.f1, g.d0, g.K, g.k, g.nk, g.img, blockIdx.x, g.gx);
+}
+
+// left contraction of one member against its Khatri-Rao image (k_tc_long,
+// K-major): rows j < R, K = l < L, nsplit its own launch's split count
+struct TcgLong {
+  const uint8_t* wimg;
+  double* part;  // min(nsplit, 8) partials of R x k (the result itself for one)
+  int64_t R, L;
+  int k;
+  int nsplit;
+};
+
+// The long-K contraction of every member in one persistent launch. A member's
+// own launch spreads its K over up to 148 splits, a few blocks each, and a
+// tensor of a few MB then writes and reads more partials than it has data. A
+// unit here is the splits y = sub, sub + 8, ... of a row group, for one of 8
+// values of sub: its CTA runs them one after another and adds each split's sum
+// to FP64 accumulators in shared memory, in the order in which
+// reduce_splits_body's lane `sub` adds their partials. The 8 partials left are
+// then summed as that kernel's lanes are, so the bits are those of the member's
+// own launches. Bound by the tensor's bytes and the images': 256 tensors of
+// 32..256 per mode, images, contractions and sums: see the batch's capture.
+// KP x 128 x MT accumulators in the last ACC bytes of dynamic shared memory;
+// `units` are sorted by decreasing work.
+template <int KP, int MT>
+constexpr size_t tcg_long_acc() { return (size_t)MT * TC_BM * KP * sizeof(double); }
+template <int KP, int MT, bool X2>
+constexpr uint32_t tcg_long_stage() { return (X2 ? 2u : 1u) * MT * TC_BM * TC_BK * 2 + 2 * KP * 128; }
+template <int KP, int MT, bool X2>
+constexpr int tcg_long_stages() {
+  const size_t room = (size_t)224 * 1024 - tcg_long_acc<KP, MT>();
+  const int n = (int)(room / tcg_long_stage<KP, MT, X2>());
+  return n > 8 ? 8 : n;
+}
+template <int KP, int MT, bool X2>
+constexpr size_t tcg_long_smem() {
+  return (size_t)tcg_long_stages<KP, MT, X2>() * tcg_long_stage<KP, MT, X2>() + tcg_long_acc<KP, MT>() + 1024;
+}
+
+template <int KP, int MT, bool X2>
+__global__ void __launch_bounds__(TCF_THREADS, 1)
+    k_tc_long_grp(const CUtensorMap* __restrict__ maps, const TcgLong* __restrict__ mem,
+                  const TcgUnit* __restrict__ units, int nunits, int group, int* __restrict__ status) {
+  constexpr int NCOL = 2 * KP;
+  constexpr uint32_t A_TILE = TC_BM * TC_BK * 2;
+  constexpr uint32_t A_BYTES = MT * A_TILE;
+  constexpr uint32_t A_STAGE = X2 ? 2 * A_BYTES : A_BYTES;
+  constexpr uint32_t B_STAGE = NCOL * 128;
+  constexpr uint32_t STAGE = A_STAGE + B_STAGE;
+  constexpr int STAGES = tcg_long_stages<KP, MT, X2>();
+  static_assert(STAGES >= 2, "two stages at least");
+  constexpr uint32_t ACC_COLS = MT * NCOL;
+  constexpr int NBUF = 4;
+  constexpr uint32_t TMEM_NEED = NBUF * ACC_COLS;
+  constexpr uint32_t TMEM_COLS = TMEM_NEED <= 32 ? 32 : TMEM_NEED <= 64 ? 64 : TMEM_NEED <= 128 ? 128
+                                 : TMEM_NEED <= 256 ? 256 : 512;
+  constexpr uint32_t IDESC = idesc_bf16(NCOL, false, false);
+
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t bars[2 * 8 + 2 * NBUF];
+  __shared__ uint32_t tmem_base_sh;
+  __shared__ int abort_sh;
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const uint32_t smem0 = smem_u32(smem);
+  double* acc = reinterpret_cast<double*>(smem + (size_t)STAGES * STAGE);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto full = [&](int s) { return smem_u32(&bars[s]); };
+  auto empty = [&](int s) { return smem_u32(&bars[8 + s]); };
+  auto accf = [&](int b) { return smem_u32(&bars[16 + b]); };
+  auto acce = [&](int b) { return smem_u32(&bars[16 + NBUF + b]); };
+
+  if (threadIdx.x == 0) {
+    abort_sh = 0;
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full(s), 1);
+      mbar_init(empty(s), 1);
+    }
+    for (int b = 0; b < NBUF; ++b) {
+      mbar_init(accf(b), 1);
+      mbar_init(acce(b), 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc(smem_u32(&tmem_base_sh), TMEM_COLS);
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_sh;
+  volatile int* abort_flag = &abort_sh;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+        const TcgUnit U = units[u];
+        const TcgLong& m = mem[U.member];
+        const CUtensorMap* mh = maps + 4 * U.member + 2;
+        tmap_acquire(mh);
+        if (X2) tmap_acquire(mh + 1);
+        const int nk = (int)((m.L + TC_BK - 1) / TC_BK);
+        const int ngroups = (nk + group - 1) / group;
+        const int row0 = U.jg * MT * TC_BM;
+        for (int y = U.y; y < m.nsplit && ok; y += 8)
+          for (int g = y; g < ngroups && ok; g += m.nsplit) {
+            const int kb1 = min((g + 1) * group, nk);
+            for (int kb = g * group; kb < kb1; ++kb) {
+              if (!mbar_wait(empty(s), ph ^ 1, abort_flag, status)) { ok = false; break; }
+              const uint32_t st = smem0 + s * STAGE;
+              mbar_expect_tx(full(s), STAGE);
+#pragma unroll
+              for (int mt = 0; mt < MT; ++mt) {
+                const int r0 = row0 + mt * TC_BM;
+                tma_load_2d(st + mt * A_TILE, mh, kb * TC_BK, r0, full(s));
+                if (X2) tma_load_2d(st + A_BYTES + mt * A_TILE, mh + 1, kb * TC_BK, r0, full(s));
+              }
+              bulk_load(st + A_STAGE, m.wimg + (size_t)kb * B_STAGE, B_STAGE, full(s));
+              if (++s == STAGES) { s = 0; ph ^= 1; }
+            }
+          }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 0;
+      int buf = 0;
+      uint32_t aph = 0;  // bit b: phase of accumulator b
+      bool ok = true;
+      for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+        const TcgUnit U = units[u];
+        const TcgLong& m = mem[U.member];
+        const int nk = (int)((m.L + TC_BK - 1) / TC_BK);
+        const int ngroups = (nk + group - 1) / group;
+        for (int y = U.y; y < m.nsplit && ok; y += 8)
+          for (int g = y; g < ngroups && ok; g += m.nsplit) {
+            const int kb0 = g * group, kb1 = min((g + 1) * group, nk);
+            if (!mbar_wait(acce(buf), ((aph >> buf) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t d = tmem + buf * ACC_COLS;
+            for (int kb = kb0; kb < kb1; ++kb) {
+              if (!mbar_wait(full(s), ph, abort_flag, status)) { ok = false; break; }
+              tc_fence_after();
+              const uint32_t st = smem0 + s * STAGE;
+#pragma unroll
+              for (int kk = 0; kk < TC_BK / 16; ++kk) {
+                const uint64_t bdesc = smem_desc(st + A_STAGE + kk * 32, 16, 1024);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                  const uint32_t a0 = st + mt * A_TILE + kk * 32;
+                  umma_bf16(d + mt * NCOL, smem_desc(a0, 16, 1024), bdesc, IDESC,
+                            (kb != kb0 || kk != 0) ? 1u : 0u);
+                  if (X2) umma_bf16(d + mt * NCOL, smem_desc(a0 + A_BYTES, 16, 1024), bdesc, IDESC, 1);
+                }
+              }
+              umma_commit(empty(s));
+              if (++s == STAGES) { s = 0; ph ^= 1; }
+            }
+            if (!ok) break;
+            umma_commit(accf(buf));
+            aph ^= 1u << buf;
+            buf = (buf + 1) % NBUF;
+          }
+      }
+    }
+  } else {
+    // drain warps 2..5: TMEM lane quarter = warp % 4, one row (of each tile) a thread
+    const int q4 = warp & 3;
+    double* mine = acc + q4 * 32 + lane;  // entry (mt, r) at (mt * KP + r) * TC_BM
+    int buf = 0;
+    uint32_t aph = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+      const TcgUnit U = units[u];
+      const TcgLong& m = mem[U.member];
+      const int nk = (int)((m.L + TC_BK - 1) / TC_BK);
+      const int ngroups = (nk + group - 1) / group;
+      for (int y = U.y; y < m.nsplit && ok; y += 8) {
+        float sum[MT][KP];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int r = 0; r < KP; ++r) sum[mt][r] = 0;
+        for (int g = y; g < ngroups; g += m.nsplit) {
+          if (!mbar_wait(accf(buf), (aph >> buf) & 1, abort_flag, status)) { ok = false; break; }
+          tc_fence_after();
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            const uint32_t base = tmem + ((uint32_t)(q4 * 32) << 16) + buf * ACC_COLS + mt * NCOL;
+            if (KP == 16) {
+              float v[32];
+              tmem_ld32(base, v);  // columns 0..15 hi, 16..31 lo
+#pragma unroll
+              for (int r = 0; r < 16; ++r) sum[mt][r] += v[r] + v[16 + r];
+            } else {
+#pragma unroll
+              for (int cc = 0; cc < KP; cc += 32) {  // hi and lo 32-column slices, one wait
+                float vh[32], vl[32];
+                tmem_ld32x2(base + cc, base + KP + cc, vh, vl);
+#pragma unroll
+                for (int e = 0; e < 32; e += 2)
+                  add2_acc(sum[mt][cc + e], sum[mt][cc + e + 1], vh[e], vh[e + 1], vl[e], vl[e + 1]);
+              }
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acce(buf));
+          aph ^= 1u << buf;
+          buf = (buf + 1) % NBUF;
+        }
+        if (!ok) break;
+        // the split's sum joins the unit's
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int r = 0; r < KP; ++r) {
+            double* a = mine + (size_t)(mt * KP + r) * TC_BM;
+            *a = (y == U.y ? 0.0 : *a) + (double)sum[mt][r];
+          }
+      }
+      if (!ok) break;
+      double* dst = m.part + (int64_t)U.y * m.R * m.k;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const int64_t row = ((int64_t)U.jg * MT + mt) * TC_BM + q4 * 32 + lane;
+        if (row < m.R)
+          for (int r = 0; r < m.k; ++r) dst[row * m.k + r] = mine[(size_t)(mt * KP + r) * TC_BM];
+      }
+    }
+  }
+  __syncthreads();
+  if (abort_sh) tc_drain_after_abort();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, TMEM_COLS);
+  }
+}
+
 // B images of the right contractions of many members (k_tc_bimage)
 struct TcgBimg {
   const double* F;
@@ -502,6 +757,13 @@ inline cudaError_t tcg_set_attrs() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_tc_left_grp<KP, 2, X2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(tc_stages(SL2) * SL2 + 1024));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_tc_long_grp<KP, 1, X2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)tcg_long_smem<KP, 1, X2>());
+  if constexpr (KP <= 32)
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_tc_long_grp<KP, 2, X2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)tcg_long_smem<KP, 2, X2>());
   return e;
 }
 

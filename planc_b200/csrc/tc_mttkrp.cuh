@@ -1356,56 +1356,78 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
 // Pre-swizzled hi|lo image of a Khatri-Rao product W(kk, r) = prod_t
 // F_t[digit_t(kk), r] (the B operand of k_tc_long), laid out as k_tc_bimage.
 // One thread per (k block, r, 16-byte chunk): eight consecutive kk, written
-// as one 16-byte store each for hi and lo. Two-mode products with K < 2^31
-// (the balanced 4-way tree) take their digits with 32-bit arithmetic.
+// as one 16-byte store each for hi and lo. Bound by the factor loads, two a
+// product: neighbouring lanes take neighbouring ranks, so that a load is one or
+// two whole lines (the stores, one eighth as many, go to a line a lane).
+// Two-mode products with K < 2^31 take their digits with 32-bit arithmetic,
+// one division a thread.
 template <int KP>
-__global__ void k_tc_wimage(const WGen wg, int64_t K, int k, int64_t nk, uint8_t* __restrict__ img) {
-  constexpr int NCOL = 2 * KP;
+__device__ __forceinline__ void tc_wimage_store(const double (&w)[8], int64_t kb, int ch, int r,
+                                                uint8_t* __restrict__ img) {
+  alignas(16) __nv_bfloat16 hi[8], lo[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) split_bf16(w[u], hi[u], lo[u]);
+  uint8_t* st = img + (size_t)kb * 2 * KP * 128;
+  *reinterpret_cast<uint4*>(st + sw128_kmajor_off(r, ch * 8)) = *reinterpret_cast<const uint4*>(hi);
+  *reinterpret_cast<uint4*>(st + sw128_kmajor_off(KP + r, ch * 8)) = *reinterpret_cast<const uint4*>(lo);
+}
+
+// W(kk, r) = f0[kk % d0, r] f1[kk / d0, r], K < 2^31. The eight rows' factor
+// values are all loaded before any is converted (one memory latency per
+// thread, not eight).
+template <int KP>
+__device__ __forceinline__ void tc_wimage2_body(const double* __restrict__ f0, const double* __restrict__ f1,
+                                                int d0, int64_t K, int k, int64_t nk,
+                                                uint8_t* __restrict__ img, int64_t bx, int64_t gx) {
   const int64_t total = nk * KP * (TC_BK / 8);
-  const bool two32 = wg.nf == 2 && K < ((int64_t)1 << 31);
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(e % (TC_BK / 8));
-    const int r = (int)((e / (TC_BK / 8)) % KP);
+  for (int64_t e = bx * blockDim.x + threadIdx.x; e < total; e += gx * blockDim.x) {
+    const int r = (int)(e % KP);
+    const int ch = (int)((e / KP) % (TC_BK / 8));
     const int64_t kb = e / ((int64_t)(TC_BK / 8) * KP);
-    alignas(16) __nv_bfloat16 hi[8], lo[8];
-    // the eight rows' factor values are all loaded before any is converted
-    // (one memory latency per thread, not eight)
-    double w[8];
-    if (wg.nf == 1) {
-      const double* f0 = wg.f[0];
+    const int64_t j0 = kb * TC_BK + ch * 8;
+    const int jj = j0 < K ? (int)j0 : 0;
+    int i1 = jj / d0, i0 = jj - i1 * d0;
+    double a[8], b[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int64_t j = kb * TC_BK + ch * 8 + u;
-        w[u] = (j < K && r < k) ? f0[j * k + r] : 0.0;
-      }
-    } else if (two32) {
-      const int d0 = (int)wg.dim[0];
-      double a[8], b[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int64_t j = kb * TC_BK + ch * 8 + u;
-        const bool in = j < K && r < k;
-        const int jj = in ? (int)j : 0;
-        const int i1 = jj / d0, i0 = jj - i1 * d0;
-        a[u] = in ? wg.f[0][(int64_t)i0 * k + r] : 0.0;
-        b[u] = in ? wg.f[1][(int64_t)i1 * k + r] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) w[u] = a[u] * b[u];
-    } else {
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int64_t j = kb * TC_BK + ch * 8 + u;
-        w[u] = (j < K && r < k) ? wgen_eval(wg, j, r, k) : 0.0;
+    for (int u = 0; u < 8; ++u) {
+      const bool in = j0 + u < K && r < k;
+      a[u] = in ? f0[(int64_t)i0 * k + r] : 0.0;
+      b[u] = in ? f1[(int64_t)i1 * k + r] : 0.0;
+      if (++i0 == d0) {
+        i0 = 0;
+        ++i1;
       }
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) split_bf16(w[u], hi[u], lo[u]);
-    uint8_t* st = img + (size_t)kb * NCOL * 128;
-    *reinterpret_cast<uint4*>(st + sw128_kmajor_off(r, ch * 8)) = *reinterpret_cast<const uint4*>(hi);
-    *reinterpret_cast<uint4*>(st + sw128_kmajor_off(KP + r, ch * 8)) = *reinterpret_cast<const uint4*>(lo);
+    for (int u = 0; u < 8; ++u) a[u] = a[u] * b[u];
+    tc_wimage_store<KP>(a, kb, ch, r, img);
   }
+}
+
+template <int KP>
+__device__ __forceinline__ void tc_wimage_body(const WGen& wg, int64_t K, int k, int64_t nk,
+                                               uint8_t* __restrict__ img, int64_t bx, int64_t gx) {
+  if (wg.nf == 2 && K < ((int64_t)1 << 31)) {
+    tc_wimage2_body<KP>(wg.f[0], wg.f[1], (int)wg.dim[0], K, k, nk, img, bx, gx);
+    return;
+  }
+  const int64_t total = nk * KP * (TC_BK / 8);
+  for (int64_t e = bx * blockDim.x + threadIdx.x; e < total; e += gx * blockDim.x) {
+    const int r = (int)(e % KP);
+    const int ch = (int)((e / KP) % (TC_BK / 8));
+    const int64_t kb = e / ((int64_t)(TC_BK / 8) * KP);
+    double w[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int64_t j = kb * TC_BK + ch * 8 + u;
+      w[u] = (j < K && r < k) ? (wg.nf == 1 ? wg.f[0][j * k + r] : wgen_eval(wg, j, r, k)) : 0.0;
+    }
+    tc_wimage_store<KP>(w, kb, ch, r, img);
+  }
+}
+template <int KP>
+__global__ void k_tc_wimage(const WGen wg, int64_t K, int k, int64_t nk, uint8_t* __restrict__ img) {
+  tc_wimage_body<KP>(wg, K, k, nk, img, blockIdx.x, gridDim.x);
 }
 
 // 32-bit mix of a 64-bit counter (the finaliser of the splitmix64 generator,
@@ -2021,13 +2043,17 @@ inline size_t tc_long_scratch_elems(const TcTensor& t, bool left, int k, int sm_
   return ns > 1 ? (size_t)ns * rows * k : 0;
 }
 
+inline unsigned tc_wimage_blocks(int64_t nk, int kp) {
+  return (unsigned)std::min<int64_t>((nk * kp * (TC_BK / 8) + 255) / 256, 2048);
+}
+
 // Image of W = KRP over the K index of the left (K = l, rows j) or right
 // (K = j, rows l) contraction.
 inline void tc_long_prep(const TcTensor& t, bool left, const WGen& wg, int k, cudaStream_t st) {
   const int64_t K = left ? t.L : t.R;
   const int64_t nk = (K + TC_BK - 1) / TC_BK;
   const int kp = tc_kpad(k);
-  const unsigned blocks = (unsigned)std::min<int64_t>((nk * kp * (TC_BK / 8) + 255) / 256, 2048);
+  const unsigned blocks = tc_wimage_blocks(nk, kp);
   if (kp == 16)
     k_tc_wimage<16><<<blocks, 256, 0, st>>>(wg, K, k, nk, t.wimg);
   else if (kp == 32)

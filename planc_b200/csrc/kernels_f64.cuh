@@ -653,46 +653,51 @@ __global__ void __launch_bounds__(256, 4) k_ttv_left_f4(const float* __restrict_
   ttv_left_f4_body(T, A, B, k, F, out, blockIdx.x);
 }
 
-template <typename TT>
-__global__ void __launch_bounds__(256) k_ttv_right(const TT* __restrict__ T, int64_t A, int64_t B,
-                                                   int k, WGen wg, int64_t b_per_split,
-                                                   int64_t split_stride,
-                                                   double* __restrict__ out) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= A * k) return;
-  const int64_t a = e / k;
-  const int r = (int)(e % k);
-  int64_t b0 = (int64_t)blockIdx.y * b_per_split;
-  int64_t b1 = b0 + b_per_split;
-  if (b1 > B) b1 = B;
-  if (b0 >= b1) {
-    out[(int64_t)blockIdx.y * split_stride + e] = 0.0;
-    return;
-  }
-  double s = 0.0;
-  const TT* Tp = T + (a + A * b0) * k + r;
-  const int64_t tstride = A * k;
-  if (wg.nf == 1) {
-    const double* W = wg.f[0] + r;
-    double s1 = 0.0;
-    int64_t b = b0;
-    for (; b + 1 < b1; b += 2) {
-      s = fma((double)Tp[0], W[b * k], s);
-      s1 = fma((double)Tp[tstride], W[(b + 1) * k], s1);
-      Tp += 2 * tstride;
+// Right multi-TTV of an FP64 intermediate, a CTA per na consecutive a: threads
+// (a, r) x LB lanes over b, four b a lane in flight, lanes added in order. One
+// launch with no partials, for intermediates whose tiled form is all latency: a
+// tile of 4096 / KP rows is mostly empty when A is small, each CTA walks its
+// eight b two at a time, and the partials take a launch to sum (64 x 64 x 8:
+// 5.9 + 1.7 us against 3.3).
+template <int NF>
+__global__ void __launch_bounds__(1024) k_ttv_right_rows(const double* __restrict__ T, int64_t A, int64_t B,
+                                                         int k, int na, WGen wg, double* __restrict__ out) {
+  extern __shared__ double ttvr_red[];
+  const int tid = threadIdx.x, ne = na * k, LB = blockDim.x / ne;
+  const int e = tid % ne, lb = tid / ne;
+  const int r = e % k;
+  const int64_t a = (int64_t)blockIdx.x * na + e / k;
+  FastDiv f0{1, 1, 0};
+  if (NF == 2) f0 = make_fastdiv((uint32_t)wg.dim[0]);
+  auto w_at = [&](int64_t b) {
+    if constexpr (NF == 1) return wg.f[0][b * k + r];
+    const uint32_t i1 = fast_div((uint32_t)b, f0), i0 = (uint32_t)b - i1 * f0.d;
+    return wg.f[0][(int64_t)i0 * k + r] * wg.f[1][(int64_t)i1 * k + r];
+  };
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  if (lb < LB && a < A) {
+    const double* Ta = T + a * k + r;
+    const int64_t step = A * k;
+    int64_t b = lb;
+    for (; b + 3 * (int64_t)LB < B; b += 4 * LB) {
+      double t[4], w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        t[u] = Ta[(b + (int64_t)u * LB) * step];
+        w[u] = w_at(b + (int64_t)u * LB);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u] = fma(t[u], w[u], s[u]);
     }
-    if (b < b1) s = fma((double)Tp[0], W[b * k], s);
-    s += s1;
-  } else {
-    WIdx wi;
-    widx_init(wg, b0, wi);
-    for (int64_t b = b0; b < b1; ++b) {
-      s = fma((double)Tp[0], wgen_row(wg, wi, r, k), s);
-      Tp += tstride;
-      widx_advance(wg, wi, 1);
-    }
+    for (; b < B; b += LB) s[0] = fma(Ta[b * step], w_at(b), s[0]);
   }
-  out[(int64_t)blockIdx.y * split_stride + e] = s;
+  ttvr_red[tid] = (s[0] + s[1]) + (s[2] + s[3]);
+  __syncthreads();
+  if (tid < ne && a < A) {
+    double t = 0.0;
+    for (int l = 0; l < LB; ++l) t += ttvr_red[l * ne + tid];
+    out[a * k + r] = t;
+  }
 }
 
 // Tiled right multi-TTV: a CTA owns AT = 4096/KP consecutive a values (all

@@ -292,3 +292,17 @@ def test_set_tensor_host_and_device_sources_agree(gpu, prec, dtype):
         a.set_tensor(X)
         a.set_factors(F)
         assert np.array_equal(a.mttkrp(0), m0)
+
+
+@pytest.mark.parametrize("dims,k", [((32, 5, 4), 3), ((129, 31, 17), 16), ((200, 150, 16), 10), ((70, 64, 63), 32),
+                                    ((64, 512, 64), 1), ((32, 33, 5, 6), 7), ((257, 8, 1024), 8), ((64, 32, 130), 64),
+                                    ((65, 32, 32, 33), 9)])
+def test_dimtree_ttv_of_short_rows(gpu, oracle_lib, dims, k):
+    # the multi-TTV with a CTA per few rows: odd extents, one and two factors,
+    # either side of its largest intermediate (2^21 entries)
+    X, _ = cp_tensor(dims, 3, seed=5)
+    F = init_factors(dims, k, seed=6)
+    with _ctx(gpu, X, F) as c:
+        Fn = _normalized(F)
+        for n in range(len(dims)):
+            assert rel(c.mttkrp(n, dimtree=True), oracle_lib.mttkrp_direct(X, Fn, n)) < TOL

@@ -1180,7 +1180,7 @@ void run_update(planc_gpu_ctx* c, int algo, int n) {
     // the accelerated proximal-gradient loop from the proximal point, in one
     // cluster launch.
     launch(c, KC_UPDATE, [&] {
-      k_nes_prep<<<1, NES_PREP_THREADS, 0, c->stream>>>(c->Gloo, k, c->nes, n, c->nes_lam, c->nes_lam + k);
+      k_nes_prep<<<1, nes_prep_threads(k), 0, c->stream>>>(c->Gloo, k, c->nes, n, c->nes_lam, c->nes_lam + k);
     });
     // the smallest register-resident shape whose cluster holds every row;
     // beyond the largest the state lives in global scratch

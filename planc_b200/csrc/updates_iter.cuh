@@ -607,12 +607,14 @@ __device__ __forceinline__ int nes_count_below(const double* d, const double* e2
 // lane; warp 0 narrows the smallest eigenvalue, warp 1 the largest). Bound by
 // the k - 2 dependent reflections: eight threads per row, two barriers a
 // reflection, the short sums taken by every warp redundantly so that they
-// need no barrier: 29 us at k = 16 (cyclic Jacobi rotations, k/2 disjoint ones
-// a round, took 105 us). One CTA.
+// need no barrier: 27 us at k = 16 with the four warps that its rows fill, 28.6
+// with sixteen (cyclic Jacobi rotations, k/2 disjoint ones a round, took
+// 105 us). One CTA.
 // Then lambda, q and 1/(L + lambda) of the update (ntfnes.hpp:114-117). For
 // mode 0 it also copies the proximal lambda to the previous one
 // (ntfnes.hpp:102-104).
 constexpr int NES_PREP_THREADS = 512;
+inline int nes_prep_threads(int k) { return k <= 8 ? 64 : (8 * k + 31) / 32 * 32; }
 __global__ void __launch_bounds__(NES_PREP_THREADS) k_nes_prep(const double* __restrict__ G, int k,
                                                   NesDev* __restrict__ st, int mode,
                                                   const double* __restrict__ prox_lam,
@@ -624,7 +626,7 @@ __global__ void __launch_bounds__(NES_PREP_THREADS) k_nes_prep(const double* __r
   __shared__ double ext[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (mode == 0 && tid < k) prev_lam[tid] = prox_lam[tid];
-  for (int e = tid; e < k * k; e += NES_PREP_THREADS) A[(e / k) * LD + e % k] = G[e];
+  for (int e = tid; e < k * k; e += blockDim.x) A[(e / k) * LD + e % k] = G[e];
   __syncthreads();
   const int row = tid >> 3, part = tid & 7;
   for (int j = 0; j + 2 < k; ++j) {

@@ -306,3 +306,29 @@ def test_dimtree_ttv_of_short_rows(gpu, oracle_lib, dims, k):
         Fn = _normalized(F)
         for n in range(len(dims)):
             assert rel(c.mttkrp(n, dimtree=True), oracle_lib.mttkrp_direct(X, Fn, n)) < TOL
+
+
+def _nnls_system(n, ncols, seed):
+    rng = np.random.default_rng(seed)
+    A = rng.random((3 * n, n)) * (rng.random((3 * n, n)) < 0.7)
+    A[np.arange(n), np.arange(n)] += 0.5
+    G = A.T @ A
+    X = rng.random((n, ncols)) * (rng.random((n, ncols)) < 0.5)
+    return G, G @ X + 0.1 * rng.standard_normal((n, ncols))
+
+
+# up to a few hundred right-hand sides: a CTA each; more: a warp each
+@pytest.mark.parametrize("n,ncols", [(1, 1), (2, 3), (15, 40), (16, 2500), (17, 40), (31, 7), (32, 1200),
+                                     (33, 40), (63, 5), (64, 200), (17, 3001), (33, 1500), (50, 700), (63, 701),
+                                     (64, 1000)])
+def test_bpp_shapes(gpu, oracle_lib, n, ncols):
+    G, B = _nnls_system(n, ncols, 90 + n)
+    Xo, Po, _ = oracle_lib.bpp_update(B.T.copy(), G)
+    with gpu.Context(0, "fp64") as c:
+        Xg, Pg, its = c.bpp_solve(G, B)
+    # the bar of the other BPP tests; masks outside near ties (1e-9) are equal
+    assert np.abs(Xg.T - Xo).max() <= 1e-9 * max(np.abs(Xo).max(), 1e-300)
+    Y = G @ Xg - B
+    tie = (np.abs(Y) < 1e-9) & (np.abs(Xg) < 1e-9)
+    assert np.array_equal(Pg[~tie], Po.T[~tie])
+    assert its.max() <= 5 * n

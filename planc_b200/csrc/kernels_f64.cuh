@@ -30,7 +30,13 @@ namespace pg {
 // tiles (a warp whose rows all lie past M skips its products). The next
 // reduction tile is loaded into registers while the current one is
 // multiplied out of shared memory, then stored into the other of two
-// shared-memory stages: one CTA barrier per tile. Dynamic shared memory:
+// shared-memory stages: one CTA barrier per tile. With RING (right contraction
+// of a single factor, rank above 16, even M and ldx and a 16-byte aligned X) the
+// tensor's tile goes to the other stage by 16-byte asynchronous copies instead,
+// which take its 16 registers a thread and its stores out of the products' way:
+// 512^3 rank 32, 341 -> 303 us. (The left contraction's tiles, and odd strides'
+// 8-byte copies, were no faster that way: 328 -> 343 us, and 8.6 -> 9.8 at
+// 61 x 47 x 33 x 29 rank 11.) Dynamic shared memory:
 // ct_smem_bytes<KP, LEFT>(). Shared-memory layouts are chosen so
 // that every fragment load is two 128-byte wavefronts (no bank conflicts):
 //   RIGHT: Xs[kk][m], row stride 128 + 4 doubles (X is m-contiguous);
@@ -136,11 +142,12 @@ __device__ __forceinline__ double wgen_at32(const WGen& wg, const FastDiv& f0, c
 // F_1[i1, r] * F_2[i2, r] with b = i1 + dim[1] i2 (NF = 3): a thread takes
 // tail once per tile, then one F_0 load and one multiply per entry (the same
 // products as wgen_at, so the same W).
-template <int KP, bool LEFT, int NF, bool RUNS = false>
+template <int KP, bool LEFT, int NF, bool RUNS = false, bool RING = false>
 __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restrict__ X,
                                                          ContractGeom g, WGen wg, int k,
                                                          double* __restrict__ out) {
   static_assert(!RUNS || (LEFT && (NF == 2 || NF == 3)), "runs of the fastest mode");
+  static_assert(!RING || !LEFT, "asynchronous copies of the right contraction's tiles");
   constexpr int BK = ct_bk<KP>();
   constexpr int XPT = BK * CT_BM / 256;  // X elements per thread per tile
   constexpr int WPT = (BK * KP + 255) / 256;
@@ -178,29 +185,48 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restric
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  double xr[XPT];
+  double xr[RING ? 1 : XPT];
   double wr[WPT];
 
-  auto load_tile = [&](int64_t t) {
+  auto load_tile = [&](int64_t t, int stage) {
+    if constexpr (RING) {
+      // rows kk = (tid >> 6) + 4 i of the tile, the pair mm = 2 (tid & 63): both
+      // of a pair lie inside the tensor or outside (zeros)
+      double* Xs = ct_smem + stage * STAGE;
+      const int64_t j0 = t * BK;
+      const int mm = 2 * (tid & 63);
+      const bool in = m0 + mm < g.M;
+#pragma unroll
+      for (int i = 0; i < BK / 4; ++i) {
+        const int kk = (tid >> 6) + 4 * i;
+        const bool ok = in && j0 + kk < g.A;
+        const double* src = ok ? X + (m0 + mm) + g.ldx * (j0 + kk) : X;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(Xs + kk * SX + mm)),
+                     "l"(src), "r"(ok ? 16 : 0) : "memory");
+      }
+    }
     if constexpr (!LEFT) {
       const int64_t j0 = t * BK;
-      const int64_t gm = m0 + (tid & 127);
-      const bool mrow = gm < g.M;
-      // rows kk = (tid >> 7) + 2 i of the tile through one running pointer
-      const int64_t jt = j0 + (tid >> 7);
-      const double* xp = X + gm + g.ldx * jt;
-      const int64_t xstep = 2 * g.ldx;
-      if (mrow && j0 + BK <= g.A) {
+      if constexpr (!RING) {
+        const int64_t gm = m0 + (tid & 127);
+        const bool mrow = gm < g.M;
+        // rows kk = (tid >> 7) + 2 i of the tile through one running pointer
+        const int64_t jt = j0 + (tid >> 7);
+        const double* xp = X + gm + g.ldx * jt;
+        const int64_t xstep = 2 * g.ldx;
+        if (mrow && j0 + BK <= g.A) {
 #pragma unroll
-        for (int i = 0; i < XPT; ++i) {
-          xr[i] = *xp;
-          xp += xstep;
-        }
-      } else {
+          for (int i = 0; i < XPT; ++i) {
+            xr[i] = *xp;
+            xp += xstep;
+          }
+        } else {
 #pragma unroll
-        for (int i = 0; i < XPT; ++i) {
-          xr[i] = (mrow && jt + 2 * i < g.A) ? *xp : 0.0;
-          xp += xstep;
+          for (int i = 0; i < XPT; ++i) {
+            xr[i] = (mrow && jt + 2 * i < g.A) ? *xp : 0.0;
+            xp += xstep;
+          }
         }
       }
       if constexpr (NF == 1) {
@@ -336,7 +362,9 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restric
   auto store_tile = [&](int stage) {
     double* Xs = ct_smem + stage * STAGE;
     double* Ws = Xs + XS_ELEMS;
-    if constexpr (!LEFT) {
+    if constexpr (RING) {
+      // the tile is on its way
+    } else if constexpr (!LEFT) {
       const int mm = tid & 127;
 #pragma unroll
       for (int i = 0; i < XPT; ++i) Xs[((tid >> 7) + 2 * i) * SX + mm] = xr[i];
@@ -353,14 +381,15 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restric
   };
 
   if (t_begin < t_end) {
-    load_tile(t_begin);
+    load_tile(t_begin, 0);
     store_tile(0);
   }
   for (int64_t t = t_begin; t < t_end; ++t) {
     const int stage = (int)((t - t_begin) & 1);
     // stage `stage` is complete and every warp is done with the other one
+    if constexpr (RING) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (t + 1 < t_end) load_tile(t + 1);
+    if (t + 1 < t_end) load_tile(t + 1, stage ^ 1);
     if (warp_live) {
       const double* Xs = ct_smem + stage * STAGE;
       const double* Ws = Xs + XS_ELEMS;

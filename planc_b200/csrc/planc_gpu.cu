@@ -666,6 +666,12 @@ void launch_contract_f64(dim3 grid, cudaStream_t st, const double* X, const Cont
       return;
     }
   }
+  if constexpr (!LEFT && KP >= 32) {
+    if (wg.nf == 1 && g.M % 2 == 0 && g.ldx % 2 == 0 && ((uintptr_t)X & 15) == 0) {
+      k_contract_f64<KP, false, 1, false, true><<<grid, 256, sm, st>>>(X, g, wg, k, dst);
+      return;
+    }
+  }
   switch (wg.nf) {
     case 1: k_contract_f64<KP, LEFT, 1><<<grid, 256, sm, st>>>(X, g, wg, k, dst); break;
     case 2: k_contract_f64<KP, LEFT, 2><<<grid, 256, sm, st>>>(X, g, wg, k, dst); break;
@@ -681,6 +687,8 @@ void contract_f64_attrs_kp() {
   CK(cudaFuncSetAttribute(k_contract_f64<KP, LEFT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   CK(cudaFuncSetAttribute(k_contract_f64<KP, LEFT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   CK(cudaFuncSetAttribute(k_contract_f64<KP, LEFT, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+  if constexpr (!LEFT && KP >= 32)
+    CK(cudaFuncSetAttribute(k_contract_f64<KP, false, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   if constexpr (LEFT) {
     CK(cudaFuncSetAttribute(k_contract_f64<KP, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     CK(cudaFuncSetAttribute(k_contract_f64<KP, true, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));

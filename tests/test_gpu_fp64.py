@@ -332,3 +332,18 @@ def test_bpp_shapes(gpu, oracle_lib, n, ncols):
     tie = (np.abs(Y) < 1e-9) & (np.abs(Xg) < 1e-9)
     assert np.array_equal(Pg[~tie], Po.T[~tie])
     assert its.max() <= 5 * n
+
+
+@pytest.mark.parametrize("dims,k", [((64, 6, 5), 32), ((66, 34, 66), 17), ((65, 34, 64), 32), ((64, 33, 37), 33),
+                                    ((130, 129, 31), 64), ((2, 32, 70), 20), ((62, 4, 258), 24)])
+def test_contraction_of_the_last_mode(gpu, oracle_lib, dims, k):
+    # ranks 17 to 64, where whole 16-byte pieces of X are copied when the rows
+    # allow it (even extents) and single values when not; extents either side of
+    # the tiles, few and many steps of the contracted mode
+    X, _ = cp_tensor(dims, 3, seed=9)
+    F = init_factors(dims, k, seed=10)
+    with _ctx(gpu, X, F) as c:
+        Fn = _normalized(F)
+        for n in range(len(dims)):
+            for dimtree in (False, True):
+                assert rel(c.mttkrp(n, dimtree=dimtree), oracle_lib.mttkrp_direct(X, Fn, n)) < TOL

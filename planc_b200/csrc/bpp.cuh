@@ -12,11 +12,24 @@
 // Gaussian elimination with partial pivoting when the Cholesky meets a
 // non-positive pivot.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace pg {
 
 constexpr int BPP_WARPS = 2;  // right-hand sides per CTA (they share the AtA copy)
+
+// Places of a Cholesky factor's strict lower triangle, column by column: with
+// a leading dimension, or packed for an m-row factor (column c from row c + 1).
+struct FactorLd {
+  int ld;
+  __device__ __forceinline__ int base(int c) const { return ld * c; }
+};
+struct FactorPacked {
+  int m;
+  __device__ __forceinline__ int base(int c) const { return c * (m - 2) - ((c * (c - 1)) >> 1) - 1; }
+};
 
 __device__ __forceinline__ uint64_t warp_mask64(bool pred_lo, bool pred_hi) {
   uint64_t lo = __ballot_sync(0xffffffffu, pred_lo);
@@ -25,9 +38,9 @@ __device__ __forceinline__ uint64_t warp_mask64(bool pred_lo, bool pred_hi) {
 }
 
 // Blocked left-looking (Crout) Cholesky of the passive principal submatrix
-// A(i,j) = AtA[idx[i] + n*idx[j]], i,j < m, into Ls (column-major, leading
-// dimension KP+1: odd, so that walking a row and walking a column are both
-// free of shared-memory bank conflicts). Lane l owns rows l and l+32 of the
+// A(i,j) = AtA[idx[i] + n*idx[j]], i,j < m, into Ls (entry (i, c) at
+// place.base(c) + i; with an odd leading dimension walking a row and walking a
+// column are both free of shared-memory bank conflicts). Lane l owns rows l and l+32 of the
 // factor; inv[q] receives 1/L(row,row) for its rows. Columns go in panels of
 // NB: first every owned row at or below the panel takes the contribution of
 // all finished columns to the NB panel columns (NB independent accumulators
@@ -36,10 +49,11 @@ __device__ __forceinline__ uint64_t warp_mask64(bool pred_lo, bool pred_hi) {
 // travelling by shuffle. Only the strict lower triangle is stored.
 // Returns false when a pivot is not positive and finite (uniform across the
 // warp), where the reference's Cholesky solve fails too.
-template <int KP>
+template <int KP, typename Place>
 __device__ __forceinline__ bool warp_chol_crout(const double* __restrict__ AtA, int n, const int* idx,
-                                                int m, double* Ls, double (&inv)[KP > 32 ? 2 : 1]) {
-  constexpr int LD = KP + 1, R = KP > 32 ? 2 : 1, NB = 8;
+                                                int m, double* Ls, const Place place,
+                                                double (&inv)[KP > 32 ? 2 : 1]) {
+  constexpr int R = KP > 32 ? 2 : 1, NB = 8;
   const int lane = threadIdx.x & 31;
   int gi[R];
 #pragma unroll
@@ -57,14 +71,15 @@ __device__ __forceinline__ bool warp_chol_crout(const double* __restrict__ AtA, 
       for (int t = 0; t < NB; ++t) acc[q][t] = 0.0;
     // contribution of the finished columns c < j0
     for (int c = 0; c < j0; ++c) {
+      const double* Lc = Ls + place.base(c);
       double lj[NB];
 #pragma unroll
-      for (int t = 0; t < NB; ++t) lj[t] = t < pw ? Ls[j0 + t + LD * c] : 0.0;
+      for (int t = 0; t < NB; ++t) lj[t] = t < pw ? Lc[j0 + t] : 0.0;
 #pragma unroll
       for (int q = 0; q < R; ++q) {
         const int row = lane + 32 * q;
         if (32 * q + 31 >= j0) {  // warp-uniform: some owned row of this slot is in play
-          const double li = (row >= j0 && row < m) ? Ls[row + LD * c] : 0.0;
+          const double li = (row >= j0 && row < m) ? Lc[row] : 0.0;
 #pragma unroll
           for (int t = 0; t < NB; ++t) acc[q][t] = fma(li, lj[t], acc[q][t]);
         }
@@ -94,7 +109,7 @@ __device__ __forceinline__ bool warp_chol_crout(const double* __restrict__ AtA, 
         for (int q = 0; q < R; ++q) {
           const int row = lane + 32 * q;
           lcol[q] = acc[q][t] * ij;
-          if (row > jj && row < m) Ls[row + LD * jj] = lcol[q];
+          if (row > jj && row < m) Ls[place.base(jj) + row] = lcol[q];
           if (row == jj) inv[q] = ij;
         }
 #pragma unroll
@@ -117,19 +132,24 @@ __device__ __forceinline__ bool warp_chol_crout(const double* __restrict__ AtA, 
 // owned rows' right-hand side) becomes the solution in place. Each step is
 // one shuffle of the finished entry plus one fused multiply-add per owned
 // row; the factor entries are independent loads that the compiler hoists.
-template <int KP>
-__device__ __forceinline__ void warp_chol_subst(const double* Ls, int m, const double (&inv)[KP > 32 ? 2 : 1],
-                                double (&z)[KP > 32 ? 2 : 1]) {
-  constexpr int LD = KP + 1, R = KP > 32 ? 2 : 1;
+template <int KP, typename Place>
+__device__ __forceinline__ void warp_chol_subst(const double* Ls, int m, const Place place,
+                                                const double (&inv)[KP > 32 ? 2 : 1],
+                                                double (&z)[KP > 32 ? 2 : 1]) {
+  constexpr int R = KP > 32 ? 2 : 1;
   const int lane = threadIdx.x & 31;
+  int mine[R];  // place of the owned rows' columns
+#pragma unroll
+  for (int q = 0; q < R; ++q) mine[q] = place.base(lane + 32 * q);
   for (int j = 0; j < m; ++j) {  // L y = z
     const double t = j < 32 ? z[0] * inv[0] : z[R - 1] * inv[R - 1];
     const double yj = __shfl_sync(0xffffffffu, t, j & 31);
+    const double* Lj = Ls + place.base(j);
 #pragma unroll
     for (int q = 0; q < R; ++q) {
       const int row = lane + 32 * q;
       if (row == j) z[q] = yj;
-      else if (row > j && row < m) z[q] = fma(-Ls[row + LD * j], yj, z[q]);
+      else if (row > j && row < m) z[q] = fma(-Lj[row], yj, z[q]);
     }
   }
   for (int j = m - 1; j >= 0; --j) {  // L^T x = y
@@ -139,7 +159,7 @@ __device__ __forceinline__ void warp_chol_subst(const double* Ls, int m, const d
     for (int q = 0; q < R; ++q) {
       const int row = lane + 32 * q;
       if (row == j) z[q] = xj;
-      else if (row < j) z[q] = fma(-Ls[j + LD * row], xj, z[q]);
+      else if (row < j) z[q] = fma(-Ls[mine[q] + j], xj, z[q]);
     }
   }
 }
@@ -194,6 +214,25 @@ __device__ __forceinline__ int warp_lu_solve(double* A, int ld, int m, double* z
   return 0;
 }
 
+constexpr int kBppNeedLu = -100;  // internal: the passive system needs the general solver
+
+// doubles of the packed factor of an n-row system (even)
+__host__ __device__ constexpr int bpp_pack_factor(int n) { return (n * (n - 1) / 2 + 2) & ~1; }
+constexpr size_t bpp_pack_smem(int KP, int n, int warps) {
+  return ((size_t)n * n + (size_t)warps * (bpp_pack_factor(n) + 4 * KP)) * 8 + (size_t)warps * KP * 4;
+}
+// Warps of a PACK CTA (one per SM): as many as 227 KB hold, evened out over the
+// rounds that the right-hand sides take, so that no SM idles while others
+// finish (n = 50, 700 of them: 205 us with 16 warps on 44 SMs, 164 with 5).
+constexpr int BPP_PACK_MOST = 16;
+inline int bpp_pack_warps(int KP, int n, int64_t ncols, int sms) {
+  int w = BPP_PACK_MOST;
+  while (w > 1 && bpp_pack_smem(KP, n, w) > 226 * 1024) --w;
+  const int64_t rounds = (ncols + (int64_t)sms * w - 1) / ((int64_t)sms * w);
+  const int64_t even = (ncols + sms * rounds - 1) / (sms * rounds);
+  return (int)(even < 2 ? 2 : even);
+}
+
 // One warp per right-hand side c, BPP_WARPS right-hand sides per CTA: AtA
 // (n x n) is staged once in shared memory for all warps of the CTA; rhs
 // b_c = B[c*n .. c*n+n-1] (row-major ncols x n == column-major n x ncols),
@@ -206,17 +245,35 @@ __host__ __device__ constexpr size_t bpp_smem_bytes(int KP) {
   return (size_t)KP * KP * 8 + (size_t)BPP_WARPS * ((size_t)KP * (KP + 1) * 8 + 4 * KP * 8 + KP * 4);
 }
 
-template <int KP>
-__global__ void __launch_bounds__(32 * BPP_WARPS, 1) k_bpp(const double* __restrict__ AtA_g,
-                                                        const double* __restrict__ Bm, int n,
-                                                        int64_t ncols, double* __restrict__ Xout,
-                                                        int* __restrict__ passive_out,
-                                                        int* __restrict__ iters_out,
-                                                        int* __restrict__ status, int max_iter_override,
-                                                        const double* __restrict__ Pinit) {
+// PACK: for many right-hand sides above rank 32, where the factors' shared
+// memory limits the warps an SM holds and each warp is one chain of dependent
+// steps. The factor is packed (its strict lower triangle) and AtA is shared by
+// up to 16 warps, which take the right-hand sides in turn: 16 warps an SM in
+// place of 4 at n = 50 (bpp_pack_warps), with which the FP64 and shared-memory
+// pipes are what bounds it. A passive system that is not positive definite
+// needs a full square for the general solver: the right-hand side is left
+// untouched and flagged in need_lu, and a launch without PACK, over the flagged
+// ones only, follows. Values are those of the plain form. Right-hand sides at
+// n = 50: 3000, 567 -> 409 us; 20000, 3310 -> 2140 us. Up to rank 32 the plain
+// form already holds 16 warps an SM and is faster (n = 24, 3000: 81 us against
+// 120).
+template <int KP, bool PACK>
+__global__ void __launch_bounds__(PACK ? 32 * BPP_PACK_MOST : 32 * BPP_WARPS, 1)
+    k_bpp(const double* __restrict__ AtA_g, const double* __restrict__ Bm, int n, int64_t ncols,
+          double* __restrict__ Xout, int* __restrict__ passive_out, int* __restrict__ iters_out,
+          int* __restrict__ status, int max_iter_override, const double* __restrict__ Pinit,
+          int* __restrict__ need_lu) {
   constexpr int LD = KP + 1, R = KP > 32 ? 2 : 1;
   extern __shared__ __align__(16) unsigned char bpp_smem[];
   double* AtA = reinterpret_cast<double*>(bpp_smem);  // n x n, leading dimension n
+  if (!PACK && need_lu) {  // nothing flagged among this CTA's right-hand sides
+    bool any = false;
+    for (int q = 0; q < BPP_WARPS; ++q) {
+      const int64_t c = (int64_t)blockIdx.x * BPP_WARPS + q;
+      any |= c < ncols && need_lu[c];
+    }
+    if (!any) return;
+  }
   {
     const int nn = n * n;
     for (int e0 = threadIdx.x; e0 < nn; e0 += 8 * blockDim.x) {
@@ -235,165 +292,178 @@ __global__ void __launch_bounds__(32 * BPP_WARPS, 1) k_bpp(const double* __restr
   }
   __syncthreads();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* Ls = AtA + KP * KP + (size_t)w * (KP * LD + 4 * KP);
-  double* x = Ls + KP * LD;
+  const int nw = PACK ? (int)(blockDim.x >> 5) : BPP_WARPS;
+  const int fac = PACK ? bpp_pack_factor(n) : KP * LD;  // doubles of a warp's factor
+  double* Ls = AtA + (PACK ? n * n : KP * KP) + (size_t)w * (fac + 4 * KP);
+  double* x = Ls + fac;
   double* y = x + KP;
   double* b = y + KP;
   double* zs = b + KP;
-  int* idx = reinterpret_cast<int*>(AtA + KP * KP + (size_t)BPP_WARPS * (KP * LD + 4 * KP)) + w * KP;
-  const int64_t c = (int64_t)blockIdx.x * BPP_WARPS + w;
-  if (c >= ncols) return;  // whole warp leaves together (no CTA barrier follows)
-  const bool has_lo = lane < n, has_hi = lane + 32 < n;
-  for (int i = lane; i < n; i += 32) {
-    b[i] = Bm[c * n + i];
-    x[i] = 0.0;
-    y[i] = -b[i];  // Y = AtA*0 - AtB, bppnnls.hpp:73
-  }
-  __syncwarp();
-  uint64_t passive = 0;  // PassiveSet = (X > 0) = {}, bppnnls.hpp:74
-  const int pbar = 3;
-  int P = pbar, Ninf = n + 1;  // bppnnls.hpp:76-81
-  // bppnnls.hpp:69 (MAX_ITERATIONS = 5n); a positive override lowers the cap
-  const unsigned max_it = max_iter_override > 0 ? (unsigned)max_iter_override : 5u * (unsigned)n;
-  auto classify = [&](uint64_t& nonopt, uint64_t& infea) {
-    bool lo_no = has_lo && (y[lane] < 0) && !((passive >> lane) & 1);
-    bool hi_no = has_hi && (y[lane + 32] < 0) && !((passive >> (lane + 32)) & 1);
-    bool lo_in = has_lo && (x[lane] < 0) && ((passive >> lane) & 1);
-    bool hi_in = has_hi && (x[lane + 32] < 0) && ((passive >> (lane + 32)) & 1);
-    nonopt = warp_mask64(lo_no, hi_no);
-    infea = warp_mask64(lo_in, hi_in);
-  };
-  // X(P) = solve(AtA(P,P), AtB(P)), X(~P) = 0, Y = AtA X - AtB and the 1e-12
-  // zeroing for the current passive set; returns 0 or a failure status
-  auto solve_passive = [&]() -> int {
-    int bad = 0;
-    // solve the passive system AtA(P,P) x_P = AtB(P), bppnnls.hpp:163-166 / 204-259
-    const int m = __popcll(passive);
-    // idx[q] = position of the q-th passive index (warp-parallel compaction)
-    if ((passive >> lane) & 1) idx[__popcll(passive & ((1ull << lane) - 1ull))] = lane;
-    if ((passive >> (lane + 32)) & 1)
-      idx[__popcll(passive & ((1ull << (lane + 32)) - 1ull))] = lane + 32;
-    __syncwarp();
-    double z[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int row = lane + 32 * q;
-      z[q] = row < m ? b[idx[row]] : 0.0;
-    }
-    double inv[R];
-    if (m > 0) {
-      if (warp_chol_crout<KP>(AtA, n, idx, m, Ls, inv)) {
-        warp_chol_subst<KP>(Ls, m, inv, z);
-      } else {  // not positive definite: the general solver, as arma::solve falls back
-        for (int e = lane; e < m * m; e += 32) {
-          const int ii = e % m, jj = e / m;
-          Ls[ii + LD * jj] = AtA[idx[ii] + n * idx[jj]];
-        }
-        for (int i = lane; i < m; i += 32) zs[i] = b[idx[i]];
-        __syncwarp();
-        const int rc = warp_lu_solve(Ls, LD, m, zs);
-        if (rc != 0) return rc;
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-          const int row = lane + 32 * q;
-          z[q] = row < m ? zs[row] : 0.0;
-        }
-      }
-    }
-    // scatter: X(P) = x_P, X(~P) = 0
-    for (int i = lane; i < n; i += 32) x[i] = 0.0;
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int row = lane + 32 * q;
-      if (row < m) {
-        x[idx[row]] = z[q];
-        zs[row] = z[q];
-      }
-    }
-    __syncwarp();
-    // Y = AtA*X - AtB over the passive columns (bppnnls.hpp:167-168), then the
-    // 1e-12 zeroing of X and Y (bppnnls.hpp:170-172)
+  int* idx = reinterpret_cast<int*>(AtA + (PACK ? n * n : KP * KP) + (size_t)nw * (fac + 4 * KP)) + w * KP;
+  // whole warps leave or go on together (no CTA barrier follows)
+  for (int64_t c = (int64_t)blockIdx.x * nw + w; c < ncols; c += PACK ? (int64_t)gridDim.x * nw : ncols) {
+    if (!PACK && need_lu && !need_lu[c]) return;
+    const bool has_lo = lane < n, has_hi = lane + 32 < n;
     for (int i = lane; i < n; i += 32) {
-      double a0 = 0.0, a1 = 0.0;
-      int q = 0;
-      for (; q + 2 <= m; q += 2) {
-        a0 = fma(AtA[i + n * idx[q]], zs[q], a0);
-        a1 = fma(AtA[i + n * idx[q + 1]], zs[q + 1], a1);
-      }
-      if (q < m) a0 = fma(AtA[i + n * idx[q]], zs[q], a0);
-      const double yi = (a0 + a1) - b[i];
-      y[i] = (fabs(yi) < kEps12) ? 0.0 : yi;
-      const double xi = x[i];
-      if (!isfinite(xi) || !isfinite(yi)) bad = kStNonFinite;
-      x[i] = (fabs(xi) < kEps12) ? 0.0 : xi;
+      b[i] = Bm[c * n + i];
+      x[i] = 0.0;
+      y[i] = -b[i];  // Y = AtA*0 - AtB, bppnnls.hpp:73
     }
     __syncwarp();
-    __syncwarp();
-    return __reduce_min_sync(0xffffffffu, bad);
-  };
-  unsigned iter = 0;
-  int st = 0;
-  if (Pinit) {
-    // warm start from the previous solution's passive set: with AtA positive
-    // definite BPP reaches the unique NNLS optimum from any starting set (Kim
-    // & Park), so the result is the reference's; only the number of exchange
-    // steps changes. When AtA is singular (a component whose factor column
-    // collapsed to zero leaves a zero row and column) the optimum is not
-    // unique and the warm set's system may be singular: a failed warm solve
-    // restarts from the reference's start, X = 0 (bppnnls.hpp:73-74).
-    const bool lo = has_lo && Pinit[c * n + lane] > 0.0;
-    const bool hi = has_hi && Pinit[c * n + lane + 32] > 0.0;
-    passive = warp_mask64(lo, hi);
-    __syncwarp();  // every lane has read its Pinit before any store below
-    if (passive) {
-      ++iter;
-      st = solve_passive();
-      if (st != 0) {
-        st = 0;
-        iter = 0;
-        passive = 0;
-        for (int i = lane; i < n; i += 32) {
-          x[i] = 0.0;
-          y[i] = -b[i];
+    uint64_t passive = 0;  // PassiveSet = (X > 0) = {}, bppnnls.hpp:74
+    const int pbar = 3;
+    int P = pbar, Ninf = n + 1;  // bppnnls.hpp:76-81
+    // bppnnls.hpp:69 (MAX_ITERATIONS = 5n); a positive override lowers the cap
+    const unsigned max_it = max_iter_override > 0 ? (unsigned)max_iter_override : 5u * (unsigned)n;
+    auto classify = [&](uint64_t& nonopt, uint64_t& infea) {
+      bool lo_no = has_lo && (y[lane] < 0) && !((passive >> lane) & 1);
+      bool hi_no = has_hi && (y[lane + 32] < 0) && !((passive >> (lane + 32)) & 1);
+      bool lo_in = has_lo && (x[lane] < 0) && ((passive >> lane) & 1);
+      bool hi_in = has_hi && (x[lane + 32] < 0) && ((passive >> (lane + 32)) & 1);
+      nonopt = warp_mask64(lo_no, hi_no);
+      infea = warp_mask64(lo_in, hi_in);
+    };
+    // X(P) = solve(AtA(P,P), AtB(P)), X(~P) = 0, Y = AtA X - AtB and the 1e-12
+    // zeroing for the current passive set; returns 0 or a failure status
+    auto solve_passive = [&]() -> int {
+      int bad = 0;
+      // solve the passive system AtA(P,P) x_P = AtB(P), bppnnls.hpp:163-166 / 204-259
+      const int m = __popcll(passive);
+      // idx[q] = position of the q-th passive index (warp-parallel compaction)
+      if ((passive >> lane) & 1) idx[__popcll(passive & ((1ull << lane) - 1ull))] = lane;
+      if ((passive >> (lane + 32)) & 1)
+        idx[__popcll(passive & ((1ull << (lane + 32)) - 1ull))] = lane + 32;
+      __syncwarp();
+      double z[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int row = lane + 32 * q;
+        z[q] = row < m ? b[idx[row]] : 0.0;
+      }
+      double inv[R];
+      if (m > 0) {
+        using Place = typename std::conditional<PACK, FactorPacked, FactorLd>::type;
+        const Place place{PACK ? m : LD};
+        if (warp_chol_crout<KP>(AtA, n, idx, m, Ls, place, inv)) {
+          warp_chol_subst<KP>(Ls, m, place, inv, z);
+        } else if constexpr (PACK) {
+          return kBppNeedLu;
+        } else {  // not positive definite: the general solver, as arma::solve falls back
+          for (int e = lane; e < m * m; e += 32) {
+            const int ii = e % m, jj = e / m;
+            Ls[ii + LD * jj] = AtA[idx[ii] + n * idx[jj]];
+          }
+          for (int i = lane; i < m; i += 32) zs[i] = b[idx[i]];
+          __syncwarp();
+          const int rc = warp_lu_solve(Ls, LD, m, zs);
+          if (rc != 0) return rc;
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < R; ++q) {
+            const int row = lane + 32 * q;
+            z[q] = row < m ? zs[row] : 0.0;
+          }
         }
-        __syncwarp();
+      }
+      // scatter: X(P) = x_P, X(~P) = 0
+      for (int i = lane; i < n; i += 32) x[i] = 0.0;
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int row = lane + 32 * q;
+        if (row < m) {
+          x[idx[row]] = z[q];
+          zs[row] = z[q];
+        }
+      }
+      __syncwarp();
+      // Y = AtA*X - AtB over the passive columns (bppnnls.hpp:167-168), then the
+      // 1e-12 zeroing of X and Y (bppnnls.hpp:170-172)
+      for (int i = lane; i < n; i += 32) {
+        double a0 = 0.0, a1 = 0.0;
+        int q = 0;
+        for (; q + 2 <= m; q += 2) {
+          a0 = fma(AtA[i + n * idx[q]], zs[q], a0);
+          a1 = fma(AtA[i + n * idx[q + 1]], zs[q + 1], a1);
+        }
+        if (q < m) a0 = fma(AtA[i + n * idx[q]], zs[q], a0);
+        const double yi = (a0 + a1) - b[i];
+        y[i] = (fabs(yi) < kEps12) ? 0.0 : yi;
+        const double xi = x[i];
+        if (!isfinite(xi) || !isfinite(yi)) bad = kStNonFinite;
+        x[i] = (fabs(xi) < kEps12) ? 0.0 : xi;
+      }
+      __syncwarp();
+      __syncwarp();
+      return __reduce_min_sync(0xffffffffu, bad);
+    };
+    unsigned iter = 0;
+    int st = 0;
+    if (Pinit) {
+      // warm start from the previous solution's passive set: with AtA positive
+      // definite BPP reaches the unique NNLS optimum from any starting set (Kim
+      // & Park), so the result is the reference's; only the number of exchange
+      // steps changes. When AtA is singular (a component whose factor column
+      // collapsed to zero leaves a zero row and column) the optimum is not
+      // unique and the warm set's system may be singular: a failed warm solve
+      // restarts from the reference's start, X = 0 (bppnnls.hpp:73-74).
+      const bool lo = has_lo && Pinit[c * n + lane] > 0.0;
+      const bool hi = has_hi && Pinit[c * n + lane + 32] > 0.0;
+      passive = warp_mask64(lo, hi);
+      __syncwarp();  // every lane has read its Pinit before any store below
+      if (passive) {
+        ++iter;
+        st = solve_passive();
+        if (st != 0 && st != kBppNeedLu) {
+          st = 0;
+          iter = 0;
+          passive = 0;
+          for (int i = lane; i < n; i += 32) {
+            x[i] = 0.0;
+            y[i] = -b[i];
+          }
+          __syncwarp();
+        }
       }
     }
-  }
-  uint64_t nonopt = 0, infea = 0;
-  int notgood = 0;
-  if (st == 0) {
-    classify(nonopt, infea);
-    notgood = __popcll(nonopt) + __popcll(infea);
-  }
-  while (st == 0 && notgood > 0) {
-    ++iter;
-    if (iter > max_it) { st = kStBppMaxIter; break; }
-    if (notgood < Ninf) {  // Cols1, bppnnls.hpp:109, 115-129
-      P = pbar;
-      Ninf = notgood;
-      passive = (passive | nonopt) & ~infea;
-    } else if (P >= 1) {  // Cols2, bppnnls.hpp:110, 133-146
-      P -= 1;
-      passive = (passive | nonopt) & ~infea;
-    } else {  // backup rule: flip the largest offending index, bppnnls.hpp:149-160
-      int rowidx = 63 - __clzll(nonopt | infea);
-      passive ^= (1ull << rowidx);
+    uint64_t nonopt = 0, infea = 0;
+    int notgood = 0;
+    if (st == 0) {
+      classify(nonopt, infea);
+      notgood = __popcll(nonopt) + __popcll(infea);
     }
-    st = solve_passive();
-    if (st != 0) break;
-    classify(nonopt, infea);
-    notgood = __popcll(nonopt) + __popcll(infea);
-  }
-  for (int i = lane; i < n; i += 32) {
-    Xout[c * n + i] = x[i];
-    if (passive_out) passive_out[c * n + i] = (int)((passive >> i) & 1);
-  }
-  if (lane == 0) {
-    if (iters_out) iters_out[c] = (int)iter;
-    if (st != 0) atomicMin(status, st);
+    while (st == 0 && notgood > 0) {
+      ++iter;
+      if (iter > max_it) { st = kStBppMaxIter; break; }
+      if (notgood < Ninf) {  // Cols1, bppnnls.hpp:109, 115-129
+        P = pbar;
+        Ninf = notgood;
+        passive = (passive | nonopt) & ~infea;
+      } else if (P >= 1) {  // Cols2, bppnnls.hpp:110, 133-146
+        P -= 1;
+        passive = (passive | nonopt) & ~infea;
+      } else {  // backup rule: flip the largest offending index, bppnnls.hpp:149-160
+        int rowidx = 63 - __clzll(nonopt | infea);
+        passive ^= (1ull << rowidx);
+      }
+      st = solve_passive();
+      if (st != 0) break;
+      classify(nonopt, infea);
+      notgood = __popcll(nonopt) + __popcll(infea);
+    }
+    if (PACK) {
+      if (lane == 0) need_lu[c] = st == kBppNeedLu;
+      if (st == kBppNeedLu) continue;
+    }
+    for (int i = lane; i < n; i += 32) {
+      Xout[c * n + i] = x[i];
+      if (passive_out) passive_out[c * n + i] = (int)((passive >> i) & 1);
+    }
+    if (lane == 0) {
+      if (iters_out) iters_out[c] = (int)iter;
+      if (st != 0) atomicMin(status, st);
+    }
+    __syncwarp();  // the next right-hand side reuses this one's buffers
   }
 }
 

@@ -213,6 +213,8 @@ struct planc_gpu_ctx {
   double kms[KC_COUNT] = {0};
   int64_t klaunch[KC_COUNT] = {0};
   int64_t launch_count = 0;
+  int* bpp_lu = nullptr;  // right-hand sides left to the general solver (k_bpp)
+  int64_t bpp_lu_cap = 0;
   int bpp_max_iter = 0;  // 0: the reference's 5k cap
   bool bpp_warm = true;  // ANLS/BPP rows start from the replaced factor's passive set
   int bpp_kernel = 0;    // 0: by size, 1: a warp per right-hand side, 2: a CTA per right-hand side
@@ -276,12 +278,23 @@ void launch_bpp(planc_gpu_ctx* c, const double* AtA, const double* B, int n, int
     return;
   }
   const unsigned blocks = (unsigned)((ncols + BPP_WARPS - 1) / BPP_WARPS);
+  int* lu = nullptr;
+  if (kp == 64 && c->bpp_lu_cap >= ncols) {
+    // packed factors first, then the right-hand sides whose passive system
+    // was not positive definite
+    lu = c->bpp_lu;
+    const int w = bpp_pack_warps(kp, n, ncols, c->sm_count);
+    const unsigned grid = (unsigned)std::min<int64_t>((ncols + w - 1) / w, c->sm_count);
+    k_bpp<64, true><<<grid, 32 * w, bpp_pack_smem(kp, n, w), c->stream>>>(
+        AtA, B, n, ncols, X, P, I, c->status_dev, c->bpp_max_iter, warm, lu);
+    CK(cudaGetLastError());
+    c->launch_count++;
+  }
   switch (kp) {
 #define CASE(KP)                                                                                    \
   case KP:                                                                                          \
-    k_bpp<KP><<<blocks, 32 * BPP_WARPS, bpp_smem_bytes(KP), c->stream>>>(AtA, B, n, ncols, X, P, I, \
-                                                                         c->status_dev,             \
-                                                                         c->bpp_max_iter, warm);    \
+    k_bpp<KP, false><<<blocks, 32 * BPP_WARPS, bpp_smem_bytes(KP), c->stream>>>(                    \
+        AtA, B, n, ncols, X, P, I, c->status_dev, c->bpp_max_iter, warm, lu);                       \
     break;
     CASE(8) CASE(16) CASE(32) CASE(64)
 #undef CASE
@@ -296,6 +309,15 @@ void dalloc(T** p, size_t n) {
   }
   if (n == 0) return;
   CK(cudaMalloc((void**)p, n * sizeof(T)));
+}
+
+// Flags of the batched BPP for ncols right-hand sides (outside graph capture).
+void ensure_bpp_lu(planc_gpu_ctx* c, int64_t ncols) {
+  if (c->bpp_lu_cap >= ncols) return;
+  c->bpp_lu_cap = 0;
+  dalloc(&c->bpp_lu, (size_t)ncols);
+  c->bpp_lu_cap = ncols;
+  c->buf_epoch++;
 }
 
 cudaEvent_t get_event(planc_gpu_ctx* c) {
@@ -1554,6 +1576,7 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
   const int k = c->k;
   int64_t maxI = 1;
   for (int n = 0; n < c->N; ++n) maxI = std::max(maxI, c->dims[n]);
+  if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(c, maxI);
   if (algo == PLANC_GPU_AOADMM && !c->admm_ready) {
     for (int n = 0; n < c->N; ++n) {
       dalloc(&c->aux[n], (size_t)c->dims[n] * k);
@@ -1674,6 +1697,8 @@ void free_all(planc_gpu_ctx* c) {
   c->scratch_elems = 0;
   f(c->errs_dev);
   c->errs_cap = 0;
+  f(c->bpp_lu);
+  c->bpp_lu_cap = 0;
   f(c->counter_dev);
   f(c->status_dev);
 }
@@ -1705,10 +1730,11 @@ int planc_gpu_create(planc_gpu_ctx** out, int device, int precision, void* cuda_
       // k_bpp<64> needs more than the default 48 KB of dynamic shared memory
       static bool attrs_set[64] = {false};
       if (device < 64 && !attrs_set[device]) {
-        CK(cudaFuncSetAttribute(k_bpp<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CK(cudaFuncSetAttribute(k_bpp<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)bpp_smem_bytes(64)));
-        CK(cudaFuncSetAttribute(k_bpp<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CK(cudaFuncSetAttribute(k_bpp<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)bpp_smem_bytes(32)));
+        CK(cudaFuncSetAttribute(k_bpp<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         contract_f64_attrs(device);
         CK(cudaFuncSetAttribute(k_bpp_cta<64, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)BppCta<64, 8>::SMEM));
@@ -2250,6 +2276,7 @@ int planc_gpu_bpp_solve(planc_gpu_ctx* c, const double* AtA, const double* AtB, 
     if (ncols < 0) fail(PLANC_GPU_ERR_ARG, "ncols < 0");
     if (ncols == 0) return;
     set_device(c);
+    ensure_bpp_lu(c, ncols);
     // one workspace for operands and results, kept by the context: five
     // allocations and frees a call cost several times the solve
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -2307,6 +2334,11 @@ int planc_gpu_update_device(planc_gpu_ctx* c, int algo, double* H, const double*
       });
       return;
     }
+    // the flags' buffer grows here, except while the stream is captured (the
+    // solves then run in their plain form)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(c->stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone) ensure_bpp_lu(c, rows);
     launch(c, KC_BPP, [&] {
       launch_bpp(c, G, M, k, rows, H, nullptr, nullptr, c->bpp_warm ? H : nullptr);
     });
@@ -2717,10 +2749,11 @@ int64_t batch_epoch(const planc_gpu_batch* b) {
 }
 
 // every buffer the batch graph will reference, allocated before capture
-void batch_ensure(planc_gpu_batch* b, int iters, bool err) {
+void batch_ensure(planc_gpu_batch* b, int algo, int iters, bool err) {
   for (auto* m : b->members) {
     ensure_buffers(m);
     ensure_errs(m, err ? iters : 1);
+    if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(m, *std::max_element(m->dims, m->dims + m->N));
   }
   if (b->g_epoch != batch_epoch(b)) batch_reset_graph(b);
 }
@@ -3302,7 +3335,7 @@ int planc_gpu_batch_run(planc_gpu_batch* b, int algo, int iters, int compute_err
     if (iters <= 0) return;
     CK(cudaSetDevice(b->device));
     const bool err = compute_error != 0;
-    batch_ensure(b, iters, err);
+    batch_ensure(b, algo, iters, err);
     if (!b->gexec || b->g_algo != algo || b->g_err != (int)err) batch_capture(b, algo, err);
     batch_prepare(b);
     for (int it = 0; it < iters; ++it) CK(cudaGraphLaunch(b->gexec, b->master));
@@ -3355,7 +3388,7 @@ int planc_gpu_batch_autotune(planc_gpu_batch* b, int algo, int trials, double* b
         m->par_scale = scale[batch_class(m)];
         m->left_chunks = lch[batch_class(m)];
       }
-      batch_ensure(b, 1, false);
+      batch_ensure(b, algo, 1, false);
       batch_capture(b, algo, false);
       batch_prepare(b);
       CK(cudaGraphLaunch(b->gexec, b->master));  // warm-up
@@ -3887,6 +3920,7 @@ int planc_gpu_nmf_run(planc_gpu_ctx* c, int algo, int iters, double* objective,
     if (iters == 0) return;
     set_device(c);
     ensure_nmf(c, iters);
+    if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(c, std::max(c->dims[0], c->dims[1]));
     if (c->nmf_gepoch != c->buf_epoch && c->nmf_gexec) {
       cudaGraphExecDestroy(c->nmf_gexec);
       c->nmf_gexec = nullptr;

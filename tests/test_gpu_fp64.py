@@ -347,3 +347,29 @@ def test_contraction_of_the_last_mode(gpu, oracle_lib, dims, k):
         for n in range(len(dims)):
             for dimtree in (False, True):
                 assert rel(c.mttkrp(n, dimtree=dimtree), oracle_lib.mttkrp_direct(X, Fn, n)) < TOL
+
+
+@pytest.mark.parametrize("kern", BPP_KERNELS)
+@pytest.mark.parametrize("n,ncols", [(17, 1300), (32, 700), (50, 1001), (64, 800)])
+def test_bpp_systems_without_a_cholesky_factor(gpu, oracle_lib, n, ncols, kern, monkeypatch):
+    # AtA = blockdiag(PD, [[0, 1], [1, 0]]) with its unknowns mixed: where both
+    # unknowns of the second block are passive (every third right-hand side has
+    # positive entries there) the general solver takes the system, and they
+    # are each other's right-hand side; elsewhere they stay 0.
+    if kern:
+        monkeypatch.setenv("PLANC_GPU_BPP_KERNEL", kern)
+    G0, B0 = _nnls_system(n - 2, ncols, 60 + n)
+    X0, _, _ = oracle_lib.bpp_update(B0.T.copy(), G0)
+    rng = np.random.default_rng(61 + n)
+    at = rng.permutation(n)
+    G, B, X = np.zeros((n, n)), np.empty((n, ncols)), np.zeros((n, ncols))
+    G[np.ix_(at[2:], at[2:])] = G0
+    G[at[0], at[1]] = G[at[1], at[0]] = 1.0
+    B[at[2:]], X[at[2:]] = B0, X0.T
+    B[at[:2]] = -1.0
+    B[at[:2], ::3] = 0.5 + rng.random((2, (ncols + 2) // 3))
+    X[at[0], ::3], X[at[1], ::3] = B[at[1], ::3], B[at[0], ::3]
+    with gpu.Context(0, "fp64") as c:
+        Xg, Pg, its = c.bpp_solve(G, B)
+    assert np.abs(Xg - X).max() <= 1e-9 * np.abs(X).max()  # the bar of the other BPP tests
+    assert np.all(Pg[at[:2], ::3] == 1)

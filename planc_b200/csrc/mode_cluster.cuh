@@ -26,10 +26,13 @@
 // loads of G by 16 SMs would cost more than the launch they save (at 1024 rows,
 // rank 32: 4.4 us for k_hals_warp over the whole GPU), so the update stays a
 // launch of its own there.
-// Measured a mode: 64^3 rank 8, HALS and error included, 6.8 us (2.2 + 8.8 as
-// two launches, and 4.7 a sweep for the error's own); without the update, at
-// 333 rows of rank 20, 8.8 us with the error (9.5, and 6.4 for the error), at
-// 1024 rows of rank 32 10.9 us (12.0 and 9.4).
+// Loads are what a CTA waits for first: the rows, G and M are copied to shared
+// memory asynchronously, all in flight together, and the other modes' Grams are
+// prefetched meanwhile. Measured a mode, against staging them one after another
+// and dividing by k for every element: 64^3 rank 8, HALS and every third error
+// included, 6.0 us (6.7; 2.2 + 8.8 as two launches, and 4.7 a sweep for the
+// error's own); without the update, 512 rows of rank 32 8.8 (10.1; 11.0 and
+// 9.4), 192 rows of rank 64 13.8 (14.7).
 #pragma once
 #include "common.cuh"
 #include "updates_iter.cuh"
@@ -88,6 +91,21 @@ inline size_t mode_smem(int k, int64_t rows) {
   return k <= 16 ? mode_smem_bytes<16>(rows) : k <= 32 ? mode_smem_bytes<32>(rows) : mode_smem_bytes<64>(rows);
 }
 
+// 8 bytes to shared memory, asynchronously; zeros (and no access) where !in
+__device__ __forceinline__ void mode_copy8(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(in ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void mode_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void mode_prefetch(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+// sum of the eight warps' values
+__device__ __forceinline__ double mode_warp_sums(const double* r) {
+  static_assert(MODE_THREADS == 256, "eight warps");
+  return ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
+}
+
 template <int KP, int UPD>
 __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
   using S = ModeShape<KP>;
@@ -112,29 +130,51 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool err = a.errs != nullptr;
 
-  // ---- stage G and the rows (columns past k as zeros)
+  // e / k for e < 2^16 by one multiplication (the quotient of the rounding
+  // error, e / 2^32, stays below 1 / k)
+  const uint32_t inv_k = k > 1 ? 0xffffffffu / (uint32_t)k + 1 : 0;
+  auto div_k = [&](int e) { return k > 1 ? (int)__umulhi((uint32_t)e, inv_k) : e; };
+  // this CTA's slice of the Grams
+  const int sl = (kk2 + CLm - 1) / CLm;
+  const int s0 = me * sl, s1 = me < CLm ? ((s0 + sl) < kk2 ? (s0 + sl) : kk2) : 0;
+
+  // ---- stage the rows, G and M (columns past k as zeros): every copy is in
+  // flight before the first wait
+  auto stage = [&](double* dst, const double* src, int rows) {
+    for (int e = tid; e < rows * KP; e += MODE_THREADS) {
+      const int i = e / KP, c = e % KP;
+      mode_copy8(dst + i * LDH + c, src + (c < k ? i * k + c : 0), c < k);
+    }
+  };
+  if (nrows > 0) stage(tile, a.F + r0 * k, nrows);
   if constexpr (UPD != MODE_NONE) {
     for (int e = tid; e < KP * KP; e += MODE_THREADS) {
       const int i = e / KP, j = e % KP;
-      gs[e] = (i < k && j < k) ? a.Gloo[i * k + j] : 0.0;
+      const bool in = i < k && j < k;
+      mode_copy8(gs + e, a.Gloo + (in ? i * k + j : 0), in);
     }
+    if (nrows > 0) stage(mt, a.M + r0 * k, nrows < CHUNK ? nrows : CHUNK);
   }
-  {
-    const double* F0 = a.F + r0 * k;
-    for (int e = tid; e < nrows * KP; e += MODE_THREADS) {
-      const int i = e / KP, c = e % KP;
-      tile[i * LDH + c] = c < k ? F0[i * k + c] : 0.0;
-    }
+  // the other modes' Grams and the error's inputs, read at the end (a sector
+  // holds four doubles)
+  const bool err0 = err && me == 0;
+  for (int m = 0; m < a.N && (err0 || a.next >= 0); ++m)
+    if (m != a.n)
+      for (int e = (err0 ? 0 : s0) + 4 * tid; e < (err0 ? kk2 : s1); e += 4 * MODE_THREADS)
+        mode_prefetch(a.Gall + (int64_t)m * kk2 + e);
+  if (err0 && tid == 0) {
+    mode_prefetch(a.normX2);
+    mode_prefetch(a.counter);
   }
+  if (UPD == MODE_NONE && err)
+    for (int e = 4 * tid; e < nrows * k; e += 4 * MODE_THREADS) mode_prefetch(a.M + r0 * k + e);
   if constexpr (UPD != MODE_NONE) {
     for (int ch = 0; ch < nrows; ch += CHUNK) {
-      const int nr = (nrows - ch) < CHUNK ? (nrows - ch) : CHUNK;
-      if (ch > 0) __syncthreads();  // the previous chunk's M is read
-      const double* M0 = a.M + (r0 + ch) * k;
-      for (int e = tid; e < nr * KP; e += MODE_THREADS) {
-        const int i = e / KP, c = e % KP;
-        mt[i * LDH + c] = c < k ? M0[i * k + c] : 0.0;
+      if (ch > 0) {
+        __syncthreads();  // the previous chunk's M is read
+        stage(mt, a.M + (r0 + ch) * k, (nrows - ch) < CHUNK ? (nrows - ch) : CHUNK);
       }
+      mode_copy_wait();
       __syncthreads();  // M, and for the first chunk G and the rows
       const int q = lane % LPR;
       const int row = ch + warp * S::RPW + lane / LPR;  // this lane's row
@@ -215,23 +255,26 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
       }
     }
   }
+  mode_copy_wait();
   __syncthreads();  // the (updated) rows
-  if (err) {  // <M, U> over this CTA's rows
+  if (err) {  // <M, U> over this CTA's rows, a warp's part each
     double inner = 0.0;
     const double* M0 = a.M + r0 * k;
-    for (int e = tid; e < nrows * k; e += MODE_THREADS) {
-      const int i = e / k, c = e - i * k;
-      inner = fma(M0[e], tile[i * LDH + c], inner);
+    if (UPD != MODE_NONE && nrows <= CHUNK) {  // M is still in shared memory
+      for (int e = tid; e < nrows * k; e += MODE_THREADS) {
+        const int i = div_k(e), c = e - i * k;
+        inner = fma(mt[i * LDH + c], tile[i * LDH + c], inner);
+      }
+    } else {
+#pragma unroll 4
+      for (int e = tid; e < nrows * k; e += MODE_THREADS) {
+        const int i = div_k(e), c = e - i * k;
+        inner = fma(M0[e], tile[i * LDH + c], inner);
+      }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) inner += __shfl_xor_sync(0xffffffffu, inner, o);
     if (lane == 0) red[warp] = inner;
-    __syncthreads();
-    if (tid == 0) {
-      double s = 0.0;
-      for (int w = 0; w < MODE_THREADS / 32; ++w) s += red[w];
-      inner_sum = s;
-    }
   }
 
   // ---- U^T U of this CTA's rows: a BE x BE block of the upper triangle a
@@ -278,6 +321,7 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
         }
     }
     __syncthreads();
+    if (err && tid == 0) inner_sum = mode_warp_sums(red);
   }
 
   // ---- the factor's U^T U in every CTA: partials summed in rank order
@@ -318,28 +362,31 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
     }
   }
   double inner_all = 0.0;
-  if (err && me == 0 && tid == 0)
-    for (int b = 0; b < CLm; ++b) inner_all += *cluster.map_shared_rank(&inner_sum, b);
+  const bool many = cluster.num_blocks() > 1;
+  if (err0 && warp == 0) {
+    static_assert(MODE_MAX_CL == 16, "one CTA per lane of a half warp");
+    if (lane < CLm) inner_all = *cluster.map_shared_rank(&inner_sum, lane);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) inner_all += __shfl_xor_sync(0xffffffffu, inner_all, o);
+  }
   // no CTA reads another's shared memory from here on; a CTA may leave once
   // all have come this far
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (many) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   if (me < CLm) {
     if (tid < k) lam[tid] = sqrt(gram[tid * KP + tid]);
     __syncthreads();
     // normalised rows
     double* F0 = a.F + r0 * k;
     for (int e = tid; e < nrows * k; e += MODE_THREADS) {
-      const int i = e / k, c = e - i * k;
+      const int i = div_k(e), c = e - i * k;
       const double nrm = lam[c], u = tile[i * LDH + c];
       F0[e] = nrm > 0 ? u / nrm : u;
     }
     if (me == 0 && tid < k && a.lambda) a.lambda[tid] = lam[tid];
     // G_n and the leave-one-out product of mode `next`: a slice per CTA
-    const int sl = (kk2 + CLm - 1) / CLm;
-    const int e0 = me * sl, e1 = (e0 + sl) < kk2 ? (e0 + sl) : kk2;
     double* Gn = a.Gall + (int64_t)a.n * kk2;
-    for (int e = e0 + tid; e < e1; e += MODE_THREADS) {
-      const int i = e / k, j = e - i * k;
+    for (int e = s0 + tid; e < s1; e += MODE_THREADS) {
+      const int i = div_k(e), j = e - i * k;
       const double la = lam[i], lb = lam[j], s = gram[i * KP + j];
       const double gn = (la > 0 && lb > 0) ? s / (la * lb) : s;
       Gn[e] = gn;
@@ -350,12 +397,12 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
         a.Gloo[e] = g;
       }
     }
-    if (err && me == 0) {
+    if (err0) {
       // ||X||^2 - 2 <M, U> + sum_ab lambda_a lambda_b prod_m G_m[a, b], with
       // lambda_a lambda_b G_n[a, b] = (U^T U)_ab
       double mn = 0.0;
       for (int e = tid; e < kk2; e += MODE_THREADS) {
-        const int i = e / k, j = e - i * k;
+        const int i = div_k(e), j = e - i * k;
         const double la = lam[i], lb = lam[j];
         double g = (la > 0 && lb > 0) ? gram[i * KP + j] : 0.0;
         for (int m = 0; m < a.N; ++m)
@@ -367,8 +414,7 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
       if (lane == 0) red[warp] = mn;
       __syncthreads();
       if (tid == 0) {
-        double t = 0.0;
-        for (int w = 0; w < MODE_THREADS / 32; ++w) t += red[w];
+        const double t = mode_warp_sums(red);
         const double nx = *a.normX2;
         const double e2 = nx - 2.0 * inner_all + t;
         const int c = *a.counter;
@@ -377,7 +423,7 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
       }
     }
   }
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (many) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 template <int KP, int UPD>

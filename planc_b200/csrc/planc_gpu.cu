@@ -253,18 +253,22 @@ int eff_sm(const planc_gpu_ctx* c) {
   return v < 1 ? 1 : v;
 }
 
+// Whether a CTA (else a warp) takes each of ncols right-hand sides.
+bool bpp_by_cta(const planc_gpu_ctx* c, int kp, int64_t ncols) {
+  if (c->bpp_kernel == 1) return false;
+  if (c->bpp_kernel == 2) return kp >= 32;
+  return kp >= 32 && ncols <= 4 * (int64_t)c->sm_count;
+}
+
 // Batched BPP of ncols right-hand sides with the k x k matrix AtA (k_bpp: a
 // warp per right-hand side; k_bpp_cta: a CTA per right-hand side, for k > 16
 // while the right-hand sides are too few to give every SM several warps).
 // Launched on the context's stream; the caller times it.
 void launch_bpp(planc_gpu_ctx* c, const double* AtA, const double* B, int n, int64_t ncols,
-                double* X, int* P, int* I, const double* warm) {
+                double* X, int* P, int* I, const double* warm, bool packed = true) {
   if (ncols <= 0) return;
   const int kp = kpad(n);
-  bool cta = kp >= 32 && ncols <= 4 * (int64_t)c->sm_count;
-  if (c->bpp_kernel == 1) cta = false;
-  if (c->bpp_kernel == 2) cta = kp >= 32;
-  if (cta) {
+  if (bpp_by_cta(c, kp, ncols)) {
     const unsigned grid = (unsigned)std::min<int64_t>(ncols, 2 * (int64_t)c->sm_count);
     if (kp == 32) {
       using C = BppCta<32, 8>;
@@ -279,7 +283,7 @@ void launch_bpp(planc_gpu_ctx* c, const double* AtA, const double* B, int n, int
   }
   const unsigned blocks = (unsigned)((ncols + BPP_WARPS - 1) / BPP_WARPS);
   int* lu = nullptr;
-  if (kp == 64 && c->bpp_lu_cap >= ncols) {
+  if (packed && kp == 64 && c->bpp_lu_cap >= ncols) {
     // packed factors first, then the right-hand sides whose passive system
     // was not positive definite
     lu = c->bpp_lu;
@@ -311,9 +315,10 @@ void dalloc(T** p, size_t n) {
   CK(cudaMalloc((void**)p, n * sizeof(T)));
 }
 
-// Flags of the batched BPP for ncols right-hand sides (outside graph capture).
-void ensure_bpp_lu(planc_gpu_ctx* c, int64_t ncols) {
-  if (c->bpp_lu_cap >= ncols) return;
+// Flags of the batched BPP for ncols right-hand sides of n unknowns, where its
+// packed form takes them (outside graph capture).
+void ensure_bpp_lu(planc_gpu_ctx* c, int n, int64_t ncols) {
+  if (c->bpp_lu_cap >= ncols || kpad(n) != 64 || bpp_by_cta(c, 64, ncols)) return;
   c->bpp_lu_cap = 0;
   dalloc(&c->bpp_lu, (size_t)ncols);
   c->bpp_lu_cap = ncols;
@@ -1576,7 +1581,7 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
   const int k = c->k;
   int64_t maxI = 1;
   for (int n = 0; n < c->N; ++n) maxI = std::max(maxI, c->dims[n]);
-  if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(c, maxI);
+  if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(c, c->k, maxI);
   if (algo == PLANC_GPU_AOADMM && !c->admm_ready) {
     for (int n = 0; n < c->N; ++n) {
       dalloc(&c->aux[n], (size_t)c->dims[n] * k);
@@ -2276,7 +2281,7 @@ int planc_gpu_bpp_solve(planc_gpu_ctx* c, const double* AtA, const double* AtB, 
     if (ncols < 0) fail(PLANC_GPU_ERR_ARG, "ncols < 0");
     if (ncols == 0) return;
     set_device(c);
-    ensure_bpp_lu(c, ncols);
+    ensure_bpp_lu(c, n, ncols);
     // one workspace for operands and results, kept by the context: five
     // allocations and frees a call cost several times the solve
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -2334,13 +2339,14 @@ int planc_gpu_update_device(planc_gpu_ctx* c, int algo, double* H, const double*
       });
       return;
     }
-    // the flags' buffer grows here, except while the stream is captured (the
-    // solves then run in their plain form)
+    // a caller's graph must not hold the flags' buffer, which a later call may
+    // replace: under capture the solves take their plain form
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(c->stream, &cap));
-    if (cap == cudaStreamCaptureStatusNone) ensure_bpp_lu(c, rows);
+    const bool packed = cap == cudaStreamCaptureStatusNone;
+    if (packed) ensure_bpp_lu(c, k, rows);
     launch(c, KC_BPP, [&] {
-      launch_bpp(c, G, M, k, rows, H, nullptr, nullptr, c->bpp_warm ? H : nullptr);
+      launch_bpp(c, G, M, k, rows, H, nullptr, nullptr, c->bpp_warm ? H : nullptr, packed);
     });
   });
 }
@@ -2753,7 +2759,7 @@ void batch_ensure(planc_gpu_batch* b, int algo, int iters, bool err) {
   for (auto* m : b->members) {
     ensure_buffers(m);
     ensure_errs(m, err ? iters : 1);
-    if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(m, *std::max_element(m->dims, m->dims + m->N));
+    if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(m, m->k, *std::max_element(m->dims, m->dims + m->N));
   }
   if (b->g_epoch != batch_epoch(b)) batch_reset_graph(b);
 }
@@ -3920,7 +3926,7 @@ int planc_gpu_nmf_run(planc_gpu_ctx* c, int algo, int iters, double* objective,
     if (iters == 0) return;
     set_device(c);
     ensure_nmf(c, iters);
-    if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(c, std::max(c->dims[0], c->dims[1]));
+    if (algo == PLANC_GPU_ANLSBPP) ensure_bpp_lu(c, c->k, std::max(c->dims[0], c->dims[1]));
     if (c->nmf_gepoch != c->buf_epoch && c->nmf_gexec) {
       cudaGraphExecDestroy(c->nmf_gexec);
       c->nmf_gexec = nullptr;

@@ -373,3 +373,33 @@ def test_bpp_systems_without_a_cholesky_factor(gpu, oracle_lib, n, ncols, kern, 
         Xg, Pg, its = c.bpp_solve(G, B)
     assert np.abs(Xg - X).max() <= 1e-9 * np.abs(X).max()  # the bar of the other BPP tests
     assert np.all(Pg[at[:2], ::3] == 1)
+
+
+def test_bpp_update_captured_before_a_larger_one(gpu, oracle_lib):
+    # a caller's graph of a row-block update, replayed after a larger update has
+    # replaced the context's own buffers
+    import torch
+    k, small, large = 40, 700, 3000
+    G, B = _nnls_system(k, large, 31)
+    ref, _, _ = oracle_lib.bpp_update(B.T.copy(), G)
+    side = torch.cuda.Stream()
+    Gd = torch.tensor(G, device="cuda")
+    M = torch.tensor(np.ascontiguousarray(B.T), device="cuda")
+    H = torch.zeros((large, k), device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    with gpu.Context(0, "fp64", stream=side.cuda_stream) as c:
+        def update(rows):
+            c.update_device("anlsbpp", H.data_ptr(), M.data_ptr(), Gd.data_ptr(), rows, k)
+        update(small)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            update(small)
+        update(large)
+        side.synchronize()
+        assert np.abs(H.cpu().numpy() - ref).max() <= 1e-9 * np.abs(ref).max()
+        H.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+    assert np.abs(H[:small].cpu().numpy() - ref[:small]).max() <= 1e-9 * np.abs(ref).max()
+    assert not H[small:].any()

@@ -46,8 +46,18 @@ namespace pg {
 // (row t, col g), C elements (row g, cols 2t, 2t+1), g = lane / 4, t = lane % 4.
 // ---------------------------------------------------------------------------
 constexpr int CT_BM = 128;
-template <int KP>
-constexpr int ct_bk() { return KP == 64 ? 16 : 32; }
+// Reduction steps of a tile of BM rows. Left contractions of few rows (a small
+// last mode, down to a couple of dozen rows against a reduction of 10^5) take
+// tiles of 32 or 64 rows and four or two times as many steps, and the warps that
+// the rows leave idle split the steps among them (summed once, at the end):
+// with 128-row tiles a thread has few loads in flight a tile and a CTA many
+// tiles to go through. 61 x 47 x 33 x 29, rank 11, last mode: 19.8 -> 13.5 us.
+template <int KP, int BM = CT_BM>
+constexpr int ct_bk() {
+  return BM == 128 ? (KP == 64 ? 16 : 32) : BM == 64 ? (KP == 64 ? 32 : 64) : KP <= 16 ? 128 : KP == 32 ? 64 : 32;
+}
+// Rows of the tile for a left contraction with M rows.
+constexpr int ct_rows(int64_t M) { return M <= 32 ? 32 : M <= 64 ? 64 : CT_BM; }
 // Row strides (in doubles) of the shared-memory tiles. A fragment load of
 // lane (g, t) = (lane / 4, lane % 4) reads word t * S + g (+ a constant);
 // a half warp (g < 4 or g >= 4) is one 128-byte wavefront when t * S mod 16
@@ -56,12 +66,13 @@ template <int KP>
 constexpr int ct_ws() { return KP + 4; }
 constexpr int CT_SXR = CT_BM + 4;  // RIGHT: Xs[kk][m]
 // doubles of one shared-memory stage (X tile + W tile)
-template <int KP, bool LEFT>
+template <int KP, bool LEFT, int BM = CT_BM>
 constexpr int ct_stage_elems() {
-  return (LEFT ? CT_BM * (ct_bk<KP>() + 4) : ct_bk<KP>() * CT_SXR) + ct_bk<KP>() * ct_ws<KP>();
+  constexpr int BK = ct_bk<KP, BM>();
+  return (LEFT ? BM * (BK + 4) : BK * CT_SXR) + BK * ct_ws<KP>();
 }
-template <int KP, bool LEFT>
-constexpr size_t ct_smem_bytes() { return 2 * sizeof(double) * (size_t)ct_stage_elems<KP, LEFT>(); }
+template <int KP, bool LEFT, int BM = CT_BM>
+constexpr size_t ct_smem_bytes() { return 2 * sizeof(double) * (size_t)ct_stage_elems<KP, LEFT, BM>(); }
 
 struct ContractGeom {
   int64_t M;        // output rows
@@ -142,30 +153,33 @@ __device__ __forceinline__ double wgen_at32(const WGen& wg, const FastDiv& f0, c
 // F_1[i1, r] * F_2[i2, r] with b = i1 + dim[1] i2 (NF = 3): a thread takes
 // tail once per tile, then one F_0 load and one multiply per entry (the same
 // products as wgen_at, so the same W).
-template <int KP, bool LEFT, int NF, bool RUNS = false, bool RING = false>
+template <int KP, bool LEFT, int NF, bool RUNS = false, bool RING = false, int BM = CT_BM>
 __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restrict__ X,
                                                          ContractGeom g, WGen wg, int k,
                                                          double* __restrict__ out) {
   static_assert(!RUNS || (LEFT && (NF == 2 || NF == 3)), "runs of the fastest mode");
   static_assert(!RING || !LEFT, "asynchronous copies of the right contraction's tiles");
-  constexpr int BK = ct_bk<KP>();
-  constexpr int XPT = BK * CT_BM / 256;  // X elements per thread per tile
+  static_assert(BM == CT_BM || (LEFT && !RUNS), "tiles of few rows");
+  constexpr int BK = ct_bk<KP, BM>();
+  constexpr int XPT = BK * BM / 256;  // X elements per thread per tile
   constexpr int WPT = (BK * KP + 255) / 256;
-  constexpr int WARPS_M = KP >= 32 ? 4 : 8;
-  constexpr int WARPS_N = 8 / WARPS_M;
-  constexpr int MT = CT_BM / WARPS_M / 8;  // 8-row MMA tiles per warp
+  constexpr int WARPS_M = BM < CT_BM ? BM / 16 : KP >= 32 ? 4 : 8;
+  constexpr int WARPS_K = CT_BM / BM;
+  constexpr int WARPS_N = 8 / (WARPS_M * WARPS_K);
+  constexpr int MT = BM / WARPS_M / 8;     // 8-row MMA tiles per warp
   constexpr int NT = KP / WARPS_N / 8;     // 8-rank MMA tiles per warp
   constexpr int SX = LEFT ? BK + 4 : CT_SXR;
   constexpr int SW = ct_ws<KP>();
-  constexpr int XS_ELEMS = LEFT ? CT_BM * SX : BK * SX;
-  constexpr int STAGE = ct_stage_elems<KP, LEFT>();
+  constexpr int XS_ELEMS = LEFT ? BM * SX : BK * SX;
+  constexpr int STAGE = ct_stage_elems<KP, LEFT, BM>();
   extern __shared__ __align__(16) double ct_smem[];
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const int fg = lane >> 2, ft = lane & 3;
   const int wm0 = (warp % WARPS_M) * (MT * 8);
-  const int wn0 = (warp / WARPS_M) * (NT * 8);
-  const int64_t m0 = (int64_t)blockIdx.x * CT_BM;
+  const int wn0 = (warp / WARPS_M % WARPS_N) * (NT * 8);
+  const int wk = warp / (WARPS_M * WARPS_N);  // this warp's part of a tile's steps
+  const int64_t m0 = (int64_t)blockIdx.x * BM;
   const int64_t t_begin = (int64_t)blockIdx.y * g.tiles_per_split;
   int64_t t_end = t_begin + g.tiles_per_split;
   if (t_end > g.ktiles) t_end = g.ktiles;
@@ -266,7 +280,7 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restric
       const int64_t gm0 = m0 + tid / BK;
       const double* xp = X + ga + g.ldx * gm0 + g.ldb * b;
       const int64_t xstep = MSTEP * g.ldx;
-      if (ga < g.A && m0 + CT_BM <= g.M) {
+      if (ga < g.A && m0 + BM <= g.M) {
 #pragma unroll
         for (int i = 0; i < XPT; ++i) {
           xr[i] = *xp;
@@ -394,8 +408,8 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restric
       const double* Xs = ct_smem + stage * STAGE;
       const double* Ws = Xs + XS_ELEMS;
 #pragma unroll
-      for (int s4 = 0; s4 < BK / 4; ++s4) {
-        const int kk = s4 * 4 + ft;
+      for (int s4 = 0; s4 < BK / 4 / WARPS_K; ++s4) {
+        const int kk = (wk * (BK / 4 / WARPS_K) + s4) * 4 + ft;
         double af[MT], bf[NT];
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
@@ -411,6 +425,24 @@ __global__ void __launch_bounds__(256, 2) k_contract_f64(const double* __restric
       }
     }
     if (t + 1 < t_end) store_tile(stage ^ 1);
+  }
+  if constexpr (WARPS_K > 1) {  // the parts of the steps, in order
+    constexpr int NW = WARPS_M * WARPS_N;
+    static_assert((WARPS_K - 1) * NW * MT * NT * 64 <= 2 * STAGE, "partial sums fit the stages");
+    double* red = ct_smem + (size_t)(warp % NW) * (MT * NT * 64) + lane;
+    __syncthreads();
+    if (wk > 0) {
+      double* r = red + (size_t)(wk - 1) * NW * (MT * NT * 64);
+#pragma unroll
+      for (int e = 0; e < MT * NT * 2; ++e) r[32 * e] = acc[e / (2 * NT)][e / 2 % NT][e % 2];
+    }
+    __syncthreads();
+    if (wk > 0) return;
+#pragma unroll
+    for (int w = 1; w < WARPS_K; ++w)
+#pragma unroll
+      for (int e = 0; e < MT * NT * 2; ++e)
+        acc[e / (2 * NT)][e / 2 % NT][e % 2] += red[(size_t)(w - 1) * NW * (MT * NT * 64) + 32 * e];
   }
   double* o = out + (int64_t)blockIdx.y * g.split_stride;
 #pragma unroll

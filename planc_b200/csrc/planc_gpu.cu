@@ -518,11 +518,24 @@ WGen make_wgen(planc_gpu_ctx* c, const std::vector<int>& modes) {
 struct ContractPlan {
   ContractGeom g;
   int nsplit;
+  int bm;  // rows of a tile
   dim3 grid;
 };
 
+// Reduction steps of a tile of bm rows at rank k.
+int contract_bk(int k, int bm) {
+  switch (kpad(k)) {
+    case 32: return bm == 32 ? ct_bk<32, 32>() : bm == 64 ? ct_bk<32, 64>() : ct_bk<32>();
+    case 64: return bm == 32 ? ct_bk<64, 32>() : bm == 64 ? ct_bk<64, 64>() : ct_bk<64>();
+    default: return bm == 32 ? ct_bk<16, 32>() : bm == 64 ? ct_bk<16, 64>() : ct_bk<16>();
+  }
+}
+
+// nf: factors of the Khatri-Rao operand; runs: the reduction index as runs of
+// mode 0 (k_contract_f64). Left contractions of up to 64 rows against two or
+// three factors take tiles of 32 or 64 rows.
 ContractPlan plan_contract(planc_gpu_ctx* c, bool left, int64_t M, int64_t ldx, int64_t A,
-                           int64_t B, int64_t ldb) {
+                           int64_t B, int64_t ldb, int nf, bool runs) {
   ContractPlan p;
   memset(&p, 0, sizeof(p));
   p.g.M = M;
@@ -530,10 +543,11 @@ ContractPlan plan_contract(planc_gpu_ctx* c, bool left, int64_t M, int64_t ldx, 
   p.g.A = A;
   p.g.B = B;
   p.g.ldb = ldb;
-  const int bk = c->k > 32 ? ct_bk<64>() : ct_bk<32>();
+  p.bm = left && !runs && (nf == 2 || nf == 3) ? ct_rows(M) : CT_BM;
+  const int bk = contract_bk(c->k, p.bm);
   int64_t tilesA = (A + bk - 1) / bk;
   p.g.ktiles = left ? tilesA * B : tilesA;
-  int64_t mtiles = (M + CT_BM - 1) / CT_BM;
+  int64_t mtiles = (M + p.bm - 1) / p.bm;
   int64_t target = 2 * (int64_t)eff_sm(c);
   int64_t ns = (target + mtiles - 1) / mtiles;
   ns = std::max<int64_t>(1, std::min<int64_t>(ns, p.g.ktiles));
@@ -584,6 +598,28 @@ void direct_geom(planc_gpu_ctx* c, int n, int64_t* A, int64_t* B) {
 
 void ensure_buffers_impl(planc_gpu_ctx* c);
 
+// The FP64 tree's left contraction. Above 64 rows, reduction tiles aligned to
+// runs of I_0 where its tiles fit them (the same tiles and splits as the flat
+// view): one Khatri-Rao tail per tile.
+bool left_runs(planc_gpu_ctx* c) {
+  const int nf = c->s + 1;
+  return (nf == 2 || nf == 3) && ct_rows(c->R) == CT_BM && c->dims[0] % contract_bk(c->k, CT_BM) == 0;
+}
+ContractPlan plan_left(planc_gpu_ctx* c) {
+  const int nf = c->s + 1;
+  return left_runs(c) ? plan_contract(c, true, c->R, c->L, c->dims[0], c->L / c->dims[0], c->dims[0], nf, true)
+                      : plan_contract(c, true, c->R, c->L, c->L, 1, 0, nf, false);
+}
+
+// The direct MTTKRP of mode n (A, B: direct_geom). Mode 1's reduction index is
+// already runs of I_0 (A = I_0), so each tile takes one Khatri-Rao tail of the
+// slower modes.
+bool direct_runs(planc_gpu_ctx* c, int n) { return n == 1 && (c->N == 3 || c->N == 4); }
+ContractPlan plan_direct(planc_gpu_ctx* c, int n, int64_t A, int64_t B) {
+  return n == 0 ? plan_contract(c, false, c->dims[0], c->dims[0], B, 1, 0, c->N - 1, false)
+                : plan_contract(c, true, c->dims[n], A, A, B, A * c->dims[n], c->N - 1, direct_runs(c, n));
+}
+
 // Computes the largest scratch any MTTKRP path needs and (re)allocates; any
 // reallocation invalidates the cached graph (it holds the old pointers).
 void ensure_buffers(planc_gpu_ctx* c) {
@@ -626,9 +662,9 @@ void ensure_buffers_impl(planc_gpu_ctx* c) {
   const int k = c->k;
   size_t need = 0;
   if (c->N == 3 || c->N == 4) {
-    ContractPlan pl = plan_contract(c, true, c->R, c->L, c->L, 1, 0);
+    ContractPlan pl = plan_left(c);
     need = std::max(need, contract_scratch(pl));
-    ContractPlan pr = plan_contract(c, false, c->L, c->L, c->R, 1, 0);
+    ContractPlan pr = plan_contract(c, false, c->L, c->L, c->R, 1, 0, c->N - 1 - c->s, false);
     need = std::max(need, contract_scratch(pr));
     TtvRightPlan tr = plan_ttv_right(c, c->dims[0], c->L / c->dims[0]);
     need = std::max(need, (size_t)tr.nsplit * c->dims[0] * k);
@@ -655,8 +691,7 @@ void ensure_buffers_impl(planc_gpu_ctx* c) {
   for (int n = 0; n < c->N; ++n) {
     int64_t A, B;
     direct_geom(c, n, &A, &B);
-    ContractPlan pl = n == 0 ? plan_contract(c, false, c->dims[0], c->dims[0], B, 1, 0)
-                             : plan_contract(c, true, c->dims[n], A, A, B, A * c->dims[n]);
+    ContractPlan pl = plan_direct(c, n, A, B);
     need = std::max(need, contract_scratch(pl));
   }
   need = std::max<size_t>(need, 4096);
@@ -681,9 +716,20 @@ void ensure_buffers_impl(planc_gpu_ctx* c) {
 // other count takes the generic generator)
 template <int KP, bool LEFT>
 void launch_contract_f64(dim3 grid, cudaStream_t st, const double* X, const ContractGeom& g,
-                         const WGen& wg, int k, double* dst, bool runs = false) {
+                         const WGen& wg, int k, double* dst, bool runs = false, int bm = CT_BM) {
   constexpr size_t sm = ct_smem_bytes<KP, LEFT>();
   if constexpr (LEFT) {
+    if (bm < CT_BM) {
+#define SHORT(NF, BM)                                                                                        \
+  k_contract_f64<KP, true, NF, false, false, BM><<<grid, 256, ct_smem_bytes<KP, true, BM>(), st>>>(X, g, wg, \
+                                                                                                   k, dst)
+      if (wg.nf == 2 && bm == 32) SHORT(2, 32);
+      else if (wg.nf == 2) SHORT(2, 64);
+      else if (bm == 32) SHORT(3, 32);
+      else SHORT(3, 64);
+#undef SHORT
+      return;
+    }
     if (runs && wg.nf == 2) {
       k_contract_f64<KP, true, 2, true><<<grid, 256, sm, st>>>(X, g, wg, k, dst);
       return;
@@ -717,6 +763,12 @@ void contract_f64_attrs_kp() {
   if constexpr (!LEFT && KP >= 32)
     CK(cudaFuncSetAttribute(k_contract_f64<KP, false, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   if constexpr (LEFT) {
+    for (auto kern : {k_contract_f64<KP, true, 2, false, false, 32>, k_contract_f64<KP, true, 3, false, false, 32>})
+      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)ct_smem_bytes<KP, true, 32>()));
+    for (auto kern : {k_contract_f64<KP, true, 2, false, false, 64>, k_contract_f64<KP, true, 3, false, false, 64>})
+      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)ct_smem_bytes<KP, true, 64>()));
     CK(cudaFuncSetAttribute(k_contract_f64<KP, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     CK(cudaFuncSetAttribute(k_contract_f64<KP, true, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   }
@@ -751,7 +803,7 @@ void run_contract(planc_gpu_ctx* c, const ContractPlan& p, bool left, const doub
 #define CASE(KP)                                                                      \
   case KP:                                                                            \
     if (left)                                                                         \
-      launch_contract_f64<KP, true>(p.grid, c->stream, X, p.g, wg, k, dst, runs);     \
+      launch_contract_f64<KP, true>(p.grid, c->stream, X, p.g, wg, k, dst, runs, p.bm); \
     else                                                                              \
       launch_contract_f64<KP, false>(p.grid, c->stream, X, p.g, wg, k, dst);          \
     break;
@@ -958,13 +1010,9 @@ void mttkrp_direct(planc_gpu_ctx* c, int n, double* out) {
   int64_t A, B;
   direct_geom(c, n, &A, &B);
   if (n == 0) {
-    ContractPlan p = plan_contract(c, false, c->dims[0], c->dims[0], B, 1, 0);
-    run_contract(c, p, false, c->X64, wg, out);
+    run_contract(c, plan_direct(c, n, A, B), false, c->X64, wg, out);
   } else {
-    // mode 1: the reduction index is already runs of I_0 (A = I_0), so each
-    // tile takes one Khatri-Rao tail of the slower modes
-    ContractPlan p = plan_contract(c, true, c->dims[n], A, A, B, A * c->dims[n]);
-    run_contract(c, p, true, c->X64, wg, out, n == 1 && (wg.nf == 2 || wg.nf == 3));
+    run_contract(c, plan_direct(c, n, A, B), true, c->X64, wg, out, direct_runs(c, n));
   }
 }
 
@@ -972,7 +1020,7 @@ void mttkrp_direct(planc_gpu_ctx* c, int n, double* out) {
 void partial_right(planc_gpu_ctx* c) {
   if (c->precision == PLANC_GPU_PREC_FP64) {
     WGen wg = make_wgen(c, {c->N - 1});
-    ContractPlan p = plan_contract(c, false, c->L, c->L, c->R, 1, 0);
+    ContractPlan p = plan_contract(c, false, c->L, c->L, c->R, 1, 0, wg.nf, false);
     run_contract(c, p, false, c->X64, wg, c->P);
   } else {
     launch(c, KC_PREP, [&] { tc_right_prep(c->tct, c->F[c->N - 1], c->k, c->stream); });
@@ -994,13 +1042,8 @@ void partial_left(planc_gpu_ctx* c, double* out) {
   }
   if (c->precision == PLANC_GPU_PREC_FP64) {
     WGen wg = make_wgen(c, modes);
-    // reduction tiles aligned to runs of I_0 (the same tiles and splits as the
-    // flat view when I_0 is a multiple of the tile): one Khatri-Rao tail per tile
-    const int64_t bk = kpad(c->k) == 64 ? ct_bk<64>() : ct_bk<32>();
-    const bool runs = (wg.nf == 2 || wg.nf == 3) && c->dims[0] % bk == 0;
-    ContractPlan p = runs ? plan_contract(c, true, c->R, c->L, c->dims[0], c->L / c->dims[0], c->dims[0])
-                          : plan_contract(c, true, c->R, c->L, c->L, 1, 0);
-    run_contract(c, p, true, c->X64, wg, out, runs);
+    ContractPlan p = plan_left(c);
+    run_contract(c, p, true, c->X64, wg, out, left_runs(c));
   } else {
     WGen wg = make_wgen(c, modes);
     int nsplit = 0;

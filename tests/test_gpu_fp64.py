@@ -403,3 +403,20 @@ def test_bpp_update_captured_before_a_larger_one(gpu, oracle_lib):
         torch.cuda.synchronize()
     assert np.abs(H[:small].cpu().numpy() - ref[:small]).max() <= 1e-9 * np.abs(ref).max()
     assert not H[small:].any()
+
+
+@pytest.mark.parametrize("dims,k", [((40, 30, 1), 3), ((33, 29, 16), 8), ((64, 31, 31), 16), ((65, 64, 32), 11),
+                                    ((47, 33, 33), 9), ((32, 48, 63), 17), ((61, 50, 64), 32), ((64, 40, 65), 12),
+                                    ((23, 31, 30, 29), 11), ((17, 12, 50, 40), 33), ((9, 70, 20, 64), 64),
+                                    ((200, 130, 7), 64)])
+def test_contraction_onto_few_rows(gpu, oracle_lib, dims, k):
+    # left contractions with tiles of 32 and 64 rows (and one row more): a
+    # reduction of less than a tile's steps, of a few and of many tiles, flat and
+    # in batches (direct, mode 2 of 4)
+    X, _ = cp_tensor(dims, 3, seed=11)
+    F = init_factors(dims, k, seed=12)
+    with _ctx(gpu, X, F) as c:
+        Fn = _normalized(F)
+        for n in range(len(dims)):
+            for dimtree in (False, True):
+                assert rel(c.mttkrp(n, dimtree=dimtree), oracle_lib.mttkrp_direct(X, Fn, n)) < TOL

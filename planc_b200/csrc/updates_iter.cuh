@@ -580,23 +580,40 @@ __device__ __forceinline__ double nes_alpha_of(double alpha, double q) {
 // diagonal d and squared off-diagonals e2 (both scaled so that no entry
 // exceeds 1): the sign changes of the leading minors of T - sigma I
 // (p_i+1 = (d_i - sigma) p_i - e_i^2 p_i-1). No division on the chain; a
-// vanishing minor counts as a change, and both minors are rescaled by a power
-// of two whenever they leave [2^-300, 2^300].
+// vanishing minor counts as a change. Signs and zeros are read from the words,
+// off the FP64 pipe, and both minors are rescaled by a power of two every fourth
+// step when they have left [2^-300, 2^300]: a step grows the larger of the two
+// by 2^2 at most and shrinks it by 2^-165 at most (2^-59 of a shift next to an
+// entry, 2^-106 of a cancellation). More shifts a lane (129 sections a round in
+// place of 33) were slower: the chains share one warp's issue.
+__device__ __forceinline__ double nes_nonzero(double p2, double p1) {
+  return ((__double2hiint(p2) & 0x7fffffff) | __double2loint(p2)) == 0 ? p1 * -0x1p-60 : p2;
+}
 __device__ __forceinline__ int nes_count_below(const double* d, const double* e2, int k, double sigma) {
-  double p0 = 1.0, p1 = d[0] - sigma;
-  if (p1 == 0.0) p1 = -0x1p-60;
-  int cnt = p1 < 0.0;
-  for (int i = 1; i < k; ++i) {
-    double p2 = fma(d[i] - sigma, p1, -(e2[i - 1] * p0));
-    if (p2 == 0.0) p2 = p1 * -0x1p-60;
-    cnt += (p2 < 0.0) != (p1 < 0.0);
+  double p0 = 1.0, p1 = nes_nonzero(d[0] - sigma, 1.0);
+  int cnt = (unsigned)__double2hiint(p1) >> 31;
+  auto step = [&](double di, double ei) {
+    const double p2 = nes_nonzero(fma(di - sigma, p1, -(ei * p0)), p1);
+    cnt += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
     p0 = p1;
     p1 = p2;
+  };
+  int i = 1;
+  for (; i + 4 <= k; i += 4) {
+    double di[4], ei[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      di[u] = d[i + u];
+      ei[u] = e2[i + u - 1];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) step(di[u], ei[u]);
     const double m = fmax(fabs(p0), fabs(p1));
     const double f = m > 0x1p300 ? 0x1p-300 : m < 0x1p-300 ? 0x1p300 : 1.0;
     p0 *= f;
     p1 *= f;
   }
+  for (; i < k; ++i) step(d[i], e2[i - 1]);
   return cnt;
 }
 
@@ -607,9 +624,8 @@ __device__ __forceinline__ int nes_count_below(const double* d, const double* e2
 // lane; warp 0 narrows the smallest eigenvalue, warp 1 the largest). Bound by
 // the k - 2 dependent reflections: eight threads per row, two barriers a
 // reflection, the short sums taken by every warp redundantly so that they
-// need no barrier: 27 us at k = 16 with the four warps that its rows fill, 28.6
-// with sixteen (cyclic Jacobi rotations, k/2 disjoint ones a round, took
-// 105 us). One CTA.
+// need no barrier: 22 us at k = 16 with the four warps that its rows fill
+// (cyclic Jacobi rotations, k/2 disjoint ones a round, took 105 us). One CTA.
 // Then lambda, q and 1/(L + lambda) of the update (ntfnes.hpp:114-117). For
 // mode 0 it also copies the proximal lambda to the previous one
 // (ntfnes.hpp:102-104).

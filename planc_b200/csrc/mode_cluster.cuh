@@ -15,24 +15,26 @@
 //
 // Layout: a cluster of up to 16 CTAs splits the rows evenly, 64 (16 above rank
 // 32) or more a CTA. U^T U of a CTA's rows is summed row by row in increasing
-// order, one upper-triangle block of outputs a thread (the transposed outputs
-// have the same products in the same order), and over the cluster in rank
+// order on the FP64 tensor cores, an 8 x 8 block of the upper triangle a warp
+// (the transposed outputs have the same products in the same order), and over the cluster in rank
 // order: the sums, hence the bits, depend on I and k alone, not on the launch
 // (alone, or a member of a grouped launch) nor on how the threads share it.
 // The update gives a row to 4 lanes, each holding 4 columns in pairs, so that a
 // warp carries 8 rows through the recurrence at once; G is read as 16-byte
-// loads and only the step's change travels by shuffle. Its sums run in the
+// loads and only the step's change travels by shuffle; H G starts as tensor-core
+// products in the lanes' own layout. Its sums run in the
 // order of the one-row-per-warp kernels (the same bits). Above rank 16 the
 // loads of G by 16 SMs would cost more than the launch they save (at 1024 rows,
 // rank 32: 4.4 us for k_hals_warp over the whole GPU), so the update stays a
 // launch of its own there.
 // Loads are what a CTA waits for first: the rows, G and M are copied to shared
 // memory asynchronously, all in flight together, and the other modes' Grams are
-// prefetched meanwhile. Measured a mode, against staging them one after another
-// and dividing by k for every element: 64^3 rank 8, HALS and every third error
-// included, 6.0 us (6.7; 2.2 + 8.8 as two launches, and 4.7 a sweep for the
-// error's own); without the update, 512 rows of rank 32 8.8 (10.1; 11.0 and
-// 9.4), 192 rows of rank 64 13.8 (14.7).
+// prefetched meanwhile. Measured a mode: 64^3 rank 8, HALS and every third error
+// included, 5.4 us (6.7 with the copies one after another, a division by k for
+// every element and the sums by fused multiply-adds, 6.0 without those sums on
+// the tensor cores; 2.2 + 8.8 as two launches, and 4.7 a sweep for the error's
+// own); without the update, 512 rows of rank 32 8.0 (10.1, 8.8; 11.0 and 9.4),
+// 192 rows of rank 64 12.8 (14.7, 13.8).
 #pragma once
 #include "common.cuh"
 #include "updates_iter.cuh"
@@ -68,8 +70,10 @@ struct ModeShape {
   static constexpr int RPW = 32 / LPR;              // rows of a warp
   static constexpr int CHUNK = RPW * (MODE_THREADS / 32);
   static constexpr int LDH = KP + 2;                // row stride: conflict-free 16-byte rows
-  static constexpr int BE = KP == 16 ? 1 : KP == 32 ? 2 : 4;  // edge of a thread's block of outputs
-  static constexpr int KB = KP / BE;                // blocks per edge: KB (KB + 1) / 2 <= 256 threads
+  static constexpr int LDG = KP + 4;                // row stride of G: conflict-free fragments
+  static constexpr int KB = KP / 8;                 // 8 x 8 blocks of U^T U per edge
+  static constexpr int NT = KB * (KB + 1) / 2;      // blocks of its upper triangle
+  static constexpr int TPW = (NT + MODE_THREADS / 32 - 1) / (MODE_THREADS / 32);  // a warp's blocks
 };
 
 // CTAs of a factor's cluster: one per 64 rows (16 above rank 32, where a
@@ -84,7 +88,7 @@ __host__ __device__ constexpr int mode_ctas(int64_t I, int k, int most) {
 template <int KP>
 constexpr size_t mode_smem_bytes(int64_t rows) {
   using S = ModeShape<KP>;
-  return ((size_t)rows * S::LDH + (KP == 16 ? (size_t)S::CHUNK * S::LDH : 0) + 2 * (size_t)KP * KP) *
+  return ((size_t)rows * S::LDH + (KP == 16 ? (size_t)S::CHUNK * S::LDH : 0) + (size_t)KP * (S::LDG + KP)) *
          sizeof(double);
 }
 inline size_t mode_smem(int k, int64_t rows) {
@@ -109,7 +113,7 @@ __device__ __forceinline__ double mode_warp_sums(const double* r) {
 template <int KP, int UPD>
 __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
   using S = ModeShape<KP>;
-  constexpr int LPR = S::LPR, CP = S::CP, LDH = S::LDH, CHUNK = S::CHUNK;
+  constexpr int LPR = S::LPR, CP = S::CP, LDH = S::LDH, CHUNK = S::CHUNK, LDG = S::LDG;
   static_assert(UPD == MODE_NONE || KP == 16, "the fused update is for ranks up to 16");
   cg::cluster_group cluster = cg::this_cluster();
   const int me = (int)cluster.block_rank(), CLm = a.CLm;
@@ -120,8 +124,8 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
   const int64_t r0 = me < CLm ? (int64_t)me * per : I;
   const int64_t r1 = (r0 + per) < I ? (r0 + per) : I;
   const int nrows = (int)(r1 > r0 ? r1 - r0 : 0);
-  double* gs = mode_sm;                    // G of the update; later the factor's U^T U
-  double* gsum = gs + KP * KP;             // U^T U of this CTA's rows
+  double* gs = mode_sm;                    // G of the update at stride LDG; later the factor's U^T U
+  double* gsum = gs + KP * LDG;            // U^T U of this CTA's rows
   double* tile = gsum + KP * KP;           // rows at stride LDH
   double* mt = tile + (size_t)per * LDH;   // CHUNK rows of M (update)
   __shared__ double lam[KP];
@@ -151,7 +155,7 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
     for (int e = tid; e < KP * KP; e += MODE_THREADS) {
       const int i = e / KP, j = e % KP;
       const bool in = i < k && j < k;
-      mode_copy8(gs + e, a.Gloo + (in ? i * k + j : 0), in);
+      mode_copy8(gs + i * LDG + j, a.Gloo + (in ? i * k + j : 0), in);
     }
     if (nrows > 0) stage(mt, a.M + r0 * k, nrows < CHUNK ? nrows : CHUNK);
   }
@@ -182,20 +186,20 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
         const bool live = row < nrows;
         // lanes past the last row shadow the warp's first one
         double* hrow = tile + (size_t)(live ? row : ch + warp * S::RPW) * LDH;
-        double g[CP], h[CP];
+        // H G of the warp's eight rows, four columns of H a product; a lane's
+        // columns are those of its accumulators
+        static_assert(LPR == 4, "the accumulators' layout");
+        double g[CP / 2][2], h[CP];
 #pragma unroll
-        for (int s = 0; s < CP; ++s) g[s] = 0.0;
-#pragma unroll 2
-        for (int j = 0; j < k; j += 2) {
-          const double2 hj = *reinterpret_cast<const double2*>(hrow + j);
+        for (int p = 0; p < CP / 2; ++p) g[p][0] = g[p][1] = 0.0;
 #pragma unroll
-          for (int p = 0; p < CP / 2; ++p) {
-            const double2 ga = *reinterpret_cast<const double2*>(gs + j * KP + p * 2 * LPR + 2 * q);
-            const double2 gb = *reinterpret_cast<const double2*>(gs + (j + 1) * KP + p * 2 * LPR + 2 * q);
-            g[2 * p] = fma(hj.y, gb.x, fma(hj.x, ga.x, g[2 * p]));
-            g[2 * p + 1] = fma(hj.y, gb.y, fma(hj.x, ga.y, g[2 * p + 1]));
+        for (int j = 0; j < KP; j += 4)
+          if (j < k) {
+            const double ha = hrow[j + q];
+#pragma unroll
+            for (int p = 0; p < CP / 2; ++p)
+              dmma_m8n8k4(g[p], ha, gs[(j + q) * LDG + p * 2 * LPR + lane / LPR]);
           }
-        }
 #pragma unroll
         for (int p = 0; p < CP / 2; ++p) {
           const double2 v = *reinterpret_cast<const double2*>(hrow + p * 2 * LPR + 2 * q);
@@ -222,15 +226,15 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
               for (int b = 0; b < 2; ++b) {
                 const int i = p * 2 * LPR + 2 * o + b;
                 if (i < k) {
-                  double u = h[2 * p + b] + (m[2 * p + b] - g[2 * p + b]);
+                  double u = h[2 * p + b] + (m[2 * p + b] - g[p][b]);
                   u = (u < kEps17) ? kEps17 : u;
                   const double delta = __shfl_sync(0xffffffffu, u - h[2 * p + b], o, LPR);
                   if (q == o) h[2 * p + b] = u;
 #pragma unroll
                   for (int p2 = p; p2 < CP / 2; ++p2) {
-                    const double2 gi = *reinterpret_cast<const double2*>(gs + i * KP + p2 * 2 * LPR + 2 * q);
-                    g[2 * p2] = fma(delta, gi.x, g[2 * p2]);
-                    g[2 * p2 + 1] = fma(delta, gi.y, g[2 * p2 + 1]);
+                    const double2 gi = *reinterpret_cast<const double2*>(gs + i * LDG + p2 * 2 * LPR + 2 * q);
+                    g[p2][0] = fma(delta, gi.x, g[p2][0]);
+                    g[p2][1] = fma(delta, gi.y, g[p2][1]);
                   }
                 }
               }
@@ -240,7 +244,7 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
               const int i = p * 2 * LPR + 2 * q + b;
-              if (i < k) h[2 * p + b] = (h[2 * p + b] * mrow[i]) / (g[2 * p + b] + a.eps);
+              if (i < k) h[2 * p + b] = (h[2 * p + b] * mrow[i]) / (g[p][b] + a.eps);
             }
         }
         __syncwarp();  // every lane of the row has read the old values
@@ -277,49 +281,40 @@ __device__ __forceinline__ void mode_cluster_body(const ModeArgs& a) {
     if (lane == 0) red[warp] = inner;
   }
 
-  // ---- U^T U of this CTA's rows: a BE x BE block of the upper triangle a
-  // thread, rows in increasing order
+  // ---- U^T U of this CTA's rows: a warp per 8 x 8 block of the upper triangle,
+  // four rows a product, in increasing order
   {
-    constexpr int BE = S::BE, KB = S::KB;
-    int ta, tb;
-    tri_block(tid, KB, ta, tb);
-    if (ta < KB && BE * ta < k) {
-      double acc[BE][BE];
+    constexpr int KB = S::KB, TPW = S::TPW, NW = MODE_THREADS / 32;
+    const int fg = lane >> 2, ft = lane & 3;
+    double acc[TPW][2];
+    int oa[TPW], ob[TPW];  // columns of the blocks' operands (-1: none)
 #pragma unroll
-      for (int u = 0; u < BE; ++u)
-#pragma unroll
-        for (int v = 0; v < BE; ++v) acc[u][v] = 0.0;
-#pragma unroll 4
-      for (int i = 0; i < nrows; ++i) {
-        const double* r = tile + (size_t)i * LDH;
-        double av[BE], bv[BE];
-        if constexpr (BE == 1) {
-          av[0] = r[ta];
-          bv[0] = r[tb];
-        } else {
-#pragma unroll
-          for (int u = 0; u < BE; u += 2) {
-            const double2 x = *reinterpret_cast<const double2*>(r + BE * ta + u);
-            const double2 y = *reinterpret_cast<const double2*>(r + BE * tb + u);
-            av[u] = x.x;
-            av[u + 1] = x.y;
-            bv[u] = y.x;
-            bv[u + 1] = y.y;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < BE; ++u)
-#pragma unroll
-          for (int v = 0; v < BE; ++v) acc[u][v] = fma(av[u], bv[v], acc[u][v]);
-      }
-#pragma unroll
-      for (int u = 0; u < BE; ++u)
-#pragma unroll
-        for (int v = 0; v < BE; ++v) {
-          gsum[(BE * ta + u) * KP + BE * tb + v] = acc[u][v];
-          gsum[(BE * tb + v) * KP + BE * ta + u] = acc[u][v];
-        }
+    for (int u = 0; u < TPW; ++u) {
+      int ta, tb;
+      tri_block(warp + NW * u, KB, ta, tb);
+      oa[u] = ta < KB && 8 * ta < k ? 8 * ta : -1;
+      ob[u] = 8 * tb;
+      acc[u][0] = acc[u][1] = 0.0;
     }
+    const double* r = tile + (size_t)ft * LDH + fg;
+    auto step = [&](const double* r4, bool in) {
+#pragma unroll
+      for (int u = 0; u < TPW; ++u)
+        if (oa[u] >= 0) dmma_m8n8k4(acc[u], in ? r4[oa[u]] : 0.0, in ? r4[ob[u]] : 0.0);
+    };
+    int i = 0;
+#pragma unroll 4
+    for (; i + 4 <= nrows; i += 4) step(r + (size_t)i * LDH, true);
+    if (i < nrows) step(r + (size_t)i * LDH, i + ft < nrows);
+#pragma unroll
+    for (int u = 0; u < TPW; ++u)
+      if (oa[u] >= 0) {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          gsum[(oa[u] + fg) * KP + ob[u] + 2 * ft + v] = acc[u][v];
+          if (oa[u] != ob[u]) gsum[(ob[u] + 2 * ft + v) * KP + oa[u] + fg] = acc[u][v];
+        }
+      }
     __syncthreads();
     if (err && tid == 0) inner_sum = mode_warp_sums(red);
   }

@@ -1412,15 +1412,20 @@ __device__ __forceinline__ void tc_wimage_body(const WGen& wg, int64_t K, int k,
     return;
   }
   const int64_t total = nk * KP * (TC_BK / 8);
+  const bool one = wg.nf == 1;
   for (int64_t e = bx * blockDim.x + threadIdx.x; e < total; e += gx * blockDim.x) {
     const int r = (int)(e % KP);
     const int ch = (int)((e / KP) % (TC_BK / 8));
     const int64_t kb = e / ((int64_t)(TC_BK / 8) * KP);
+    const int64_t j0 = kb * TC_BK + ch * 8;
     double w[8];
+    if (one) {  // all eight loads before any is converted
+      const double* f = wg.f[0] + j0 * k + r;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int64_t j = kb * TC_BK + ch * 8 + u;
-      w[u] = (j < K && r < k) ? (wg.nf == 1 ? wg.f[0][j * k + r] : wgen_eval(wg, j, r, k)) : 0.0;
+      for (int u = 0; u < 8; ++u) w[u] = (j0 + u < K && r < k) ? f[(int64_t)u * k] : 0.0;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) w[u] = (j0 + u < K && r < k) ? wgen_eval(wg, j0 + u, r, k) : 0.0;
     }
     tc_wimage_store<KP>(w, kb, ch, r, img);
   }

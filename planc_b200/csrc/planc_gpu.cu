@@ -2881,16 +2881,15 @@ bool batch_groupable(const planc_gpu_batch* b, int algo) {
 
 // Host copies of the argument tables, laid out as they are copied to the
 // batch's device buffer after capture (the captured launches hold device
-// addresses inside that buffer).
+// addresses inside that buffer). Tables larger than the buffer are laid out all
+// the same: the capture is then repeated with a buffer of their size.
 struct GrpTables {
   std::vector<uint8_t> host;
   uint8_t* dev = nullptr;
-  size_t cap = 0;
   template <typename T>
   const T* put(const std::vector<T>& v) {
     size_t off = (host.size() + 255) & ~(size_t)255;
     const size_t bytes = v.size() * sizeof(T);
-    if (off + bytes > cap) fail(PLANC_GPU_ERR_STATE, "internal: grouped argument tables too large");
     host.resize(off + bytes);
     memcpy(host.data() + off, v.data(), bytes);
     return reinterpret_cast<const T*>(dev + off);
@@ -2959,17 +2958,9 @@ void grp_mode(GrpTables& tab, cudaStream_t st, const std::vector<planc_gpu_ctx*>
   }
 }
 
-void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
-  batch_reset_graph(b);
+// One iteration of every member, captured on the master stream.
+cudaGraph_t grp_capture(planc_gpu_batch* b, int algo, bool err, GrpTables& tab) {
   const auto& ms = b->members;
-  const size_t cap = 32 * ((size_t)ms.size() * 512 + 256);
-  if (b->grp_cap < cap) {
-    dalloc(&b->grp_dev, cap);
-    b->grp_cap = cap;
-  }
-  GrpTables tab;
-  tab.dev = b->grp_dev;
-  tab.cap = b->grp_cap;
   cudaStream_t st = b->master;
   auto fork = [&] {
     CK(cudaEventRecord(b->fork, st));
@@ -2981,15 +2972,6 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
       CK(cudaStreamWaitEvent(st, b->joins[i], 0));
     }
   };
-  if (b->precision == PLANC_GPU_PREC_BF16X2) {
-    CK((tcg_set_attrs<16, true>()));
-    CK((tcg_set_attrs<32, true>()));
-    CK((tcg_set_attrs<64, true>()));
-  } else {
-    CK((tcg_set_attrs<16, false>()));
-    CK((tcg_set_attrs<32, false>()));
-    CK((tcg_set_attrs<64, false>()));
-  }
   cudaGraph_t graph = nullptr;
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   try {
@@ -3232,13 +3214,45 @@ void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
     throw;
   }
   CK(cudaStreamEndCapture(st, &graph));
+  return graph;
+}
+
+void batch_capture_grouped(planc_gpu_batch* b, int algo, bool err) {
+  batch_reset_graph(b);
+  if (b->precision == PLANC_GPU_PREC_BF16X2) {
+    CK((tcg_set_attrs<16, true>()));
+    CK((tcg_set_attrs<32, true>()));
+    CK((tcg_set_attrs<64, true>()));
+  } else {
+    CK((tcg_set_attrs<16, false>()));
+    CK((tcg_set_attrs<32, false>()));
+    CK((tcg_set_attrs<64, false>()));
+  }
+  // 16 KB a member hold the tables of tensors up to about 230000 rows of P;
+  // the tile lists of larger ones grow with their size
+  size_t need = 32 * (b->members.size() * 512 + 256);
+  GrpTables tab;
+  cudaGraph_t graph = nullptr;
+  for (;;) {
+    if (b->grp_cap < need) {
+      b->grp_cap = 0;
+      dalloc(&b->grp_dev, need);
+      b->grp_cap = need;
+    }
+    tab.host.clear();
+    tab.dev = b->grp_dev;
+    graph = grp_capture(b, algo, err, tab);
+    need = tab.host.size();
+    if (need <= b->grp_cap) break;
+    cudaGraphDestroy(graph);
+  }
   cudaError_t e = cudaGraphInstantiate(&b->gexec, graph, 0);
   cudaGraphDestroy(graph);
   cuda_check(e, "cudaGraphInstantiate (grouped batch)");
   // the captured launches read their tables from grp_dev from the first replay
   // on (no earlier replay of this batch is still running: the master stream
   // is drained first)
-  CK(cudaStreamSynchronize(st));
+  CK(cudaStreamSynchronize(b->master));
   CK(cudaMemcpy(b->grp_dev, tab.host.data(), tab.host.size(), cudaMemcpyHostToDevice));
   b->g_algo = algo;
   b->g_err = err ? 1 : 0;

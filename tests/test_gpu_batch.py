@@ -92,3 +92,26 @@ def test_batch_grouped_phases_give_the_same_bits(gpu, prec, algo, monkeypatch):
     for (Fa, la), (Fb, lb) in zip(f1, f0):
         assert np.array_equal(la, lb)
         assert all(np.array_equal(a, b_) for a, b_ in zip(Fa, Fb))
+
+
+@pytest.mark.parametrize("count,dims", [(64, (492, 487, 2)), (4, (560, 541, 3))])
+def test_batch_tables_grow_with_the_members(gpu, count, dims):
+    # the tile lists of tensors with this many rows (I_0 I_1) need more than
+    # 16 KB of argument tables a member
+    k = 4
+    members = [cp_tensor(dims, k, noise=0.01, seed=80 + i)[0].astype(np.float32) for i in range(2)]
+    F0 = [init_factors(dims, k, seed=180 + i) for i in range(2)]
+    with gpu.Batch(0, "bf16", nstreams=4) as b:
+        for i in range(count):
+            b.add(members[i % 2], F0[i % 2])
+        errs = b.run("hals", 2)
+        last = b.get_factors(count - 1)
+    for i in range(2):
+        with gpu.Context(0, "bf16") as c:
+            c.set_tensor(members[i])
+            c.set_factors(F0[i])
+            e = c.run("hals", 2)
+            F, lam = c.get_factors()
+        assert np.array_equal(errs[i::2], np.tile(e, (count // 2, 1)))
+    assert np.array_equal(last[1], lam)
+    assert all(np.array_equal(a, b_) for a, b_ in zip(last[0], F))

@@ -55,13 +55,15 @@ struct GrpTtvL {
   unsigned gx;
 };
 
-// Four consecutive b a CTA: a member's rows are few (32 to 256), and the
-// launch has CTAs enough (256 members: 340 us an iteration with one b a CTA).
+// NB consecutive b a CTA: four where the launch still has CTAs enough (256
+// members of 32..256 per mode: 340 us an iteration with one b a CTA, 228 with
+// four), one where it would leave SMs idle (the rule is the caller's).
 constexpr int GRP_TTVL_NB = 4;
+template <int NB>
 __global__ void __launch_bounds__(256) k_grp_ttv_left(const GrpTtvL* __restrict__ a) {
   const GrpTtvL& g = a[blockIdx.z];
   if (blockIdx.x >= g.gx) return;
-  ttv_left_body<float, GRP_TTVL_NB>(g.T, g.A, g.B, g.k, g.F, g.out, blockIdx.x, g.gx);
+  ttv_left_body<float, NB>(g.T, g.A, g.B, g.k, g.F, g.out, blockIdx.x, g.gx);
 }
 
 __global__ void __launch_bounds__(256, 4) k_grp_ttv_left_f4(const GrpTtvL* __restrict__ a) {

@@ -3083,12 +3083,22 @@ cudaGraph_t grp_capture(planc_gpu_batch* b, int algo, bool err, GrpTables& tab) 
         if (k % 4 == 0 && g2 >= eff_sm(m) && g2 <= 65535)
           f4.push_back(GrpTtvL{m->P32, A, B, k, m->F[0], m->M[1], (unsigned)g2});
         else
-          plain.push_back(GrpTtvL{m->P32, A, B, k, m->F[0], m->M[1],
-                                  (unsigned)std::min<int64_t>((B + GRP_TTVL_NB - 1) / GRP_TTVL_NB, 65535)});
+          plain.push_back(GrpTtvL{m->P32, A, B, k, m->F[0], m->M[1], 0});
       }
-      if (!plain.empty())
-        k_grp_ttv_left<<<dim3(grp_max(plain, &GrpTtvL::gx), 1, (unsigned)plain.size()), 256, 0, st>>>(
-            tab.put(plain));
+      if (!plain.empty()) {
+        // GRP_TTVL_NB b a CTA while that leaves two CTAs an SM, else one (the
+        // sums' order is the same): 32 members of 200 x 150 x 40, rank 4, 209 us
+        // an iteration against 214 with one; a single one of 250 x 250 x 250 has
+        // 63 CTAs of four
+        int64_t ctas = 0;
+        for (const GrpTtvL& t : plain) ctas += (t.B + GRP_TTVL_NB - 1) / GRP_TTVL_NB;
+        const bool many = ctas >= 2 * (int64_t)sms;
+        const int nb = many ? GRP_TTVL_NB : 1;
+        for (GrpTtvL& t : plain) t.gx = (unsigned)std::min<int64_t>((t.B + nb - 1) / nb, 65535);
+        const dim3 g(grp_max(plain, &GrpTtvL::gx), 1, (unsigned)plain.size());
+        if (many) k_grp_ttv_left<GRP_TTVL_NB><<<g, 256, 0, st>>>(tab.put(plain));
+        else k_grp_ttv_left<1><<<g, 256, 0, st>>>(tab.put(plain));
+      }
       if (!f4.empty())
         k_grp_ttv_left_f4<<<dim3(grp_max(f4, &GrpTtvL::gx), 1, (unsigned)f4.size()), 256, 0, st>>>(
             tab.put(f4));
@@ -3106,6 +3116,12 @@ cudaGraph_t grp_capture(planc_gpu_batch* b, int algo, bool err, GrpTables& tab) 
     std::vector<TcgLong> gmem(ms.size());
     std::vector<TcgWimg> wimgs[3][2];
     std::vector<TcgUnit> gunits[3][2];
+    int64_t image_tiles = 0;  // tensor tiles of those members' contractions
+    for (auto* m : ms)
+      if (!tc_left_factored(m->tct) && left_via_long(m)) {
+        const int64_t MT = tc_long_mt(m->tct.R, m->k);
+        image_tiles += (m->tct.L + TC_BK - 1) / TC_BK * ((m->tct.R + MT * TC_BM - 1) / (MT * TC_BM)) * MT;
+      }
     fork();
     for (size_t mi = 0; mi < ms.size(); ++mi) {
       planc_gpu_ctx* m = ms[mi];
@@ -3122,17 +3138,24 @@ cudaGraph_t grp_capture(planc_gpu_batch* b, int algo, bool err, GrpTables& tab) 
         continue;
       }
       if (left_via_long(m)) {
-        // as long_contract; min(splits, 8) partials are left to the grouped sum
+        // as long_contract; the partials are left to the grouped sum
         if (tc_long_scratch_elems(m->tct, true, m->k, eff_sm(m)) > m->scratch_elems)
           fail(PLANC_GPU_ERR_STATE, "internal: split-K scratch larger than planned");
         const int ci = kpi(m->k), kp = tc_kpad(m->k), MT = tc_long_mt(m->tct.R, m->k);
         const int64_t nk = (m->tct.L + TC_BK - 1) / TC_BK;
         int mg = 0, ns = 0;
         tc_long_plan(m->tct.R, m->tct.L, m->k, eff_sm(m), &mg, &ns);
-        const int np = std::min(ns, 8);
+        // units of an eighth of a row group while they last no longer than two
+        // average SMs' shares of all members' tiles, else a unit a split: few
+        // members leave most SMs idle with eighths (one of 250^3, rank 16: 147 us
+        // an iteration against 87; four, 184 / 158; one of 500 x 490 x 500, 397 /
+        // 193), many write and read more partials without (sixteen of 250^3, 418
+        // against 373; eight of 250 x 249 x 200, rank 40, 484 / 460)
+        const bool eighths = nk * MT * sms <= 2 * tcg_lanes * image_tiles;
+        const int np = eighths ? std::min(ns, tcg_lanes) : ns;
         wimgs[ci][MT - 1].push_back(TcgWimg{m->F[0], m->F[1], m->tct.L, nk, (int)m->dims[0], m->k,
                                             tc_wimage_blocks(nk, kp), m->tct.wimg});
-        gmem[mi] = TcgLong{m->tct.wimg, np > 1 ? m->scratch : m->M[2], m->tct.R, m->tct.L, m->k, ns};
+        gmem[mi] = TcgLong{m->tct.wimg, np > 1 ? m->scratch : m->M[2], m->tct.R, m->tct.L, m->k, ns, np};
         for (int jg = 0; jg < mg; ++jg)
           for (int y = 0; y < np; ++y) gunits[ci][MT - 1].push_back(TcgUnit{(int)mi, jg, y, 0});
         if (np > 1) red.push_back(grp_red(m->scratch, np, m->R * m->k, m->M[2]));
@@ -3154,7 +3177,8 @@ cudaGraph_t grp_capture(planc_gpu_batch* b, int algo, bool err, GrpTables& tab) 
           if (uv.empty()) continue;
           // longest units first: the CTAs take them in turn
           std::stable_sort(uv.begin(), uv.end(), [&](const TcgUnit& a, const TcgUnit& c) {
-            return gmem[a.member].L > gmem[c.member].L;
+            const TcgLong &x = gmem[a.member], &y = gmem[c.member];
+            return x.L * y.parts > y.L * x.parts;
           });
           const auto& wv = wimgs[ci][mt - 1];
           cudaStream_t ws = b->workers[(size_t)(ci * 2 + mt - 1) % b->workers.size()];

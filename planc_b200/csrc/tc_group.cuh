@@ -493,22 +493,29 @@ __global__ void k_tc_wimage_grp(const TcgWimg* __restrict__ a) {
 // K-major): rows j < R, K = l < L, nsplit its own launch's split count
 struct TcgLong {
   const uint8_t* wimg;
-  double* part;  // min(nsplit, 8) partials of R x k (the result itself for one)
+  double* part;  // `parts` partials of R x k (the result itself for one)
   int64_t R, L;
   int k;
   int nsplit;
+  int parts;  // units a row group: nsplit, or tcg_lanes of them
 };
+
+// Lanes of reduce_splits_body's sum: lane s adds the partials s, s + 8, ...
+constexpr int tcg_lanes = 8;
 
 // The long-K contraction of every member in one persistent launch. A member's
 // own launch spreads its K over up to 148 splits, a few blocks each, and a
-// tensor of a few MB then writes and reads more partials than it has data. A
-// unit here is the splits y = sub, sub + 8, ... of a row group, for one of 8
-// values of sub: its CTA runs them one after another and adds each split's sum
-// to FP64 accumulators in shared memory, in the order in which
-// reduce_splits_body's lane `sub` adds their partials. The 8 partials left are
-// then summed as that kernel's lanes are, so the bits are those of the member's
-// own launches. Bound by the tensor's bytes and the images': 256 tensors of
-// 32..256 per mode, images, contractions and sums: see the batch's capture.
+// tensor of a few MB then writes and reads more partials than it has data. So
+// in a batch that fills the GPU a unit is the splits y = sub, sub + 8, ... of a
+// row group, for one of 8 values of sub: its CTA runs them one after another
+// and adds each split's sum to FP64 accumulators in shared memory, in the order
+// in which reduce_splits_body's lane `sub` adds their partials. The 8 partials
+// left are then summed as that kernel's lanes are, so the bits are those of the
+// member's own launches. A member whose eighth would outlast the rest of the
+// batch (see the capture) has a unit a split and leaves all its partials to the
+// sum, as its own launch does. Bound by the tensor's bytes and the images': 256
+// tensors of 32..256 per mode, images, contractions and sums: see the batch's
+// capture.
 // KP x 128 x MT accumulators in the last ACC bytes of dynamic shared memory;
 // `units` are sorted by decreasing work.
 template <int KP, int MT>
@@ -590,7 +597,7 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
         const int nk = (int)((m.L + TC_BK - 1) / TC_BK);
         const int ngroups = (nk + group - 1) / group;
         const int row0 = U.jg * MT * TC_BM;
-        for (int y = U.y; y < m.nsplit && ok; y += 8)
+        for (int y = U.y; y < m.nsplit && ok; y += m.parts)
           for (int g = y; g < ngroups && ok; g += m.nsplit) {
             const int kb1 = min((g + 1) * group, nk);
             for (int kb = g * group; kb < kb1; ++kb) {
@@ -621,7 +628,7 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
         const TcgLong& m = mem[U.member];
         const int nk = (int)((m.L + TC_BK - 1) / TC_BK);
         const int ngroups = (nk + group - 1) / group;
-        for (int y = U.y; y < m.nsplit && ok; y += 8)
+        for (int y = U.y; y < m.nsplit && ok; y += m.parts)
           for (int g = y; g < ngroups && ok; g += m.nsplit) {
             const int kb0 = g * group, kb1 = min((g + 1) * group, nk);
             if (!mbar_wait(acce(buf), ((aph >> buf) & 1) ^ 1, abort_flag, status)) { ok = false; break; }
@@ -664,7 +671,7 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
       const TcgLong& m = mem[U.member];
       const int nk = (int)((m.L + TC_BK - 1) / TC_BK);
       const int ngroups = (nk + group - 1) / group;
-      for (int y = U.y; y < m.nsplit && ok; y += 8) {
+      for (int y = U.y; y < m.nsplit && ok; y += m.parts) {
         float sum[MT][KP];
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)

@@ -115,3 +115,38 @@ def test_batch_tables_grow_with_the_members(gpu, count, dims):
         assert np.array_equal(errs[i::2], np.tile(e, (count // 2, 1)))
     assert np.array_equal(last[1], lam)
     assert all(np.array_equal(a, b_) for a, b_ in zip(last[0], F))
+
+
+def _image_members(few):
+    # last modes above 128 (two row tiles a CTA up to rank 32, several row
+    # groups above), I_0 not a multiple of 64, I_1 not a multiple of 4
+    specs = [((61, 55, 200), 16)] if few else [
+        ((61, 54, 129), 8), ((59, 57, 200), 16), ((62, 53, 300), 20), ((66, 50, 256), 32),
+        ((60, 55, 140), 40), ((65, 51, 128), 64), ((57, 58, 90), 4), ((63, 52, 513), 24),
+        ((61, 53, 300), 12), ((58, 57, 257), 33), ((67, 49, 131), 30), ((70, 47, 2), 5)]
+    out = []
+    for i, (dims, k) in enumerate(specs):
+        X, _ = cp_tensor(dims, min(k, 8), noise=0.01, seed=90 + i)
+        out.append((X.astype(np.float32), init_factors(dims, k, seed=190 + i)))
+    return out
+
+
+@pytest.mark.parametrize("few", [True, False])
+@pytest.mark.parametrize("prec", ["bf16", "bf16x2"])
+def test_batch_long_contraction_gives_the_same_bits(gpu, prec, few, monkeypatch):
+    # units of a split (few members) and of an eighth of a row group (many)
+    # against the members' own launches
+    members = _image_members(few)
+    res = {}
+    for grouped in ("1", "0"):
+        monkeypatch.setenv("PLANC_GPU_BATCH_GROUPED", grouped)
+        with gpu.Batch(0, prec, nstreams=4) as b:
+            for X, F0 in members:
+                b.add(X, F0)
+            errs = b.run("hals", 3)
+            res[grouped] = (errs, [b.get_factors(i) for i in range(len(members))])
+    (e1, f1), (e0, f0) = res["1"], res["0"]
+    assert np.array_equal(e1, e0)
+    for (Fa, la), (Fb, lb) in zip(f1, f0):
+        assert np.array_equal(la, lb)
+        assert all(np.array_equal(a, b_) for a, b_ in zip(Fa, Fb))

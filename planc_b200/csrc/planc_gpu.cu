@@ -193,14 +193,15 @@ struct planc_gpu_ctx {
   int nmf_galgo = -1;
   int64_t nmf_gepoch = -1;
 
-  // cached graphs of g_iters iterations: [0] the plain iteration, [1] iteration
-  // + Nesterov acceleration
-  cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  int g_algo[2] = {-1, -1}, g_dimtree[2] = {-1, -1}, g_err[2] = {-1, -1}, g_iters[2] = {0, 0};
-  // configuration of the last run (its buffers' epoch with it): a run of
-  // another one launches its kernels one by one
-  int r_algo = -1, r_dimtree = -1, r_err = -1;
-  int64_t r_epoch = -1;
+  // graphs of iterations (planc_gpu_run), at most kMaxGraphs: the least
+  // recently used one goes first
+  struct IterGraph {
+    int algo, dimtree, err, accel, iters;  // accel: Nesterov's acceleration after each iteration
+    cudaGraphExec_t exec;                  // null: asked for once, launched kernel by kernel
+    int64_t used;
+  };
+  std::vector<IterGraph> graphs;
+  int64_t graph_clock = 0;
 
   bool timing = false;
   bool capturing = false;
@@ -633,10 +634,13 @@ void ensure_buffers(planc_gpu_ctx* c) {
     }
 }
 
-// Error-history buffer of at least `n` entries (reallocation bumps the epoch).
+// Error-history buffer of at least `n` entries (reallocation bumps the epoch):
+// 256 or more, then twice as many each time, so that a longer run than the ones
+// before it seldom moves the buffer that the cached graphs hold.
 void ensure_errs(planc_gpu_ctx* c, int n) {
-  if (n < 1) n = 1;
   if (!c->errs_dev || n > c->errs_cap) {
+    n = std::max(n, std::max(256, 2 * std::min(c->errs_cap, 1 << 20)));
+    c->errs_cap = 0;
     dalloc(&c->errs_dev, (size_t)n);
     c->errs_cap = n;
     c->buf_epoch++;
@@ -1535,15 +1539,17 @@ void check_status(planc_gpu_ctx* c) {
   }
 }
 
-void reset_graph(planc_gpu_ctx* c) {
-  for (int v = 0; v < 2; ++v) {
-    if (c->gexec[v]) {
-      cudaGraphExecDestroy(c->gexec[v]);
-      c->gexec[v] = nullptr;
-    }
-    c->g_algo[v] = c->g_dimtree[v] = c->g_err[v] = -1;
-    c->g_iters[v] = 0;
+// Drops the captured graphs; which ones were asked for is remembered.
+void drop_graphs(planc_gpu_ctx* c) {
+  for (auto& g : c->graphs) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
   }
+}
+
+void reset_graph(planc_gpu_ctx* c) {
+  drop_graphs(c);
+  c->graphs.clear();
 }
 
 void free_update_state(planc_gpu_ctx* c) {
@@ -2100,7 +2106,7 @@ bool known_algo(int algo) {
 }
 
 // Iterations of a graph for a run of `count`: up to 8, so that the run divides
-// evenly where it can (the rest are launched one by one). Between two graph
+// evenly where it can (a second graph takes the rest). Between two graph
 // launches the GPU idles for 5 to 6 us, a tenth of a small iteration.
 int graph_iters(int count) {
   if (count <= 8) return count;
@@ -2110,23 +2116,35 @@ int graph_iters(int count) {
   return best;
 }
 
-// Captures (once) and returns the graph of g_iters[variant] iterations for a
-// run of `count`; variant 1 appends the Nesterov acceleration to each. A graph
-// of fewer iterations than such a run takes is captured again.
-cudaGraphExec_t iteration_graph(planc_gpu_ctx* c, int algo, bool dt, bool err, int variant, int count) {
-  const int iters = graph_iters(count);
-  if (c->gexec[variant] && c->g_algo[variant] == algo && c->g_dimtree[variant] == (int)dt &&
-      c->g_err[variant] == (int)err && c->g_iters[variant] >= iters)
-    return c->gexec[variant];
-  if (c->gexec[variant]) {
-    cudaGraphExecDestroy(c->gexec[variant]);
-    c->gexec[variant] = nullptr;
+constexpr size_t kMaxGraphs = 16;
+
+// The graph of `iters` iterations, captured when it is asked for a second time
+// or `at_once` (else null: the caller launches the kernels one by one). The
+// capture and instantiation of a graph cost more than one short run saves.
+cudaGraphExec_t iteration_graph(planc_gpu_ctx* c, int algo, bool dt, bool err, bool accel, int iters,
+                                bool at_once) {
+  auto it = std::find_if(c->graphs.begin(), c->graphs.end(), [&](const auto& g) {
+    return g.algo == algo && g.dimtree == (int)dt && g.err == (int)err && g.accel == (int)accel &&
+           g.iters == iters;
+  });
+  if (it == c->graphs.end()) {
+    if (c->graphs.size() >= kMaxGraphs) {
+      auto old = std::min_element(c->graphs.begin(), c->graphs.end(),
+                                  [](const auto& a, const auto& b) { return a.used < b.used; });
+      if (old->exec) cudaGraphExecDestroy(old->exec);
+      c->graphs.erase(old);
+    }
+    c->graphs.push_back({algo, (int)dt, (int)err, (int)accel, iters, nullptr, ++c->graph_clock});
+    if (!at_once) return nullptr;
+    it = c->graphs.end() - 1;
   }
-  cudaGraph_t graph;
+  it->used = ++c->graph_clock;
+  if (it->exec) return it->exec;
+  cudaGraph_t graph = nullptr;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   c->capturing = true;
   try {
-    for (int i = 0; i < iters; ++i) one_iteration(c, algo, dt, err, variant == 1);
+    for (int i = 0; i < iters; ++i) one_iteration(c, algo, dt, err, accel);
   } catch (...) {
     c->capturing = false;
     cudaStreamEndCapture(c->stream, &graph);
@@ -2135,14 +2153,11 @@ cudaGraphExec_t iteration_graph(planc_gpu_ctx* c, int algo, bool dt, bool err, i
   }
   c->capturing = false;
   CK(cudaStreamEndCapture(c->stream, &graph));
-  cudaError_t e = cudaGraphInstantiate(&c->gexec[variant], graph, 0);
+  cudaError_t e = cudaGraphInstantiate(&it->exec, graph, 0);
   cudaGraphDestroy(graph);
+  if (e != cudaSuccess) it->exec = nullptr;
   cuda_check(e, "cudaGraphInstantiate");
-  c->g_algo[variant] = algo;
-  c->g_dimtree[variant] = (int)dt;
-  c->g_err[variant] = (int)err;
-  c->g_iters[variant] = iters;
-  return c->gexec[variant];
+  return it->exec;
 }
 
 }  // namespace
@@ -2166,33 +2181,28 @@ int planc_gpu_run(planc_gpu_ctx* c, int algo, int iters, int dimtree, int comput
     const bool err = compute_error != 0 || nes;
     ensure_errs(c, err ? iters : 1);
     ensure_update_state(c, algo);
-    if (c->g_epoch != c->buf_epoch) reset_graph(c);
+    if (c->g_epoch != c->buf_epoch) drop_graphs(c);  // a buffer moved
+    c->g_epoch = c->buf_epoch;
     CK(cudaMemsetAsync(c->counter_dev, 0, sizeof(int), c->stream));
     gram_loo(c, 0);
-    // A configuration's first short run launches its kernels one by one (the
-    // capture and instantiation of a graph cost more than it saves there), the
-    // next ones replay graphs.
-    const bool seen = c->r_algo == algo && c->r_dimtree == (int)dt && c->r_err == (int)err &&
-                      c->r_epoch == c->buf_epoch;
-    const bool use_graph = !c->timing && (seen || iters > 32);
-    c->r_algo = algo;
-    c->r_dimtree = dt;
-    c->r_err = err;
-    c->r_epoch = c->buf_epoch;
     // AUNTF::computeNTF restarts its iteration count at 0 on every call and
     // NTFNES accelerates from iteration acc_start + 1 = 6 on
     // (ntf/auntf.hpp:129, ntf/ntfnes.hpp:65)
     const int plain = nes ? std::min(iters, 6) : iters;
     for (int variant = 0; variant < 2; ++variant) {
       const int count = variant == 0 ? plain : iters - plain;
-      int done = 0;
-      if (use_graph && count > 0) {
-        cudaGraphExec_t g = iteration_graph(c, algo, dt, err, variant, count);
-        for (; done + c->g_iters[variant] <= count; done += c->g_iters[variant])
-          CK(cudaGraphLaunch(g, c->stream));
-        c->g_epoch = c->buf_epoch;
+      const int per = graph_iters(count), tail = per > 0 ? count % per : 0;
+      auto graph_of = [&](int n, bool at_once) {
+        return n > 0 && !c->timing ? iteration_graph(c, algo, dt, err, variant == 1, n, at_once) : nullptr;
+      };
+      cudaGraphExec_t whole = graph_of(per, iters > 32), rest = graph_of(tail, false);
+      for (int done = 0; done < count - tail; done += whole ? per : 1) {
+        if (whole) CK(cudaGraphLaunch(whole, c->stream));
+        else one_iteration(c, algo, dt, err, variant == 1);
       }
-      for (; done < count; ++done) one_iteration(c, algo, dt, err, variant == 1);
+      if (rest) CK(cudaGraphLaunch(rest, c->stream));
+      else
+        for (int i = 0; i < tail; ++i) one_iteration(c, algo, dt, err, variant == 1);
     }
     if (compute_error && errs_out)
       CK(cudaMemcpyAsync(errs_out, c->errs_dev, iters * sizeof(double), cudaMemcpyDeviceToHost,

@@ -1668,6 +1668,10 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
   }
 }
 
+// Largest workspace planc_gpu_bpp_solve leaves with its context: 25000
+// right-hand sides of 64 unknowns.
+constexpr size_t kBppKeepBytes = (size_t)32 << 20;
+
 // Largest slab of factors and lambda that goes through one packed copy: above
 // 1 MB the second pass over host memory costs more than the calls it saves.
 constexpr size_t kPackElems = (size_t)1 << 17;
@@ -2335,8 +2339,9 @@ int planc_gpu_bpp_solve(planc_gpu_ctx* c, const double* AtA, const double* AtB, 
     if (ncols == 0) return;
     set_device(c);
     ensure_bpp_lu(c, n, ncols);
-    // one workspace for operands and results, kept by the context: five
-    // allocations and frees a call cost several times the solve
+    // one workspace for operands and results, kept by the context up to
+    // kBppKeepBytes: five allocations and frees a call cost several times the
+    // solve of a few thousand right-hand sides
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
     const size_t nA = up((size_t)n * n * 8), nB = up((size_t)n * ncols * 8), nP = up((size_t)n * ncols * 4),
                  nI = up((size_t)ncols * 4);
@@ -2347,6 +2352,15 @@ int planc_gpu_bpp_solve(planc_gpu_ctx* c, const double* AtA, const double* AtB, 
       CK(cudaMalloc(&c->bpp_ws, nA + 2 * nB + nP + nI));
       c->bpp_ws_bytes = nA + 2 * nB + nP + nI;
     }
+    struct Trim {  // whether the call succeeds or not
+      planc_gpu_ctx* c;
+      ~Trim() {
+        if (c->bpp_ws_bytes <= kBppKeepBytes) return;
+        cudaFree(c->bpp_ws);
+        c->bpp_ws = nullptr;
+        c->bpp_ws_bytes = 0;
+      }
+    } trim{c};
     uint8_t* w = (uint8_t*)c->bpp_ws;
     double* dA = (double*)w;
     double* dB = (double*)(w + nA);

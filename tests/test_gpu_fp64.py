@@ -420,3 +420,21 @@ def test_contraction_onto_few_rows(gpu, oracle_lib, dims, k):
         for n in range(len(dims)):
             for dimtree in (False, True):
                 assert rel(c.mttkrp(n, dimtree=dimtree), oracle_lib.mttkrp_direct(X, Fn, n)) < TOL
+
+
+def test_bpp_solve_gives_a_large_workspace_back(gpu):
+    import torch
+    n, ncols = 8, 1_000_000  # 164 MB of operands and results
+    rng = np.random.default_rng(91)
+    A = rng.random((40, n))
+    B = rng.standard_normal((n, ncols))
+    with gpu.Context(0, "fp64") as c:
+        small = c.bpp_solve(A.T @ A, B[:, :100])
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        X, P, it = c.bpp_solve(A.T @ A, B)
+        assert free - torch.cuda.mem_get_info()[0] <= 34 << 20
+        for a, b in zip((X[:, :100], P[:, :100], it[:100]), small):
+            assert np.array_equal(a, b)
+        for a, b in zip(c.bpp_solve(A.T @ A, B[:, :100]), small):
+            assert np.array_equal(a, b)

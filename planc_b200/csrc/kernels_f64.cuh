@@ -1368,7 +1368,7 @@ __global__ void __launch_bounds__(256) k_sumsq_partial(const T* __restrict__ X, 
 }
 
 // ---------------------------------------------------------------------------
-// Differentiable CP loss, 1/2 ||X - [[F_0..F_{N-1}]]||^2, in three fused
+// Differentiable CP loss, 1/2 ||X - [[F_0..F_{N-1}]]||^2, in two fused
 // launches around the MTTKRPs (the gradient form of ntf/ntfnes.hpp:138-147).
 // ---------------------------------------------------------------------------
 constexpr int CPG_BLOCKS = 16;  // row blocks per factor of the Gram kernel
@@ -1384,9 +1384,10 @@ struct CpFactors {
 // 1/2 ||X||^2 - <M_0, F_0> + 1/2 sum_ab prod_n G_n[a, b], in one launch.
 // Block (b, n) sums its share of the rows of F_n into part[n][b] (rows in
 // shared-memory tiles, a BE x BE block of the upper triangle a thread) and, for
-// n = 0, of <M_0, F_0>; the last block of a factor to finish (counter ctr[n])
-// adds the partials in order into G_n, and the last factor's (ctr[kMaxModes])
-// forms the loss. The counters are left at 0. Bound by latencies (a share is
+// n = 0, of <M_0, F_0> into the CPG_BLOCKS doubles before part; the last block
+// of a factor to finish (counter ctr[n]) adds the partials in order into G_n,
+// and the last factor's (ctr[kMaxModes]) forms the loss. The counters are left
+// at 0. Bound by latencies (a share is
 // 32 rows at 512); two loads from global memory a product, eight blocks a
 // factor and a launch of its own for the loss took 38 us at 512^3, rank 32.
 template <int KP>
@@ -1405,7 +1406,7 @@ __global__ void __launch_bounds__(256) k_cp_grams(CpFactors f, const double* __r
   const int64_t per = (I + CPG_BLOCKS - 1) / CPG_BLOCKS;
   const int64_t r0 = b * per, r1 = (r0 + per) < I ? (r0 + per) : I;
   const double* F = f.F[n];
-  double* inner_part = part + (int64_t)kMaxModes * CPG_BLOCKS * kMaxRank * kMaxRank;
+  double* inner_part = part - CPG_BLOCKS;
   int ta, tb;
   tri_block(tid, KB, ta, tb);
   const bool owner = ta < KB && BE * ta < k;

@@ -105,8 +105,10 @@ struct planc_gpu_ctx {
   double* X64 = nullptr;         // FP64 tensor (plain path)
   int64_t x64_elems = 0;
   void* stage = nullptr;         // host-upload staging buffer (kStageBytes), made on first use
-  double* cp_part = nullptr;     // CP-loss Gram partials (N x CPG_BLOCKS x k x k) and <M_0, F_0> ones
-  unsigned* cp_ctr = nullptr;    // completion counters, one a factor and one over the factors
+  // CP loss: completion counters (one a factor, one over the factors), <M_0, F_0>
+  // partials (CPG_BLOCKS), Gram partials (N x CPG_BLOCKS x k x k)
+  double* cp_ws = nullptr;
+  size_t cp_ws_elems = 0;
   double* norm_part = nullptr;   // per-block partial sums of squares of one chunk
   TcTensor tct;                  // tensor-core operand copy (BF16 paths)
   // copies with mode n moved last for the direct (non-tree) MTTKRP on the
@@ -1668,6 +1670,21 @@ void ensure_update_state(planc_gpu_ctx* c, int algo) {
   }
 }
 
+// The CP loss's workspace for the context's modes and rank (outside capture).
+constexpr size_t kCpCtrElems = 16;  // the counters' own 128-byte line
+static_assert((kMaxModes + 1) * sizeof(unsigned) <= kCpCtrElems * sizeof(double), "a counter a factor");
+size_t cp_ws_need(const planc_gpu_ctx* c) {
+  return kCpCtrElems + ((size_t)c->N * c->k * c->k + 1) * CPG_BLOCKS;
+}
+void ensure_cp_ws(planc_gpu_ctx* c) {
+  const size_t need = cp_ws_need(c);
+  if (c->cp_ws_elems >= need) return;
+  c->cp_ws_elems = 0;
+  dalloc(&c->cp_ws, need);
+  c->cp_ws_elems = need;
+  CK(cudaMemsetAsync(c->cp_ws, 0, kCpCtrElems * sizeof(double), c->stream));
+}
+
 // Largest workspace planc_gpu_bpp_solve leaves with its context: 25000
 // right-hand sides of 64 unknowns.
 constexpr size_t kBppKeepBytes = (size_t)32 << 20;
@@ -1720,9 +1737,8 @@ void free_all(planc_gpu_ctx* c) {
   c->x64_elems = 0;
   if (c->stage) cudaFree(c->stage);
   c->stage = nullptr;
-  f(c->cp_part);
-  if (c->cp_ctr) cudaFree(c->cp_ctr);
-  c->cp_ctr = nullptr;
+  f(c->cp_ws);
+  c->cp_ws_elems = 0;
   f(c->norm_part);
   tc_free(c->tct);
   for (int n = 0; n < kMaxModes; ++n) tc_free(c->tcd[n]);
@@ -2094,6 +2110,7 @@ int planc_gpu_set_factors(planc_gpu_ctx* c, const double* const* F, const double
     // lambda as set; the first leave-one-out product is formed by its user
     normalize_all(c);
     ensure_buffers(c);
+    if (c->cp_ws) ensure_cp_ws(c);  // the next loss may be under capture
     if (!packed) CK(cudaStreamSynchronize(c->stream));
     c->have_factors = true;
     c->nmf_have = false;
@@ -2502,17 +2519,16 @@ int planc_gpu_cp_loss_device(planc_gpu_ctx* c, const double* const* F_dev, const
     set_device(c);
     CpFactors f = cp_factors(c, F_dev);
     const int k = c->k;
-    if (!c->cp_part) {
+    if (c->cp_ws_elems < cp_ws_need(c)) {
       if (c->capturing) fail(PLANC_GPU_ERR_STATE, "CP-loss buffers would be made during capture");
-      CK(cudaMalloc(&c->cp_part,
-                    ((size_t)kMaxModes * CPG_BLOCKS * kMaxRank * kMaxRank + CPG_BLOCKS) * 8));
-      CK(cudaMalloc(&c->cp_ctr, (kMaxModes + 1) * sizeof(unsigned)));
-      CK(cudaMemsetAsync(c->cp_ctr, 0, (kMaxModes + 1) * sizeof(unsigned), c->stream));
+      ensure_cp_ws(c);
     }
+    unsigned* ctr = (unsigned*)c->cp_ws;
+    double* part = c->cp_ws + kCpCtrElems + CPG_BLOCKS;
     launch(c, KC_NORMGRAM, [&] {
       const dim3 grid(CPG_BLOCKS, c->N);
 #define CP_GRAMS(KP) \
-  k_cp_grams<KP><<<grid, 256, 0, c->stream>>>(f, M0_dev, c->cp_part, G_out, c->cp_ctr, c->normX2, loss_out)
+  k_cp_grams<KP><<<grid, 256, 0, c->stream>>>(f, M0_dev, part, G_out, ctr, c->normX2, loss_out)
       if (k <= 16) CP_GRAMS(16);
       else if (k <= 32) CP_GRAMS(32);
       else CP_GRAMS(64);

@@ -239,3 +239,40 @@ def test_cp_loss_grams_in_one_launch(gpu, oracle_lib, dims, k):
         # the gradient is a difference of two terms of about this size
         assert np.abs(Ft[n].grad.cpu().numpy() - (F[n] @ G - M)).max() < 1e-10 * np.abs(M).max()
     lossf.close()
+
+
+def test_cp_loss_workspace_follows_modes_and_rank(gpu):
+    import torch
+    X, F, lossf, Ft = _setup("fp64", dims=(20, 18, 16), k=4, seed=41)
+    lossf(*Ft)  # torch's own pools are warm from here on
+    X2, F2, loss2, Ft2 = _setup("fp64", dims=(20, 18, 16), k=4, seed=42)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    loss2(*Ft2)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= 2 << 20
+    loss2.close()
+    # a larger rank on the same context, its first loss under capture
+    k, c = 40, lossf.ctx
+    rng = np.random.default_rng(43)
+    G = [rng.random((d, k)) for d in X.shape]
+    Gt = [torch.tensor(g, device="cuda", dtype=torch.float64) for g in G]
+    ptrs = [g.data_ptr() for g in Gt]
+    M0 = torch.empty_like(Gt[0])
+    grams = torch.empty(3, k, k, device="cuda", dtype=torch.float64)
+    value = torch.empty((), device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    c.set_factors(G)
+    c.mttkrp_device(0, ptrs, M0.data_ptr(), dimtree=True, reuse=False)
+    c.sync()
+    s = torch.cuda.ExternalStream(c.stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s, capture_error_mode="thread_local"):
+        c.cp_loss_device(ptrs, M0.data_ptr(), grams.data_ptr(), value.data_ptr())
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    ref = 0.5 * np.sum((X - np.einsum("az,bz,cz->abc", *G)) ** 2)
+    assert abs(value.item() - ref) / ref < 1e-10
+    del graph
+    lossf.close()

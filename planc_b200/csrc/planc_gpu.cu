@@ -2397,6 +2397,17 @@ int planc_gpu_bpp_solve(planc_gpu_ctx* c, const double* AtA, const double* AtB, 
 }
 
 // ---- device building blocks of the distributed iteration
+namespace {
+// A call that only launched may run while the program captures another stream:
+// in the global mode that forbids allocations to this thread too, unless it
+// says that what it allocates has nothing to do with the capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { CK(cudaThreadExchangeStreamCaptureMode(&mode)); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+}  // namespace
+
 int planc_gpu_update_device(planc_gpu_ctx* c, int algo, double* H, const double* M,
                             const double* G, int64_t rows, int k) {
   return guarded([&] {
@@ -2428,7 +2439,10 @@ int planc_gpu_update_device(planc_gpu_ctx* c, int algo, double* H, const double*
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(c->stream, &cap));
     const bool packed = cap == cudaStreamCaptureStatusNone;
-    if (packed) ensure_bpp_lu(c, k, rows);
+    if (packed) {
+      RelaxedCapture other_streams;
+      ensure_bpp_lu(c, k, rows);
+    }
     launch(c, KC_BPP, [&] {
       launch_bpp(c, G, M, k, rows, H, nullptr, nullptr, c->bpp_warm ? H : nullptr, packed);
     });

@@ -438,3 +438,29 @@ def test_bpp_solve_gives_a_large_workspace_back(gpu):
             assert np.array_equal(a, b)
         for a, b in zip(c.bpp_solve(A.T @ A, B[:, :100]), small):
             assert np.array_equal(a, b)
+
+
+def test_update_device_while_another_stream_is_captured(gpu, oracle_lib):
+    # the packed solver's flags are allocated on the first such call
+    import torch
+    k, rows = 40, 700
+    rng = np.random.default_rng(92)
+    A = rng.random((3 * k, k))
+    G = A.T @ A
+    B = G @ np.maximum(rng.standard_normal((k, rows)), 0.0) + 0.1 * rng.standard_normal((k, rows))
+    want, _, _ = oracle_lib.bpp_update(B.T.copy(), G)
+    with gpu.Context(0, "fp64") as c:
+        Gd = torch.tensor(G, device="cuda")
+        M = torch.tensor(B.T.copy(), device="cuda")
+        H = torch.zeros(rows, k, device="cuda", dtype=torch.float64)
+        y = torch.zeros(8, device="cuda")
+        torch.cuda.synchronize()
+        graph, other = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=other):
+            y += 1
+            c.update_device("anlsbpp", H.data_ptr(), M.data_ptr(), Gd.data_ptr(), rows, k)
+        c.sync()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float(y.sum()) == 8.0
+        assert rel(H.cpu().numpy(), want) < TOL

@@ -411,6 +411,7 @@ class Batch:
     def set_factors(self, index, F):
         F = [_c64(f) for f in F]
         _check(load().planc_gpu_batch_set_factors(self.h, index, _fptrs(F), F[0].shape[1]))
+        self.members[index] = (self.members[index][0], F[0].shape[1])
 
     def run(self, algo, iters, compute_error=True):
         errs = np.zeros((len(self.members), max(iters, 1)))

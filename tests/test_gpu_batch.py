@@ -150,3 +150,35 @@ def test_batch_long_contraction_gives_the_same_bits(gpu, prec, few, monkeypatch)
     for (Fa, la), (Fb, lb) in zip(f1, f0):
         assert np.array_equal(la, lb)
         assert all(np.array_equal(a, b_) for a, b_ in zip(Fa, Fb))
+
+
+@pytest.mark.parametrize("prec,algo", [("bf16", "hals"), ("bf16", "mu"), ("bf16", "anlsbpp"), ("fp64", "hals")])
+def test_batch_runs_again_from_other_factors(gpu, prec, algo):
+    # the captured iteration stays while new factors are set; a member's rank
+    # changes, and changes back; other lengths
+    members = _members(n=5, seed=210)
+    data = [X.astype(np.float32) if prec != "fp64" else X for X, _ in members]
+    starts = [F0 for _, F0 in members]
+
+    def check(b, iters):
+        errs = b.run(algo, iters)
+        for i, X in enumerate(data):
+            Fb, lb = b.get_factors(i)
+            with gpu.Context(0, prec) as c:
+                c.set_tensor(X)
+                c.set_factors(starts[i])
+                e = c.run(algo, iters)
+                Fc, lc = c.get_factors()
+            assert rel(errs[i], e) < 1e-13 and rel(lb, lc) < 1e-13
+            assert all(rel(a, b_) < 1e-13 for a, b_ in zip(Fb, Fc))
+
+    with gpu.Batch(0, prec, nstreams=4) as b:
+        for X, F0 in zip(data, starts):
+            b.add(X, F0)
+        check(b, 4)
+        for again, iters in enumerate((4, 7, 2)):
+            for i, X in enumerate(data):
+                k = 20 if (again, i) == (1, 1) else members[i][1][0].shape[1]
+                starts[i] = init_factors(X.shape, k, seed=300 + 10 * again + i)
+                b.set_factors(i, starts[i])
+            check(b, iters)

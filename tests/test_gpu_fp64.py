@@ -464,3 +464,21 @@ def test_update_device_while_another_stream_is_captured(gpu, oracle_lib):
         torch.cuda.synchronize()
         assert float(y.sum()) == 8.0
         assert rel(H.cpu().numpy(), want) < TOL
+
+
+@pytest.mark.parametrize("dims,k", [((8186, 3, 2), 16), ((8187, 3, 2), 16), ((131063, 3, 1), 1),
+                                    ((131065, 3, 2), 1), ((2000, 3, 2), 64), ((2100, 3, 2), 64), ((7, 5, 3), 3)])
+def test_factors_in_one_copy_and_in_several(gpu, dims, k):
+    # below, at and above 1 MB of factors, odd sizes; lambda given or not
+    X, _ = cp_tensor(dims, 1, seed=93)
+    F = init_factors(dims, k, seed=94)
+    lam = 1.0 + np.arange(k)
+    with gpu.Context(0, "fp64") as c:
+        c.set_tensor(X)
+        for given in (lam, None, lam[::-1].copy()):
+            c.set_factors(F, given)
+            got, gl = c.get_factors()
+            assert np.array_equal(gl, np.ones(k) if given is None else given)
+            for a, b in zip(got, _normalized(F)):
+                assert rel(a, b) < 1e-14
+            F = [f[::-1].copy() for f in F]

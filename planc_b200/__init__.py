@@ -170,8 +170,10 @@ class Context:
         # bumped by every call that may leave new dimension-tree intermediates
         # in the context (a caller that wants to reuse them checks it)
         self.tree_epoch = 0
+        self.torch_stream = None  # the context's stream as planc_b200.autograd wraps it
 
     def close(self):
+        self.torch_stream = None
         if self.h:
             load().planc_gpu_destroy(self.h)
             self.h = None

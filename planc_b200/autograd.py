@@ -24,23 +24,32 @@ import torch
 from . import Context
 
 
+def _streams(handle, dev):
+    """The context's stream, wrapped once per context (a wrapper costs 3 us, the
+    call is host-bound), and the caller's."""
+    kept = handle.torch_stream
+    if kept is None or kept.device != dev:
+        kept = handle.torch_stream = torch.cuda.ExternalStream(handle.stream, device=dev)
+    return kept, torch.cuda.current_stream(dev)
+
+
 class _CPLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, handle, *factors):
         factors = [f.contiguous() for f in factors]
         dev = factors[0].device
         k = factors[0].shape[1]
-        stream = torch.cuda.ExternalStream(handle.stream, device=dev)
+        stream, caller = _streams(handle, dev)
         M0 = torch.empty_like(factors[0])
         G = torch.empty(len(factors), k, k, dtype=torch.float64, device=dev)
         loss = torch.empty((), dtype=torch.float64, device=dev)
         ptrs = [f.data_ptr() for f in factors]
-        stream.wait_stream(torch.cuda.current_stream(dev))
+        stream.wait_stream(caller)
         handle.mttkrp_device(0, ptrs, M0.data_ptr(), dimtree=True, reuse=False)
         ctx.tree_epoch = handle.tree_epoch
         # Grams of every factor and 1/2||X||^2 - <M_0, F_0> + 1/2 sum(*_n G_n)
         handle.cp_loss_device(ptrs, M0.data_ptr(), G.data_ptr(), loss.data_ptr())
-        torch.cuda.current_stream(dev).wait_stream(stream)
+        caller.wait_stream(stream)
         ctx.handle = handle
         ctx.save_for_backward(M0, G, *factors)
         return loss
@@ -50,13 +59,13 @@ class _CPLoss(torch.autograd.Function):
         M0, G, *factors = ctx.saved_tensors
         handle = ctx.handle
         dev = factors[0].device
-        stream = torch.cuda.ExternalStream(handle.stream, device=dev)
+        stream, caller = _streams(handle, dev)
         ptrs = [f.data_ptr() for f in factors]
         N = len(factors)
         Ms = [M0] + [torch.empty_like(factors[n]) for n in range(1, N)]
         grads = [torch.empty_like(f) for f in factors]
         gs = g.detach().to(device=dev, dtype=torch.float64).contiguous()
-        stream.wait_stream(torch.cuda.current_stream(dev))
+        stream.wait_stream(caller)
         # the tree holds this forward's mode-0 intermediates only if no other
         # MTTKRP ran on the context since
         fresh = handle.tree_epoch == ctx.tree_epoch
@@ -68,7 +77,7 @@ class _CPLoss(torch.autograd.Function):
         # every mode's gradient g (F_n (*_{m != n} G_m) - M_n) in one launch
         handle.cp_grads_device(ptrs, G.data_ptr(), [m.data_ptr() for m in Ms], gs.data_ptr(),
                                [x.data_ptr() for x in grads])
-        torch.cuda.current_stream(dev).wait_stream(stream)
+        caller.wait_stream(stream)
         return (None, *grads)
 
 
@@ -79,12 +88,12 @@ def projected_accelerated_step(loss_fn, Y, grads, Fprev, eta, mom, Fnew, Ynew):
     (outputs may be the inputs of the same factor)."""
     handle = loss_fn.ctx
     dev = Y[0].device
-    stream = torch.cuda.ExternalStream(handle.stream, device=dev)
-    stream.wait_stream(torch.cuda.current_stream(dev))
+    stream, caller = _streams(handle, dev)
+    stream.wait_stream(caller)
     handle.cp_step_device([t.data_ptr() for t in Y], [t.data_ptr() for t in grads],
                           [t.data_ptr() for t in Fprev], eta, mom, [t.data_ptr() for t in Fnew],
                           [t.data_ptr() for t in Ynew])
-    torch.cuda.current_stream(dev).wait_stream(stream)
+    caller.wait_stream(stream)
 
 
 class CPLoss:

@@ -276,3 +276,24 @@ def test_cp_loss_workspace_follows_modes_and_rank(gpu):
     assert abs(value.item() - ref) / ref < 1e-10
     del graph
     lossf.close()
+
+
+def test_cp_loss_from_several_streams_and_after_close(gpu):
+    import torch
+    X, F, lossf, Ft = _setup("fp64", dims=(24, 20, 16), k=4, seed=45)
+    want = lossf(*Ft)
+    want.backward()
+    grads = [f.grad.clone() for f in Ft]
+    torch.cuda.synchronize()
+    for s in (torch.cuda.Stream(), torch.cuda.current_stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(s):
+            for f in Ft:
+                f.grad = None
+            got = lossf(*Ft)
+            got.backward()
+            same = [torch.equal(f.grad, g) for f, g in zip(Ft, grads)]
+        torch.cuda.synchronize()
+        assert got.item() == want.item() and all(same)
+    lossf.close()
+    with pytest.raises(Exception):
+        lossf(*Ft)

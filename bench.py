@@ -325,7 +325,8 @@ def main():
     sampler.start()
     time.sleep(0.2)
     barrier()
-    # timed region: one CUDA graph per outer iteration, as a user's run executes
+    # timed region: as a user's run of this length executes (above 32 iterations
+    # a graph of up to eight is captured at its start and replayed)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record(stream)
     ctx.run(args.algo, args.steps, compute_error=True)
@@ -344,8 +345,8 @@ def main():
     ctx.run(args.algo, args.steps, compute_error=True)
     ek1.record(stream)
     barrier()
-    # the graph-timed region replays exactly these kernels (launch() counts
-    # each kernel launch; a graph replay is not counted by the library)
+    # the timed region runs exactly these kernels (launch() counts each kernel
+    # launch; a graph replay is not counted by the library)
     launches = ctx.launch_count() - n1
     kt = ctx.kernel_times()
     ctx.set_timing(False)
@@ -393,7 +394,7 @@ def main():
         ctx64 = gpu.Context(dev, "fp64")
         ctx64.set_tensor(X.data_ptr(), dims=dims, dtype="f32")
         ctx64.set_factors(F0)
-        ctx64.run(args.algo, 2, compute_error=True)  # captures the timed graph
+        ctx64.run(args.algo, 2, compute_error=True)  # warm-up
         k64 = max(3, min(args.steps, 20))
         s64 = torch.cuda.ExternalStream(ctx64.stream, device="cuda:%d" % dev)
         barrier()

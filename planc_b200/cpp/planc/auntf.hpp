@@ -11,7 +11,7 @@
 //
 // The built-in subclasses (NTFMU, NTFHALS, NTFANLSBPP, NTFAOADMM, NTFNES)
 // also report device_algo(), which lets computeNTF run the whole iteration on
-// the GPU (one CUDA graph per iteration; NTFNES's acceleration included); any
+// the GPU (replayed CUDA graphs; NTFNES's acceleration included); any
 // other subclass runs its update() on the host between the device's Gram /
 // MTTKRP and normalisation steps. With accelerated(true) on a built-in update
 // other than NTFNES, the device runs one iteration at a time and the host

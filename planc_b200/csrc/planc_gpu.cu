@@ -3,8 +3,8 @@
 // One context = one device-resident tensor + CP factors + one stream. The
 // AUNTF outer iteration (ntf/auntf.hpp:128-177) is issued as a fixed launch
 // sequence per mode: [MTTKRP] -> [update] -> [normalise + Gram + next
-// leave-one-out Gram], then the Gram-form error; it is captured once into a
-// CUDA graph and replayed for every iteration.
+// leave-one-out Gram], then the Gram-form error; a run asked for again replays
+// CUDA graphs of up to eight iterations.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -780,7 +780,7 @@ void contract_f64_attrs_kp() {
   }
 }
 
-// Dynamic shared-memory limits of every k_contract_f64 instance (up to 92 KB)
+// Dynamic shared-memory limits of every k_contract_f64 instance (up to 106 KB)
 // on device dev, set once per device before its first launch.
 std::mutex g_contract_attr_mutex;
 bool g_contract_attr_set[64] = {false};

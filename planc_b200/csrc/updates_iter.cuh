@@ -252,7 +252,10 @@ __global__ void __launch_bounds__(32 * ADMM_WARPS) k_admm_step(
 // every entry's subtractions in the order of the left-looking sums), and all
 // 5 iterations run before the cluster exchanges their 5 sets of norms: when
 // an earlier one meets the test (ntfaoadmm.hpp:63-71) the rows start again
-// from global memory and run that many. At 300 / 220 rows of rank 24: 42 / 36 us
+// from global memory and run that many. That is rare: a factor is normalised
+// after each update, so the next one has to move it back to its scale and
+// takes all 5 iterations (none of 175800 updates of random tensors stopped
+// earlier). At 300 / 220 rows of rank 24: 42 / 36 us
 // (50 with a factor formed by dot products of one thread a pivot and an
 // exchange an iteration).
 template <int KP, int R>

@@ -182,3 +182,27 @@ def test_batch_runs_again_from_other_factors(gpu, prec, algo):
                 starts[i] = init_factors(X.shape, k, seed=300 + 10 * again + i)
                 b.set_factors(i, starts[i])
             check(b, iters)
+
+
+@pytest.mark.parametrize("algo", ["hals", "mu"])
+def test_batch_of_many_small_members_gives_the_same_bits(gpu, algo, monkeypatch):
+    # enough rows of I_1 for four a CTA in the left multi-TTV, with remainders
+    # of one, two and three
+    members = []
+    for i in range(26):
+        dims, k = (20 + i, 46 + i % 7, 3 + i % 5), (4, 7, 16, 21, 32, 40)[i % 6]
+        X, _ = cp_tensor(dims, 3, noise=0.01, seed=230 + i)
+        members.append((X.astype(np.float32), init_factors(dims, k, seed=330 + i)))
+    res = {}
+    for grouped in ("1", "0"):
+        monkeypatch.setenv("PLANC_GPU_BATCH_GROUPED", grouped)
+        with gpu.Batch(0, "bf16", nstreams=4) as b:
+            for X, F0 in members:
+                b.add(X, F0)
+            errs = b.run(algo, 3)
+            res[grouped] = (errs, [b.get_factors(i) for i in range(len(members))])
+    (e1, f1), (e0, f0) = res["1"], res["0"]
+    assert np.array_equal(e1, e0)
+    for (Fa, la), (Fb, lb) in zip(f1, f0):
+        assert np.array_equal(la, lb)
+        assert all(np.array_equal(a, b_) for a, b_ in zip(Fa, Fb))

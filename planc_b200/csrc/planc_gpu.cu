@@ -702,6 +702,7 @@ void ensure_buffers_impl(planc_gpu_ctx* c) {
   }
   need = std::max<size_t>(need, 4096);
   if (need > c->scratch_elems) {
+    c->scratch_elems = 0;
     dalloc(&c->scratch, need);
     c->scratch_elems = need;
   }
@@ -924,11 +925,13 @@ void ensure_direct(planc_gpu_ctx* c) {
     grew = true;
   }
   if (tail > c->krp_tail_elems) {
+    c->krp_tail_elems = 0;
     dalloc(&c->krp_tail, tail);
     c->krp_tail_elems = tail;
     grew = true;
   }
   if (need > c->scratch_elems) {
+    c->scratch_elems = 0;
     dalloc(&c->scratch, need);
     c->scratch_elems = need;
     grew = true;
@@ -1712,19 +1715,24 @@ void ensure_factor_buffers(planc_gpu_ctx* c) {
   off[c->N] = total;
   total += even(c->k);
   if (same && c->lambda == c->fslab + off[c->N] && c->fslab_elems == total) return;
+  // an allocation that fails leaves no size or pointer of a buffer that is gone
+  for (int n = 0; n < kMaxModes; ++n) c->F[n] = nullptr;
+  c->lambda = nullptr;
+  c->fslab_elems = 0;
+  c->buf_epoch++;
   dalloc(&c->fslab, total);
-  c->fslab_elems = total;
   for (int n = 0; n < c->N; ++n) {
-    c->F[n] = c->fslab + off[n];
-    if (c->factor_cap[n] != (int64_t)c->dims[n] * c->k) {
-      dalloc(&c->M[n], (size_t)c->dims[n] * c->k);
-      c->factor_cap[n] = (int64_t)c->dims[n] * c->k;
+    const int64_t need = c->dims[n] * c->k;
+    if (c->factor_cap[n] != need) {
+      c->factor_cap[n] = 0;
+      dalloc(&c->M[n], (size_t)need);
+      c->factor_cap[n] = need;
     }
   }
-  for (int n = c->N; n < kMaxModes; ++n) c->F[n] = nullptr;
+  c->fslab_elems = total;
+  for (int n = 0; n < c->N; ++n) c->F[n] = c->fslab + off[n];
   c->lambda_off = off[c->N];
   c->lambda = c->fslab + off[c->N];
-  c->buf_epoch++;
 }
 
 void free_all(planc_gpu_ctx* c) {
@@ -2043,7 +2051,10 @@ int planc_gpu_set_factors(planc_gpu_ctx* c, const double* const* F, const double
     if (!c->have_tensor) fail(PLANC_GPU_ERR_STATE, "set the tensor before the factors");
     if (k < 1 || k > kMaxRank)
       fail(PLANC_GPU_ERR_UNSUPPORTED, "rank must be in [1, " + std::to_string(kMaxRank) + "]");
+    for (int n = 0; n < c->N; ++n)
+      if (!F[n]) fail(PLANC_GPU_ERR_ARG, "null factor");
     set_device(c);
+    c->have_factors = c->nmf_have = false;  // until the new ones are in place
     // Cached iteration graphs stay valid when no buffer moves: the new
     // factors are copied into the same device arrays. Any reallocation below
     // bumps the buffer epoch, which rebuilds the graphs before their next use.
@@ -2059,8 +2070,6 @@ int planc_gpu_set_factors(planc_gpu_ctx* c, const double* const* F, const double
       f(c->Q);
       for (int n = 0; n < kMaxModes; ++n) c->factor_cap[n] = 0;
     }
-    for (int n = 0; n < c->N; ++n)
-      if (!F[n]) fail(PLANC_GPU_ERR_ARG, "null factor");
     c->k = k;
     ensure_factor_buffers(c);
     if (!c->Gall || c->gall_elems != (size_t)c->N * k * k) {
@@ -2079,6 +2088,7 @@ int planc_gpu_set_factors(planc_gpu_ctx* c, const double* const* F, const double
       }
     }
     if (!c->Gloo || c->kvec != k) {
+      c->kvec = 0;
       dalloc(&c->Gloo, (size_t)k * k);
       dalloc(&c->lam_tmp, (size_t)k);
       c->kvec = k;
@@ -2113,7 +2123,6 @@ int planc_gpu_set_factors(planc_gpu_ctx* c, const double* const* F, const double
     if (c->cp_ws) ensure_cp_ws(c);  // the next loss may be under capture
     if (!packed) CK(cudaStreamSynchronize(c->stream));
     c->have_factors = true;
-    c->nmf_have = false;
   });
 }
 
@@ -2462,6 +2471,7 @@ int planc_gpu_gram_device(planc_gpu_ctx* c, const double* F, int64_t rows, int k
     const int nblk = (int)((rows + rpb - 1) / rpb);
     if ((size_t)nblk * k * k > c->gram_part_elems) {
       if (c->capturing) fail(PLANC_GPU_ERR_STATE, "Gram partials would grow during capture");
+      c->gram_part_elems = 0;
       dalloc(&c->gram_part, (size_t)nblk * k * k);
       c->gram_part_elems = (size_t)nblk * k * k;
       c->buf_epoch++;
@@ -3374,6 +3384,7 @@ void batch_finish(planc_gpu_batch* b, int iters = 0, double* errs = nullptr) {
   const size_t words = n * ne + (n + 1) / 2;
   if (b->out_elems < words) {
     CK(cudaStreamSynchronize(b->master));
+    b->out_elems = 0;
     dalloc(&b->out_dev, words);
     b->out_elems = words;
   }
@@ -3474,6 +3485,7 @@ int planc_gpu_batch_run(planc_gpu_batch* b, int algo, int iters, int compute_err
     if (algo != PLANC_GPU_MU && algo != PLANC_GPU_HALS && algo != PLANC_GPU_ANLSBPP)
       fail(PLANC_GPU_ERR_ARG, "unknown algorithm");
     if (iters <= 0) return;
+    for (auto* m : b->members) require_ready(m);
     CK(cudaSetDevice(b->device));
     const bool err = compute_error != 0;
     batch_ensure(b, algo, iters, err);
@@ -3499,6 +3511,7 @@ int planc_gpu_batch_get_factors(planc_gpu_batch* b, int index, double* const* F,
 int planc_gpu_batch_autotune(planc_gpu_batch* b, int algo, int trials, double* best_ms) {
   return guarded([&] {
     if (!b || b->members.empty()) fail(PLANC_GPU_ERR_STATE, "empty batch");
+    for (auto* m : b->members) require_ready(m);
     if (trials < 1) trials = 1;
     CK(cudaSetDevice(b->device));
     // save factors so the tuning iterations leave no trace
@@ -3736,6 +3749,7 @@ void ensure_nmf(planc_gpu_ctx* c, int iters) {
     size_t need = std::max(tc_long_scratch_elems(c->tct, true, k, eff_sm(c)),
                            tc_long_scratch_elems(c->tct, false, k, eff_sm(c)));
     if (need > c->scratch_elems) {
+      c->scratch_elems = 0;
       dalloc(&c->scratch, need);
       c->scratch_elems = need;
       c->buf_epoch++;
@@ -3758,6 +3772,7 @@ void ensure_nmf(planc_gpu_ctx* c, int iters) {
     c->buf_epoch++;
   }
   if (iters > c->nmf_cap) {
+    c->nmf_cap = 0;
     dalloc(&c->nmf_obj, (size_t)iters);
     dalloc(&c->nmf_rel, (size_t)iters);
     c->nmf_cap = iters;
@@ -4017,6 +4032,7 @@ int planc_gpu_nmf_set_factors(planc_gpu_ctx* c, const double* W, const double* H
       fail(PLANC_GPU_ERR_UNSUPPORTED, "rank must be in [1, " + std::to_string(kMaxRank) + "]");
     set_device(c);
     reset_graph(c);
+    c->have_factors = c->nmf_have = false;  // until the new ones are in place
     if (k != c->k) {
       free_update_state(c);
       for (int i = 0; i < kMaxModes; ++i) c->factor_cap[i] = 0;
@@ -4027,8 +4043,7 @@ int planc_gpu_nmf_set_factors(planc_gpu_ctx* c, const double* W, const double* H
     for (int i = 0; i < 2; ++i)
       CK(cudaMemcpyAsync(c->F[i], src[i], (size_t)c->dims[i] * k * 8, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    c->have_factors = false;  // the NTF factors (normalised, with Grams) are not these
-    c->nmf_have = true;
+    c->nmf_have = true;  // (the NTF factors, normalised and with Grams, are not these)
   });
 }
 

@@ -1854,6 +1854,7 @@ inline cudaError_t tc_ensure(TcTensor& t, int k) {
   e = cudaMalloc(&t.bimg, need);
   if (e == cudaSuccess && need0) e = cudaMalloc(&t.bimg0, need0);
   if (e == cudaSuccess && needw) e = cudaMalloc(&t.wimg, needw);
+  if (e != cudaSuccess) t.kpad = 0;  // nothing to take for complete next time
   return e;
 }
 

@@ -71,3 +71,42 @@ def test_zero_factor_column_is_handled(gpu, oracle_lib):
         c.set_factors(F0)
         e = c.run("mu", 2)
     assert np.allclose(e, eo, rtol=1e-10, atol=0)
+
+
+# the memory left: too little for the factors; for them but not their MTTKRPs;
+# for both but not the partial contraction
+@pytest.mark.parametrize("left_mb", [200, 450, 900])
+@pytest.mark.parametrize("prec", ["fp64", "bf16"])
+def test_factors_that_do_not_fit(gpu, prec, left_mb):
+    # the call fails, what would use the factors is refused (the old ones are
+    # gone), and the context works again once there is room
+    import torch
+    dims, k = (600_000, 4, 3), 64
+    rng = np.random.default_rng(95)
+    X = rng.random(dims, dtype=np.float32)
+    small = [rng.random((d, 2)) for d in dims]
+    large = [rng.random((d, k)) for d in dims]
+    with gpu.Context(0, prec) as ref:
+        ref.set_tensor(X)
+        ref.set_factors(large)
+        want = ref.mttkrp(2)
+    with gpu.Context(0, prec) as c:
+        c.set_tensor(X)
+        c.set_factors(small)
+        torch.cuda.empty_cache()
+        torch.cuda.synchronize()
+        fill = torch.empty(torch.cuda.mem_get_info()[0] - (left_mb << 20), dtype=torch.uint8, device="cuda")
+        try:
+            with pytest.raises(gpu.PlancGpuError):
+                c.set_factors(large)
+            with pytest.raises(gpu.PlancGpuError, match="no factors"):
+                c.run("hals", 1)
+            with pytest.raises(gpu.PlancGpuError, match="no factors"):
+                c.get_factors()
+        finally:
+            del fill
+            torch.cuda.empty_cache()
+        c.set_factors(large)
+        assert np.array_equal(c.mttkrp(2), want)
+        c.set_factors(small)
+        assert np.isfinite(c.run("hals", 1)).all()
